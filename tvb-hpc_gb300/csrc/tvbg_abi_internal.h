@@ -35,17 +35,22 @@ BlockedKernel blocked_kernel_g2do(int cfun, int tpn, int k);
 BlockedKernel blocked_kernel_mpr(int cfun, int tpn, int k);
 BlockedKernel blocked_kernel_linear(int cfun, int tpn, int k);
 BlockedKernel blocked_kernel_g2dosc(int cfun, int tpn, int k);
+// Builds of a lane-interleaved group kernel: plain or pipelined, by the
+// largest CTA they take (registers a thread: 64, 80, 128).
+enum GroupForm { kPlain1024, kPlain768, kPipe1024, kPipe768, kPipe512 };
 // Lane-interleaved group kernel signature and per-model lookup for (cfun, K).
 using GroupKernel = void (*)(const tvbg_group*, int32_t, const int32_t*, int32_t*);
-GroupKernel group_kernel_kuramoto(int cfun, int k, bool pipe);
-GroupKernel group_kernel_g2do(int cfun, int k, bool pipe);
-GroupKernel group_kernel_mpr(int cfun, int k, bool pipe);
-GroupKernel group_kernel_linear(int cfun, int k, bool pipe);
-GroupKernel group_kernel_g2dosc(int cfun, int k, bool pipe);
-GroupKernel group_kernel_rww(int cfun, int k, bool pipe);
-GroupKernel group_kernel_jansenrit(int cfun, int k, bool pipe);
+GroupKernel group_kernel_kuramoto(int cfun, int k, GroupForm form);
+GroupKernel group_kernel_g2do(int cfun, int k, GroupForm form);
+GroupKernel group_kernel_mpr(int cfun, int k, GroupForm form);
+GroupKernel group_kernel_linear(int cfun, int k, GroupForm form);
+GroupKernel group_kernel_g2dosc(int cfun, int k, GroupForm form);
+GroupKernel group_kernel_rww(int cfun, int k, GroupForm form);
+GroupKernel group_kernel_jansenrit(int cfun, int k, GroupForm form);
 // Group kernel of the engine library for (model, cfun, K), nullptr if not built.
-GroupKernel lookup_group_kernel(int model, int cfun, int k, bool pipe = false);
+GroupKernel lookup_group_kernel(int model, int cfun, int k, GroupForm form);
+// The build for a launch of `ctas` CTAs of `threads` threads.
+GroupForm group_form(int threads, long long ctas, bool pipe);
 // Shared memory of the blocked kernel beyond the ring (floats): K * nmax * (2 + NS) + 4 * nmax.
 uint32_t blocked_aux_bytes(int model, int k, int nmax);
 

@@ -231,7 +231,7 @@ __global__ void __launch_bounds__(512, 1)
     adjoint_group_kernel(const tvbg_adjoint_group* __restrict__ adj, int32_t n_groups,
                          int32_t* __restrict__ status) {
     __shared__ __align__(16) tvbg_adjoint_group s;
-    extern __shared__ float csum[];  // [(PIPE ? 2 : 1)][K][team threads]: out-edge sums
+    extern __shared__ __align__(16) float csum[];  // [(PIPE ? 2 : 1)][K][team threads]: out-edge sums
     const int cid = static_cast<int>(cluster_id_x());
     if (cid >= n_groups) return;  // uniform over the cluster
     {

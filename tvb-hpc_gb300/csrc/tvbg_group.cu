@@ -8,15 +8,15 @@ using namespace tvbg;
 
 namespace {
 
-GroupKernel lookup_group(int model, int cfun, int k, bool pipe) {
+GroupKernel lookup_group(int model, int cfun, int k, GroupForm form) {
     switch (model) {
-        case TVBG_MODEL_KURAMOTO: return group_kernel_kuramoto(cfun, k, pipe);
-        case TVBG_MODEL_G2DO: return group_kernel_g2do(cfun, k, pipe);
-        case TVBG_MODEL_MPR: return group_kernel_mpr(cfun, k, pipe);
-        case TVBG_MODEL_LINEAR: return group_kernel_linear(cfun, k, pipe);
-        case TVBG_MODEL_G2DOSC: return group_kernel_g2dosc(cfun, k, pipe);
-        case TVBG_MODEL_RWW: return group_kernel_rww(cfun, k, pipe);
-        case TVBG_MODEL_JANSENRIT: return group_kernel_jansenrit(cfun, k, pipe);
+        case TVBG_MODEL_KURAMOTO: return group_kernel_kuramoto(cfun, k, form);
+        case TVBG_MODEL_G2DO: return group_kernel_g2do(cfun, k, form);
+        case TVBG_MODEL_MPR: return group_kernel_mpr(cfun, k, form);
+        case TVBG_MODEL_LINEAR: return group_kernel_linear(cfun, k, form);
+        case TVBG_MODEL_G2DOSC: return group_kernel_g2dosc(cfun, k, form);
+        case TVBG_MODEL_RWW: return group_kernel_rww(cfun, k, form);
+        case TVBG_MODEL_JANSENRIT: return group_kernel_jansenrit(cfun, k, form);
         default: return nullptr;
     }
 }
@@ -25,11 +25,13 @@ const ErrSink kSink{set_error, set_cuda_error};
 
 // Validate a group launch; its dynamic shared memory holds the K coupling
 // sums of every thread.
-int check_group_launch(const tvbg_launch* cfg, GroupKernel* kfn, int* cluster, size_t* smem) {
+int check_group_launch(const tvbg_launch* cfg, int32_t n_groups, GroupKernel* kfn, int* cluster,
+                       size_t* smem) {
     int rc = check_group_cfg(cfg, kSink, cluster, (1u << 4) | (1u << 8), true);
     if (rc) return rc;
     const bool pipe = cfg->tpn == TVBG_GROUP_PIPELINED;
-    *kfn = lookup_group(cfg->model, cfg->cfun, cfg->block_k, pipe);
+    *kfn = lookup_group(cfg->model, cfg->cfun, cfg->block_k,
+                        group_form(cfg->threads, static_cast<long long>(n_groups) * *cluster, pipe));
     if (!*kfn)
         return set_error(TVBG_EUNSUPPORTED, "group kernel not built for this model/coupling/block_k");
     *smem = pipe ? group_pipelined_smem_bytes(cfg->block_k, cfg->threads, group_channels(cfg->cfun))
@@ -39,8 +41,25 @@ int check_group_launch(const tvbg_launch* cfg, GroupKernel* kfn, int* cluster, s
 
 }  // namespace
 
-GroupKernel tvbg::lookup_group_kernel(int model, int cfun, int k, bool pipe) {
-    return lookup_group(model, cfun, k, pipe);
+GroupKernel tvbg::lookup_group_kernel(int model, int cfun, int k, GroupForm form) {
+    return lookup_group(model, cfun, k, form);
+}
+
+// More registers a thread put more ring loads in flight, so each CTA runs
+// faster, but fewer CTAs are resident: the 512-thread build is taken unless
+// the 768-thread one needs fewer waves of CTAs.  Measured (ms, 800 steps,
+// MPR; 512 / 768 build): N = 84, 32 groups, 256 x 6 threads 0.320 / 0.369; N = 84,
+// 128 groups, 448 x 3 0.97 / 1.10 (one CTA per SM in both); N = 192, 32
+// groups, 256 x 12 0.75 / 0.55 (two waves against one).
+GroupForm tvbg::group_form(int threads, long long ctas, bool pipe) {
+    if (!pipe) return threads > 768 ? kPlain1024 : kPlain768;
+    if (threads > 768) return kPipe1024;
+    if (threads > 512) return kPipe768;
+    const int sms = device_sms();
+    if (sms <= 0) return kPipe768;
+    const long long wide = static_cast<long long>(512 / threads) * sms;       // resident CTAs, 128 registers
+    const long long mid = static_cast<long long>(65536 / (80 * threads)) * sms;  // 80 registers
+    return (ctas + wide - 1) / wide > (ctas + mid - 1) / mid ? kPipe768 : kPipe512;
 }
 
 extern "C" {
@@ -77,7 +96,7 @@ int tvbg_group_run(const tvbg_group* d_groups, int32_t n_groups, const tvbg_laun
     GroupKernel kfn = nullptr;
     int cluster = 1;
     size_t smem = 0;
-    int rc = check_group_launch(cfg, &kfn, &cluster, &smem);
+    int rc = check_group_launch(cfg, n_groups, &kfn, &cluster, &smem);
     if (rc) return rc;
     return launch_group_kernel(kfn, d_groups, n_groups, cfg, cluster, smem, stream, kSink);
 }
@@ -87,11 +106,11 @@ int tvbg_group_occupancy(const tvbg_launch* cfg, int32_t* ctas_per_sm, int32_t* 
     GroupKernel kfn = nullptr;
     int cluster = 1;
     size_t smem = 0;
-    int rc = check_group_launch(cfg, &kfn, &cluster, &smem);
+    int rc = check_group_launch(cfg, 1, &kfn, &cluster, &smem);
     if (rc) return rc;
     int n = 0;
     cudaError_t e = cudaSuccess;
-    if (smem + sizeof(tvbg_group) > 48u * 1024u) {  // beyond the default: opt in
+    if (smem + kGroupStaticBytes > 48u * 1024u) {  // beyond the default: opt in
         e = cudaFuncSetAttribute(reinterpret_cast<const void*>(kfn),
                                  cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
         if (e != cudaSuccess) return set_cuda_error(e, "tvbg_group_occupancy: smem attribute");
@@ -113,10 +132,10 @@ int tvbg_group_max_clusters(const tvbg_launch* cfg, int32_t* max_clusters) {
     GroupKernel kfn = nullptr;
     int cluster = 1;
     size_t smem = 0;
-    int rc = check_group_launch(cfg, &kfn, &cluster, &smem);
+    int rc = check_group_launch(cfg, 1, &kfn, &cluster, &smem);
     if (rc) return rc;
     cudaError_t e = cudaSuccess;
-    if (smem + sizeof(tvbg_group) > 48u * 1024u) {
+    if (smem + kGroupStaticBytes > 48u * 1024u) {
         e = cudaFuncSetAttribute(reinterpret_cast<const void*>(kfn),
                                  cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
         if (e != cudaSuccess) return set_cuda_error(e, "tvbg_group_max_clusters: smem attribute");

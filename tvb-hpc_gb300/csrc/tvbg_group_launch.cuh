@@ -38,6 +38,15 @@ inline int check_group_cfg(const tvbg_launch* cfg, const ErrSink& es, int* clust
     return TVBG_OK;
 }
 
+// SMs of the current device (0 if it cannot be asked).
+inline int device_sms() {
+    int dev = 0, n = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
+        return 0;
+    return n;
+}
+
 // Ring channels of a coupling id (the group kernel's shared-memory sums scale with it).
 inline int group_channels(int cfun) {
     return (cfun == TVBG_CFUN_KURAMOTO || cfun == TVBG_CFUN_LEMS_SC || cfun == TVBG_CFUN_LEMS_2) ? 2
@@ -53,7 +62,7 @@ inline int launch_group_kernel(GroupKernelFn kfn, const tvbg_group* d_groups, in
         return es.error(TVBG_EINVAL, "tvbg_group_run: bad group array");
     if (n_groups == 0) return TVBG_OK;
     cudaError_t e = cudaSuccess;
-    if (smem + sizeof(tvbg_group) > 48u * 1024u) {  // beyond the default: opt in
+    if (smem + kGroupStaticBytes > 48u * 1024u) {  // beyond the default: opt in
         e = cudaFuncSetAttribute(reinterpret_cast<const void*>(kfn),
                                  cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
         if (e != cudaSuccess) return es.cuda(e, "tvbg_group_run: smem attribute");

@@ -6,20 +6,32 @@
 
 namespace tvbg {
 
+template <int CF, int K>
+static GroupKernel pick_form(GroupForm form) {
+    switch (form) {
+        case kPlain1024: return group_kernel<Linear, CF, K, 1024>;
+        case kPlain768: return group_kernel<Linear, CF, K, 768>;
+        case kPipe1024: return group_kernel_pipelined<Linear, CF, K, 1024>;
+        case kPipe768: return group_kernel_pipelined<Linear, CF, K, 768>;
+        case kPipe512: return group_kernel_pipelined<Linear, CF, K, 512>;
+    }
+    return nullptr;
+}
+
 template <int CF>
-static GroupKernel pick_k(int k, bool pipe) {
+static GroupKernel pick_k(int k, GroupForm form) {
     switch (k) {
-        case 4: return pipe ? group_kernel_pipelined<Linear, CF, 4> : group_kernel<Linear, CF, 4>;
-        case 8: return pipe ? group_kernel_pipelined<Linear, CF, 8> : group_kernel<Linear, CF, 8>;
+        case 4: return pick_form<CF, 4>(form);
+        case 8: return pick_form<CF, 8>(form);
         default: return nullptr;
     }
 }
 
-GroupKernel group_kernel_linear(int cfun, int k, bool pipe) {
+GroupKernel group_kernel_linear(int cfun, int k, GroupForm form) {
     switch (cfun) {
-        case TVBG_CFUN_LINEAR: return pick_k<TVBG_CFUN_LINEAR>(k, pipe);
-        case TVBG_CFUN_DIFF: return pick_k<TVBG_CFUN_DIFF>(k, pipe);
-        case TVBG_CFUN_SIGMOIDAL: return pick_k<TVBG_CFUN_SIGMOIDAL>(k, pipe);
+        case TVBG_CFUN_LINEAR: return pick_k<TVBG_CFUN_LINEAR>(k, form);
+        case TVBG_CFUN_DIFF: return pick_k<TVBG_CFUN_DIFF>(k, form);
+        case TVBG_CFUN_SIGMOIDAL: return pick_k<TVBG_CFUN_SIGMOIDAL>(k, form);
         default: return nullptr;
     }
 }

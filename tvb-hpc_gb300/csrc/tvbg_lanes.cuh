@@ -33,15 +33,24 @@
 // block starts; with nh >= d_max + 1 + K no slot written in a block aliases
 // one read in it.  The cluster meets at one barrier per block.
 //
-// Gather.  Each thread sums its node's in-edges for the K steps of the
-// block: one edge record and one address per K steps, K sector loads per
-// edge (cache-global, __ldcg: with C > 1 the values come from other SMs,
-// ordered by the cluster barrier's release/acquire), 16 independent loads
-// in flight per thread.  The sums are parked in shared memory and the
-// node's K updates run from registers.  (Staging the edges' K-slot runs in
-// shared memory with cp.async.bulk instead was measured slower on the
-// benchmark workloads: the kernel is bound by instruction issue and latency,
-// not by bytes in flight.)
+// Gather.  The 8 lanes of a node slot sum its in-edges for the K steps of the
+// block: the K slots of an edge are one run of consecutive floats, split over
+// the lanes in 32-byte loads (gather_run), and the sums cross to their owners
+// through shared memory.  L2 serves such runs to one CTA of 512 threads per
+// SM at 20 TB/s from a 48 MB working set, 12.6 TB/s from 96 MB and 8.5 TB/s
+// from 192 MB; one float per lane and load reached 9.4, 7.2 and 6.1, two
+// 16-byte loads 32 bytes apart 10.6, 10.0 and 8.5.
+// (Staging the runs in shared memory with cp.async.bulk was measured slower;
+// a rolling window of loads or predicated loads inside the batch spill at
+// these register counts and were slower too.)
+//
+// What bounds it.  Per block of 8 steps, N = 84 on clusters of 2 CTAs (128
+// groups of MPR with noise): gather 8300-9000 cycles, update 4400, the CTA
+// barrier and phase handling under 700; before, two waits of 2300 cycles at
+// cluster barriers that also dropped the L1 lines of the edge records.
+// 128 groups x 84 nodes x 800 steps: 1.62 ms before, 0.89 now; 32 groups
+// on 6 CTAs each 0.674 -> 0.320; N = 192 (32 groups) 1.065 -> 0.55; N = 998
+// (2 groups) 1.284 -> 0.67.
 #pragma once
 
 #include "tvbg_step_blocked.cuh"
@@ -50,16 +59,15 @@ namespace tvbg {
 
 constexpr int kLanes = TVBG_GROUP_LANES;
 
-// steps of the pipelined kernel's update loop unrolled (update_node)
-#ifndef TVBG_UPDATE_UNROLL
-#define TVBG_UPDATE_UNROLL 1
-#endif
-constexpr int kUpdateUnroll = TVBG_UPDATE_UNROLL;
+// Steps of a whole block unrolled together (update_node).  Per block of 8 MPR
+// steps without noise (N = 84, 256 instances): rolled 3000 cycles, 2 at a
+// time 1440, 4 at a time 1290; 8 at a time spills and was slower.
+constexpr int kStepUnroll = 4;
 
-// 16-byte loads in flight per thread in the transposed gather (lane_gather_t)
-#ifndef TVBG_GATHER_LOADS
-#define TVBG_GATHER_LOADS 8
-#endif
+// Floats in flight per gather thread in a kernel built for CTAs of at most
+// `bound` threads: 128, 80 or 64 registers a thread for 512, 768 or 1024.
+__host__ __device__ constexpr int gather_floats(int bound) { return bound <= 512 ? 64 : 32; }
+
 
 __device__ __forceinline__ uint32_t cluster_nranks() {
     uint32_t n;
@@ -124,106 +132,131 @@ __device__ __forceinline__ float lane_post(float S, float xi, float wsum, float 
     }
 }
 
-// Coupling sums of node n (in-edges [lo, hi)) for the K steps of the block
-// starting at ring position tm, accumulated in CSR order.  U = 16 / K edges
-// per iteration: 16 independent sector loads in flight per thread.
-template <int CF, int K>
-__device__ __forceinline__ void lane_gather(const tvbg_group& g, int lo, int hi, uint32_t tm,
-                                            uint32_t mask, uint32_t R, int l, float acc[K]) {
-    constexpr int U = 16 / K;
-    const float* __restrict__ ring = g.ring + l;
-    const uint2* __restrict__ edges = reinterpret_cast<const uint2*>(g.edges);
+// W consecutive floats at p (W * 4-byte aligned) in one load, cached in L2
+// only: with a cluster the values come from other SMs.
+template <int W>
+__device__ __forceinline__ void ldcg_run(const float* p, float v[W]) {
+    if constexpr (W == 8) {
+        asm volatile("ld.global.cg.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                     : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]), "=f"(v[4]), "=f"(v[5]),
+                       "=f"(v[6]), "=f"(v[7])
+                     : "l"(p));
+    } else if constexpr (W == 4) {
+        const float4 q = __ldcg(reinterpret_cast<const float4*>(p));
+        v[0] = q.x;
+        v[1] = q.y;
+        v[2] = q.z;
+        v[3] = q.w;
+    } else if constexpr (W == 2) {
+        const float2 q = __ldcg(reinterpret_cast<const float2*>(p));
+        v[0] = q.x;
+        v[1] = q.y;
+    } else {
+        v[0] = __ldcg(p);
+    }
+}
+
+// Coupling sums of one node slot (deg in-edges at edges, shared or global
+// memory) for the K steps of the block at ring position tm.  The K slots an edge reads are one run of
+// 8 K NC consecutive floats (step-major, then channel, then instance), and
+// the 8 lanes of the slot split that run instead of each taking its own
+// instance: load j of lane l covers floats j 64 + l W .. + W - 1, so a warp
+// instruction moves whole 32-byte sectors, W floats per lane (W = 8: one
+// 32-byte load per edge and lane).  acc sums w_e pre(v_e) of its (step,
+// channel, instance) in CSR order, pairs of them in one packed FP32 FMA
+// (__ffma2_rn: each half rounded as fmaf).  The sums cross to their
+// owners through shared memory: cs_slot[(ch K + k) stride + m] holds step k
+// of instance m (the caller orders the reads after the writes).
+// VEC: run_vec holds (every ring of the Python layer); otherwise W scalar
+// loads and 64-bit indices.
+template <int CF, int K, int NC, bool VEC, int FLOATS>
+__device__ __forceinline__ void gather_run(const tvbg_group& g, const uint2* edges, int deg, uint32_t tm,
+                                           uint32_t mask, uint32_t R, int l, float* cs_slot, int stride) {
+    constexpr int F = K * NC;               // floats of a run per lane
+    constexpr int W = F < 8 ? F : 8;        // floats per load
+    constexpr int NJ = F / W;               // loads per edge and lane
+    constexpr int U = !VEC ? 1 : (FLOATS / F < 8 ? FLOATS / F : 8);  // edges in flight
+    const float* __restrict__ ring = g.ring + l * W;
+    float2 acc[NJ][(W + 1) / 2];
 #pragma unroll
-    for (int k = 0; k < K; ++k) acc[k] = 0.0f;
-    auto addr = [&](uint32_t pk) {
-        return ring + (static_cast<size_t>(pk >> 16) * R + ((tm + (pk & 0xffffu)) & mask)) * kLanes;
-    };
-    int e = lo;
-    for (; e + U <= hi; e += U) {
-        float v[U][K];
+    for (int j = 0; j < NJ; ++j)
+#pragma unroll
+        for (int i = 0; i < (W + 1) / 2; ++i) acc[j][i] = make_float2(0.0f, 0.0f);
+    // No branch inside a batch: the loads past the last edge repeat it and
+    // their products are dropped, so U ring loads leave back to back.
+    for (int e = 0; e < deg; e += U) {
+        float v[U][NJ][W];
         float w[U];
 #pragma unroll
         for (int u = 0; u < U; ++u) {
-            const uint2 ed = __ldg(edges + e + u);
-            const float* p = addr(ed.x);
+            const uint2 ed = edges[min(e + u, deg - 1)];
             w[u] = __uint_as_float(ed.y);
+            // the ring mask is below 2^16; N R < 2^32 where VEC (run_vec)
+            const uint32_t pos = (tm + ed.x) & mask;
+            const size_t row = VEC ? static_cast<size_t>((ed.x >> 16) * R + pos)
+                                   : static_cast<size_t>(ed.x >> 16) * R + pos;
+            const float* p = ring + row * (kLanes * NC);
 #pragma unroll
-            for (int k = 0; k < K; ++k) v[u][k] = __ldcg(p + k * kLanes);
+            for (int j = 0; j < NJ; ++j) {
+                if constexpr (VEC) {
+                    ldcg_run<W>(p + 64 * j, v[u][j]);
+                } else {
+#pragma unroll
+                    for (int i = 0; i < W; ++i) ldcg_run<1>(p + 64 * j + i, &v[u][j][i]);
+                }
+            }
         }
 #pragma unroll
         for (int u = 0; u < U; ++u) {
+            if (e + u < deg) {
+                const float2 ww = make_float2(w[u], w[u]);
 #pragma unroll
-            for (int k = 0; k < K; ++k) acc[k] = fmaf(w[u], lane_pre<CF>(v[u][k], g.cf_p), acc[k]);
+                for (int j = 0; j < NJ; ++j) {
+                    if constexpr (W == 1) {
+                        acc[j][0].x = fmaf(w[u], lane_pre<CF>(v[u][j][0], g.cf_p), acc[j][0].x);
+                    } else {
+#pragma unroll
+                        for (int i = 0; i < W / 2; ++i)
+                            acc[j][i] = __ffma2_rn(ww,
+                                                   make_float2(lane_pre<CF>(v[u][j][2 * i], g.cf_p),
+                                                               lane_pre<CF>(v[u][j][2 * i + 1], g.cf_p)),
+                                                   acc[j][i]);
+                    }
+                }
+            }
         }
     }
-    if (e < hi) {  // fewer than U edges left, loads still issued together
-        float v[U][K];
-        float w[U];
 #pragma unroll
-        for (int u = 0; u < U; ++u) {
-            if (e + u < hi) {
-                const uint2 ed = __ldg(edges + e + u);
-                const float* p = addr(ed.x);
-                w[u] = __uint_as_float(ed.y);
+    for (int j = 0; j < NJ; ++j) {
+        const int o = 64 * j + l * W;   // first float of this lane's part of the run
+        float* dst = cs_slot + (((o / kLanes) % NC) * K + o / (kLanes * NC)) * stride + o % kLanes;
+        if constexpr (W >= 4) {
 #pragma unroll
-                for (int k = 0; k < K; ++k) v[u][k] = __ldcg(p + k * kLanes);
-            }
-        }
-#pragma unroll
-        for (int u = 0; u < U; ++u) {
-            if (e + u < hi) {
-#pragma unroll
-                for (int k = 0; k < K; ++k) acc[k] = fmaf(w[u], lane_pre<CF>(v[u][k], g.cf_p), acc[k]);
-            }
+            for (int i = 0; i < W / 4; ++i)
+                reinterpret_cast<float4*>(dst)[i] = make_float4(acc[j][2 * i].x, acc[j][2 * i].y,
+                                                                acc[j][2 * i + 1].x, acc[j][2 * i + 1].y);
+        } else if constexpr (W == 2) {
+            *reinterpret_cast<float2*>(dst) = acc[j][0];
+        } else {
+            dst[0] = acc[j][0].x;
         }
     }
 }
 
-// Kuramoto coupling, sum_e w_e sin(x_j - x_i) = cos x_i sum_e w_e sin x_j
-// - sin x_i sum_e w_e cos x_j: the ring carries two channels, sin and cos
-// of the observable ([N][R][2][8]), and the gather sums both for the K steps
-// (16 independent loads in flight per thread, CSR order).
-template <int K>
-__device__ __forceinline__ void lane_gather_sc(const tvbg_group& g, int lo, int hi, uint32_t tm,
-                                               uint32_t mask, uint32_t R, int l, float accs[K],
-                                               float accc[K]) {
-    constexpr int RL = 2 * kLanes;
-    constexpr int U = 8 / K;
-    const float* __restrict__ ring = g.ring + l;
-    const uint2* __restrict__ edges = reinterpret_cast<const uint2*>(g.edges);
-#pragma unroll
-    for (int k = 0; k < K; ++k) accs[k] = accc[k] = 0.0f;
-    auto addr = [&](uint32_t pk) {
-        return ring + (static_cast<size_t>(pk >> 16) * R + ((tm + (pk & 0xffffu)) & mask)) * RL;
-    };
-    int e = lo;
-    for (; e < hi; e += U) {
-        float vs[U][K], vc[U][K];
-        float w[U];
-#pragma unroll
-        for (int u = 0; u < U; ++u) {
-            if (e + u < hi) {
-                const uint2 ed = __ldg(edges + e + u);
-                const float* p = addr(ed.x);
-                w[u] = __uint_as_float(ed.y);
-#pragma unroll
-                for (int k = 0; k < K; ++k) {
-                    vs[u][k] = __ldcg(p + k * RL);
-                    vc[u][k] = __ldcg(p + k * RL + kLanes);
-                }
-            }
-        }
-#pragma unroll
-        for (int u = 0; u < U; ++u) {
-            if (e + u < hi) {
-#pragma unroll
-                for (int k = 0; k < K; ++k) {
-                    accs[k] = fmaf(w[u], vs[u][k], accs[k]);
-                    accc[k] = fmaf(w[u], vc[u][k], accc[k]);
-                }
-            }
-        }
-    }
+// gather_run for a ring of any alignment, out of line: its registers stay
+// out of the callers' loops.
+template <int CF, int K, int NC>
+__device__ __noinline__ void gather_run_any(const tvbg_group& g, const uint2* edges, int deg, uint32_t tm,
+                                            uint32_t mask, uint32_t R, int l, float* cs_slot, int stride) {
+    gather_run<CF, K, NC, false, 16>(g, edges, deg, tm, mask, R, l, cs_slot, stride);
+}
+
+// Whether a ring takes gather_run's vector loads and 32-bit row indices.
+template <int K, int NC>
+__device__ __forceinline__ bool run_vec(const float* ring, int N, uint32_t R) {
+    constexpr uint32_t align = K * NC < 8 ? 4u * K * NC : 32u;
+    return (reinterpret_cast<uintptr_t>(ring) & (align - 1u)) == 0 &&
+           static_cast<unsigned long long>(N) * R <= 0xffffffffull;
 }
 
 // Ring channels per (node, slot): 2 (sin, cos) for the Kuramoto coupling and
@@ -245,337 +278,18 @@ __device__ __forceinline__ float ring_val(float o, const float* p) {
     }
 }
 
+// Static shared memory of a group CTA, at most (the descriptor, the edge
+// offsets and the cluster phases).
+constexpr size_t kGroupStaticBytes = sizeof(tvbg_group) + 640;
+
+// Bytes of staged edge records for node slots of `threads` lanes.
+constexpr int kStageEdges = 48;
+__host__ __device__ constexpr int stage_bytes(int threads) { return threads / kLanes * kStageEdges * 8; }
+
 // Dynamic shared memory of a group CTA: the K coupling sums (per ring
-// channel) of every thread.
+// channel) of every thread, and the staged edge records.
 __host__ __device__ constexpr uint32_t group_smem_bytes(int K, int threads, int nc) {
-    return static_cast<uint32_t>(4 * K * threads * nc);
-}
-
-template <class M, int CF, int K>
-__device__ __forceinline__ void run_group(const tvbg_group& g, float* csum, int32_t* status) {
-    constexpr int NS = M::NS;
-    constexpr int NP = M::NP;
-    constexpr int SPC = Noise<M>::SPC;
-    constexpr int NC = ring_channels<CF>();
-    constexpr int RL = kLanes * NC;  // floats per (node, slot)
-    const int N = g.N;
-    const uint32_t C = cluster_nranks();
-    const uint32_t rank = cluster_rank();
-    const bool cluster = C > 1;
-    if (N <= 0 || N > 65535 || g.lognh < 3 || g.lognh > 16 || g.model != M::ID || g.cfun != CF ||
-        g.nsteps < 0 || (g.flags & (TVBG_F_TRACKA | TVBG_F_MIDSYNC | TVBG_F_TRACE_CSUM)) ||
-        (!Noise<M>::kOK && !WideNoise<M>::value && (g.flags & TVBG_F_NOISE))) {
-        if (threadIdx.x == 0) report(status, TVBG_EINVAL);
-        return;  // every CTA of the cluster reads the same descriptor and leaves here
-    }
-    const int l = threadIdx.x % kLanes;
-    const int slot = threadIdx.x / kLanes;
-    const int P = blockDim.x / kLanes;
-    const int stride = static_cast<int>(C) * P;
-    const int rounds = (N + stride - 1) / stride;       // warp-uniform node loop
-    const uint32_t nh = 1u << g.lognh;
-    const uint32_t mask = nh - 1u;
-    const uint32_t R = nh + kGhost;
-    const uint32_t flags = g.flags;
-    const bool noise = (flags & TVBG_F_NOISE) != 0;
-    const bool bold = (flags & TVBG_F_BOLD) != 0 && g.bold != nullptr && g.bold_out != nullptr;
-    const bool trace = (flags & TVBG_F_TRACE) != 0 && g.trace != nullptr;
-    const float dt = g.dt, sqrt_dt = g.sqrt_dt;
-    const float cf_a = g.lanes[l].cf_a;
-    const int my_steps = g.lanes[l].nsteps < g.nsteps ? g.lanes[l].nsteps : g.nsteps;
-    const uint32_t inst_id = g.lanes[l].inst_id;
-    const long long t0 = g.t0;
-    const long long t_end = t0 + my_steps;  // this lane updates while t < t_end
-    float* __restrict__ ring = g.ring;
-    float* __restrict__ state = g.state;
-    const int q0 = slot * static_cast<int>(C) + static_cast<int>(rank);
-
-    // seed: slot t0 holds obs0 of the state at t0
-    {
-        const uint32_t pos = static_cast<uint32_t>(t0) & mask;
-        for (int q = q0; q < N; q += stride) {
-            const int n = g.nodes ? __ldg(g.nodes + q) : q;
-            float x[NS];
-#pragma unroll
-            for (int v = 0; v < NS; ++v) x[v] = state[(n * NS + v) * kLanes + l];
-            const size_t idx = (static_cast<size_t>(n) * R + pos) * RL + l;
-            const float o = M::obs(x, 0);
-            float p[NP];
-#pragma unroll
-            for (int v = 0; v < NP; ++v) p[v] = __ldg(g.nparam + (n * NP + v) * kLanes + l);
-            if constexpr (NC == 2) {
-                float sn, cs;
-                if constexpr (CF == TVBG_CFUN_LEMS_2) {
-                    sn = M::ring_value(o, p);
-                    cs = M::ring_value2(x[M::CVAR2], p);
-                } else {
-                    sincosf(o, &sn, &cs);
-                }
-                ring[idx] = sn;
-                ring[idx + kLanes] = cs;
-                if (pos < kGhost) {
-                    ring[idx + static_cast<size_t>(nh) * RL] = sn;
-                    ring[idx + static_cast<size_t>(nh) * RL + kLanes] = cs;
-                }
-            } else {
-                const float rv = ring_val<M, CF>(o, p);
-                ring[idx] = rv;
-                if (pos < kGhost) ring[idx + static_cast<size_t>(nh) * kLanes] = rv;
-            }
-        }
-    }
-    group_barrier(cluster);
-
-    // monitor schedule as 32-bit counters carried across blocks (the 64-bit
-    // divisions run once per kernel): BOLD sample after step t when
-    // (t + 1) % bold_period == 0, trace row before step t when
-    // t % trace_every == 0
-    const int bper = g.bold_period > 0 ? g.bold_period : 1;
-    const int tev = g.trace_every > 0 ? g.trace_every : 1;
-    int b_until = bold ? static_cast<int>((bper - 1) - t0 % bper) : 0;  // steps to the next sample
-    int b_row = bold ? static_cast<int>((t0 + b_until + 1) / bper - 1) : 0;
-    int tr_until = trace ? static_cast<int>((tev - t0 % tev) % tev) : 0;
-    int tr_row = trace ? static_cast<int>(((t0 + tr_until) / tev) % g.trace_len) : 0;
-    for (long long tb = t0; tb < t0 + g.nsteps; tb += K) {
-        const int cnt = (t0 + g.nsteps - tb) < K ? static_cast<int>(t0 + g.nsteps - tb) : K;
-        const uint32_t tm = static_cast<uint32_t>(tb) & mask;
-        for (int r = 0; r < rounds; ++r) {
-            const int q = q0 + r * stride;
-            const bool valid = q < N;
-            const int n = valid ? (g.nodes ? __ldg(g.nodes + q) : q) : 0;
-            {
-                const int lo = valid ? __ldg(g.row + n) : 0;
-                const int hi = valid ? __ldg(g.row + n + 1) : 0;
-                if constexpr (NC == 2) {
-                    float accs[K], accc[K];
-                    lane_gather_sc<K>(g, lo, hi, tm, mask, R, l, accs, accc);
-#pragma unroll
-                    for (int k = 0; k < K; ++k) {
-                        csum[k * blockDim.x + threadIdx.x] = accs[k];
-                        csum[(K + k) * blockDim.x + threadIdx.x] = accc[k];
-                    }
-                } else {
-                    float acc[K];
-                    lane_gather<CF, K>(g, lo, hi, tm, mask, R, l, acc);
-#pragma unroll
-                    for (int k = 0; k < K; ++k) csum[k * blockDim.x + threadIdx.x] = acc[k];
-                }
-            }
-            if (!valid) continue;
-            float x[NS], p[NP];
-#pragma unroll
-            for (int v = 0; v < NS; ++v) x[v] = state[(n * NS + v) * kLanes + l];
-#pragma unroll
-            for (int v = 0; v < NP; ++v) p[v] = __ldg(g.nparam + (n * NP + v) * kLanes + l);
-            const float wsum = (CF == TVBG_CFUN_DIFF && g.wsum) ? __ldg(g.wsum + n) : 0.0f;
-            float bs = 0.0f, bF = 0.0f, bV = 0.0f, bQ = 0.0f;
-            if (bold) {
-                bs = g.bold[(0 * N + n) * kLanes + l];
-                bF = g.bold[(1 * N + n) * kLanes + l];
-                bV = g.bold[(2 * N + n) * kLanes + l];
-                bQ = g.bold[(3 * N + n) * kLanes + l];
-            }
-            float obs0 = M::obs(x, 0);
-            float sn0 = 0.0f, cs0 = 0.0f;  // sin, cos of obs0 (Kuramoto coupling)
-            if constexpr (NC == 2 && CF != TVBG_CFUN_LEMS_2) sincosf(obs0, &sn0, &cs0);
-            float zz[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-            int b_next = b_until, tr_next = tr_until;
-            int brow = b_row, trow = tr_row;
-#pragma unroll 1
-            for (int k = 0; k < cnt; ++k) {
-                const long long t = tb + k;
-                if (t >= t_end) break;
-                if (trace && k == tr_next) {
-                    float* dst = g.trace + ((static_cast<size_t>(trow) * N + n) * g.trace_nobs) * kLanes + l;
-                    for (int o = 0; o < g.trace_nobs; ++o) dst[o * kLanes] = M::obs(x, o);
-                    tr_next += tev;
-                    trow = trow + 1 == g.trace_len ? 0 : trow + 1;
-                }
-                const float xbold = bold ? M::obs(x, g.bold_obs) : 0.0f;
-                float c, c2 = 0.0f;
-                if constexpr (CF == TVBG_CFUN_LEMS_2) {
-                    c = M::coupling(csum[k * blockDim.x + threadIdx.x], x, p);
-                    c2 = M::coupling2(csum[(K + k) * blockDim.x + threadIdx.x], x, p);
-                } else if constexpr (NC == 2) {
-                    // sum_e w sin(x_j - x_i); Kuramoto: post = a * mean (coupling.py:119-121)
-                    const float S = cs0 * csum[k * blockDim.x + threadIdx.x] -
-                                    sn0 * csum[(K + k) * blockDim.x + threadIdx.x];
-                    if constexpr (CF == TVBG_CFUN_LEMS_SC) {
-                        c = M::coupling(S, x, p);
-                    } else {
-                        c = cf_a * (S / static_cast<float>(N));
-                    }
-                } else if constexpr (CF == TVBG_CFUN_LEMS) {
-                    c = M::coupling(csum[k * blockDim.x + threadIdx.x], x, p);
-                } else {
-                    c = lane_post<CF>(csum[k * blockDim.x + threadIdx.x], obs0, wsum, cf_a, g.cf_b);
-                }
-                float f[NS];
-                if constexpr (CF == TVBG_CFUN_LEMS_2) {
-                    M::drift2(x, c, c2, p, g.consts, f);
-                } else {
-                    M::drift(x, c, p, g.consts, f);
-                }
-#pragma unroll
-                for (int v = 0; v < NS; ++v) x[v] = fmaf(dt, f[v], x[v]);
-                if constexpr (Noise<M>::kOK) {
-                    if (noise) {
-                        const int r0 = static_cast<int>(t & (SPC - 1));
-                        if (k == 0 || r0 == 0) {
-                            const u32x4 w = philox4x32_10(static_cast<uint32_t>(n),
-                                                          static_cast<uint32_t>(t / SPC), g.seed_hi, 0u,
-                                                          g.seed_lo, inst_id);
-                            box_muller_fast(w.v[0], w.v[1], zz[0], zz[1]);
-                            box_muller_fast(w.v[2], w.v[3], zz[2], zz[3]);
-                        }
-#pragma unroll
-                        for (int v = 0; v < NS; ++v)
-                            x[v] = fmaf(sqrt_dt * pick4(zz, r0 * NS + v), g.sigma[v], x[v]);
-                    }
-                } else if constexpr (WideNoise<M>::value) {
-                    if (noise) {
-                        float z8[8];
-#pragma unroll
-                        for (int b = 0; b < 2; ++b) {
-                            const u32x4 w = philox4x32_10(static_cast<uint32_t>(n),
-                                                          static_cast<uint32_t>(t), g.seed_hi,
-                                                          static_cast<uint32_t>(b), g.seed_lo, inst_id);
-                            box_muller_fast(w.v[0], w.v[1], z8[4 * b], z8[4 * b + 1]);
-                            box_muller_fast(w.v[2], w.v[3], z8[4 * b + 2], z8[4 * b + 3]);
-                        }
-#pragma unroll
-                        for (int v = 0; v < NS; ++v)
-                            x[v] = fmaf(sqrt_dt * z8[v], g.sigma[0] * NoiseScale<M>::at(v), x[v]);
-                    }
-                }
-                M::limit(x, flags);
-                obs0 = M::obs(x, 0);
-                const uint32_t pos = (static_cast<uint32_t>(t) + 1u) & mask;
-                const size_t idx = (static_cast<size_t>(n) * R + pos) * RL + l;
-                if constexpr (NC == 2) {
-                    if constexpr (CF == TVBG_CFUN_LEMS_2) {
-                        sn0 = M::ring_value(obs0, p);
-                        cs0 = M::ring_value2(x[M::CVAR2], p);
-                    } else {
-                        sincosf(obs0, &sn0, &cs0);
-                    }
-                    ring[idx] = sn0;
-                    ring[idx + kLanes] = cs0;
-                    if (pos < kGhost) {
-                        ring[idx + static_cast<size_t>(nh) * RL] = sn0;
-                        ring[idx + static_cast<size_t>(nh) * RL + kLanes] = cs0;
-                    }
-                } else {
-                    const float rv = ring_val<M, CF>(obs0, p);
-                    ring[idx] = rv;
-                    if (pos < kGhost) ring[idx + static_cast<size_t>(nh) * kLanes] = rv;
-                }
-                if (bold) {
-                    Balloon::step(bs, bF, bV, bQ, xbold, g.dt_bold);
-                    if (k == b_next) {
-                        if (brow >= 0 && brow < g.bold_len)
-                            g.bold_out[(static_cast<size_t>(brow) * N + n) * kLanes + l] =
-                                Balloon::signal(bV, bQ);
-                        b_next += bper;
-                        brow += 1;
-                    }
-                }
-            }
-#pragma unroll
-            for (int v = 0; v < NS; ++v) state[(n * NS + v) * kLanes + l] = x[v];
-            if (bold) {
-                g.bold[(0 * N + n) * kLanes + l] = bs;
-                g.bold[(1 * N + n) * kLanes + l] = bF;
-                g.bold[(2 * N + n) * kLanes + l] = bV;
-                g.bold[(3 * N + n) * kLanes + l] = bQ;
-            }
-        }
-        // advance the monitor counters past this block
-        if (bold) {
-            while (b_until < cnt) {
-                b_until += bper;
-                b_row += 1;
-            }
-            b_until -= cnt;
-        }
-        if (trace) {
-            while (tr_until < cnt) {
-                tr_until += tev;
-                tr_row = tr_row + 1 == g.trace_len ? 0 : tr_row + 1;
-            }
-            tr_until -= cnt;
-        }
-        group_barrier(cluster);
-    }
-}
-
-// ---------------------------------------------------------------------------
-// Pipelined group kernel (group_kernel_pipelined).  The per-node pieces of
-// run_group as functions; run_group itself keeps its own inline body (its
-// register allocation and instruction schedule were tuned as written).
-// ---------------------------------------------------------------------------
-
-// Transposed gather of one node for the K steps of the block at ring
-// position tm.  The 8 lanes of a node slot share the edge records; lane l
-// reads, per edge, ring position t + (l mod K) for NI = 64 / K consecutive
-// instances m0 = (l / K) NI .. m0 + NI - 1 -- 4 NI contiguous bytes, two
-// (K = 8) or one (K = 4) 16-byte loads -- and accumulates, in CSR order,
-// acc[i] = sum_e w_e pre(v_e[m0 + i]), the sum of step (l mod K) of
-// instance m0 + i.  Pairs of accumulators take one packed FP32 FMA
-// (__ffma2_rn: each half rounded as fmaf), so every sum equals
-// lane_gather's.  The sums are written transposed: cs_slot[k * stride + m]
-// holds step k of instance m, where the node's lane m reads them.  Needs the
-// ring 16-byte aligned and K in {4, 8}.
-template <int CF, int K>
-__device__ __forceinline__ void lane_gather_t(const tvbg_group& g, int lo, int hi, uint32_t tm,
-                                              uint32_t mask, uint32_t R, int l, float* cs_slot,
-                                              int stride) {
-    static_assert(K == 4 || K == 8, "transposed gather: K = 4 or 8");
-    constexpr int NI = K == 8 ? 8 : 4;   // instances per lane
-    constexpr int NV = NI / 4;           // 16-byte loads per edge
-    constexpr int U = TVBG_GATHER_LOADS / NV;  // edges per iteration (loads in flight / loads per edge)
-    const int ks = l % K;
-    const int m0 = (l / K) * NI;
-    const float* __restrict__ ring = g.ring + m0;
-    const uint2* __restrict__ edges = reinterpret_cast<const uint2*>(g.edges);
-    float2 acc[NI / 2];
-#pragma unroll
-    for (int i = 0; i < NI / 2; ++i) acc[i] = make_float2(0.0f, 0.0f);
-    auto addr = [&](uint32_t pk) {
-        return ring + (static_cast<size_t>(pk >> 16) * R + (((tm + (pk & 0xffffu)) & mask) + ks)) * kLanes;
-    };
-    for (int e = lo; e < hi; e += U) {
-        float4 v[U][NV];
-        float w[U];
-#pragma unroll
-        for (int u = 0; u < U; ++u) {
-            if (e + u < hi) {
-                const uint2 ed = __ldg(edges + e + u);
-                const float4* p = reinterpret_cast<const float4*>(addr(ed.x));
-                w[u] = __uint_as_float(ed.y);
-#pragma unroll
-                for (int j = 0; j < NV; ++j) v[u][j] = __ldcg(p + j);
-            }
-        }
-#pragma unroll
-        for (int u = 0; u < U; ++u) {
-            if (e + u < hi) {
-                const float2 ww = make_float2(w[u], w[u]);
-#pragma unroll
-                for (int j = 0; j < NV; ++j) {
-                    const float2 a = make_float2(lane_pre<CF>(v[u][j].x, g.cf_p), lane_pre<CF>(v[u][j].y, g.cf_p));
-                    const float2 b = make_float2(lane_pre<CF>(v[u][j].z, g.cf_p), lane_pre<CF>(v[u][j].w, g.cf_p));
-                    acc[2 * j] = __ffma2_rn(ww, a, acc[2 * j]);
-                    acc[2 * j + 1] = __ffma2_rn(ww, b, acc[2 * j + 1]);
-                }
-            }
-        }
-    }
-#pragma unroll
-    for (int i = 0; i < NI / 2; ++i) {
-        cs_slot[ks * stride + m0 + 2 * i] = acc[i].x;
-        cs_slot[ks * stride + m0 + 2 * i + 1] = acc[i].y;
-    }
+    return static_cast<uint32_t>(4 * K * threads * nc + stage_bytes(threads));
 }
 
 // Per-thread constants of a group run (lane l of one node slot).
@@ -584,6 +298,7 @@ struct GroupLane {
     uint32_t nh, mask, R;   // ring length, mask, row length (nh + ghost slots)
     uint32_t flags;
     bool noise, bold, trace;
+    bool vec;               // ring aligned for gather_run's vector loads
     float cf_a;
     long long t0, t_end;    // this lane updates while t < t_end
     uint32_t inst_id;
@@ -601,7 +316,7 @@ __device__ __forceinline__ bool group_descriptor_ok(const tvbg_group& g, bool al
              (!Noise<M>::kOK && !WideNoise<M>::value && (g.flags & TVBG_F_NOISE)));
 }
 
-template <class M>
+template <class M, int CF, int K>
 __device__ __forceinline__ GroupLane make_lane(const tvbg_group& g, int l) {
     GroupLane c;
     c.l = l;
@@ -612,6 +327,7 @@ __device__ __forceinline__ GroupLane make_lane(const tvbg_group& g, int l) {
     c.noise = (g.flags & TVBG_F_NOISE) != 0;
     c.bold = (g.flags & TVBG_F_BOLD) != 0 && g.bold != nullptr && g.bold_out != nullptr;
     c.trace = (g.flags & TVBG_F_TRACE) != 0 && g.trace != nullptr;
+    c.vec = run_vec<K, ring_channels<CF>()>(g.ring, g.N, c.R);
     c.cf_a = g.lanes[l].cf_a;
     const int my_steps = g.lanes[l].nsteps < g.nsteps ? g.lanes[l].nsteps : g.nsteps;
     c.inst_id = g.lanes[l].inst_id;
@@ -660,28 +376,64 @@ __device__ __forceinline__ void seed_node(const tvbg_group& g, const GroupLane& 
     }
 }
 
-// Coupling sums of node n (an invalid slot gathers nothing) for the K steps
-// of the block at ring position tm, written to cs[k * stride] (and
-// cs[(K + k) * stride] for the second ring channel); cs points at this
-// thread's own sums.  One-channel couplings take the transposed gather (the
-// caller has checked the ring's 16-byte alignment).
-template <class M, int CF, int K>
-__device__ __forceinline__ void gather_node(const tvbg_group& g, const GroupLane& c, bool valid, int n,
-                                            uint32_t tm, float* cs, int stride) {
+// Coupling sums of a node slot's node (degree 0: none) for the K steps of
+// the block at ring position tm; edges, cs_slot and stride as gather_run's.
+template <class M, int CF, int K, int BOUND>
+__device__ __forceinline__ void gather_node(const tvbg_group& g, const GroupLane& c, const uint2* edges, int deg,
+                                            uint32_t tm, float* cs_slot, int stride) {
     constexpr int NC = ring_channels<CF>();
-    const int lo = valid ? __ldg(g.row + n) : 0;
-    const int hi = valid ? __ldg(g.row + n + 1) : 0;
-    if constexpr (NC == 2) {
-        float accs[K], accc[K];
-        lane_gather_sc<K>(g, lo, hi, tm, c.mask, c.R, c.l, accs, accc);
+    if (c.vec)
+        gather_run<CF, K, NC, true, gather_floats(BOUND)>(g, edges, deg, tm, c.mask, c.R, c.l, cs_slot, stride);
+    else
+        gather_run_any<CF, K, NC>(g, edges, deg, tm, c.mask, c.R, c.l, cs_slot, stride);
+}
+
+// In-edge records of the CTA's node slots, staged in shared memory for the
+// whole run.  The acquire side of each block's barrier drops the L1 cache,
+// so records read from global memory would come from L2 again in every
+// block, in front of the ring reads that need them (measured per block at
+// N = 84: 1090 cycles for each four edges, L2's own latency being 290-440).
+// `records` holds kStageEdges per slot on average; a CTA with more edges
+// than that reads them from global memory.
+struct EdgeStage {
+    int off[129];   // first record of each node slot (at most 128 slots)
+};
+
+// All threads of the CTA; threads [0, 8 P) are the lanes of the P slots,
+// with the degree deg of their slot's node and its first edge lo.  Returns
+// the slot's records (valid for threads < 8 P).  Ends with a barrier.
+__device__ __forceinline__ const uint2* stage_edges(const tvbg_group& g, EdgeStage& st, uint2* records, int P,
+                                                    int tid, int lo, int deg) {
+    const int slot = tid / kLanes, l = tid % kLanes;
+    if (slot < P && l == 0) st.off[slot + 1] = deg;
+    __syncthreads();
+    if (tid < 32) {  // exclusive scan of at most 128 degrees by one warp
+        int base = 0;
+        for (int i = 0; i < P; i += 32) {
+            int v = i + tid < P ? st.off[i + tid + 1] : 0;
 #pragma unroll
-        for (int k = 0; k < K; ++k) {
-            cs[k * stride] = accs[k];
-            cs[(K + k) * stride] = accc[k];
+            for (int d = 1; d < 32; d <<= 1) {
+                const int o = __shfl_up_sync(kFullMask, v, d);
+                if (tid >= d) v += o;
+            }
+            __syncwarp();
+            if (i + tid < P) st.off[i + tid + 1] = base + v;
+            base += __shfl_sync(kFullMask, v, 31);
         }
-    } else {
-        lane_gather_t<CF, K>(g, lo, hi, tm, c.mask, c.R, c.l, cs - c.l, stride);
+        if (tid == 0) st.off[0] = 0;
     }
+    __syncthreads();
+    const uint2* src = reinterpret_cast<const uint2*>(g.edges) + lo;
+    const uint2* out = src;
+    if (st.off[P] <= P * kStageEdges) {
+        if (slot < P) {
+            uint2* dst = records + st.off[slot];
+            for (int e = l; e < deg; e += kLanes) dst[e] = __ldg(src + e);
+            out = dst;
+        }
+        __syncthreads();
+    }
+    return out;
 }
 
 // Monitor schedule as 32-bit counters carried across blocks (the 64-bit
@@ -720,169 +472,342 @@ struct MonitorClock {
     }
 };
 
+template <bool B>
+struct Flag {
+    static constexpr bool value = B;
+};
+
+// State, parameters and monitor state of one (node, instance), in registers.
+template <class M, int CF>
+struct NodeRegs {
+    static constexpr int NS = M::NS;
+    static constexpr int NP = M::NP;
+    float x[NS], p[NP];
+    float wsum;
+    float bs, bF, bV, bQ;    // balloon (with BOLD)
+
+    __device__ __forceinline__ void load(const tvbg_group& g, const GroupLane& c, int n) {
+        const int l = c.l, N = g.N;
+#pragma unroll
+        for (int v = 0; v < NS; ++v) x[v] = g.state[(n * NS + v) * kLanes + l];
+#pragma unroll
+        for (int v = 0; v < NP; ++v) p[v] = __ldg(g.nparam + (n * NP + v) * kLanes + l);
+        wsum = (CF == TVBG_CFUN_DIFF && g.wsum) ? __ldg(g.wsum + n) : 0.0f;
+        bs = bF = bV = bQ = 0.0f;
+        if (c.bold) {
+            bs = g.bold[(0 * N + n) * kLanes + l];
+            bF = g.bold[(1 * N + n) * kLanes + l];
+            bV = g.bold[(2 * N + n) * kLanes + l];
+            bQ = g.bold[(3 * N + n) * kLanes + l];
+        }
+    }
+    __device__ __forceinline__ void store(const tvbg_group& g, const GroupLane& c, int n) const {
+        const int l = c.l, N = g.N;
+#pragma unroll
+        for (int v = 0; v < NS; ++v) g.state[(n * NS + v) * kLanes + l] = x[v];
+        if (c.bold) {
+            g.bold[(0 * N + n) * kLanes + l] = bs;
+            g.bold[(1 * N + n) * kLanes + l] = bF;
+            g.bold[(2 * N + n) * kLanes + l] = bV;
+            g.bold[(3 * N + n) * kLanes + l] = bQ;
+        }
+    }
+};
+
 // The cnt (<= K) updates of node n for the block starting at step tb, from
 // the coupling sums cs[k * stride] (second channel cs[(K + k) * stride]):
-// drift, Euler-Maruyama, limit, ring write, balloon/BOLD and trace -- the
-// update of run_group, in the same order.
+// drift, Euler-Maruyama, limit, ring write, balloon/BOLD and trace.
 template <class M, int CF, int K>
-__device__ __forceinline__ void update_node(const tvbg_group& g, const GroupLane& c, int n, long long tb,
-                                            int cnt, const float* cs, int stride, const MonitorClock& mc) {
+__device__ __forceinline__ void update_node(const tvbg_group& g, const GroupLane& c, NodeRegs<M, CF>& r, int n,
+                                            long long tb, int cnt, const float* cs, int stride,
+                                            const MonitorClock& mc) {
     constexpr int NS = M::NS;
-    constexpr int NP = M::NP;
     constexpr int SPC = Noise<M>::SPC;
     constexpr int NC = ring_channels<CF>();
     constexpr int RL = kLanes * NC;  // floats per (node, slot)
     const int N = g.N;
     const int l = c.l;
-    const uint32_t mask = c.mask, R = c.R, nh = c.nh;
+    const uint32_t mask = c.mask, nh = c.nh;
     const bool noise = c.noise, bold = c.bold, trace = c.trace;
     const float dt = g.dt, sqrt_dt = g.sqrt_dt;
-    float* __restrict__ ring = g.ring;
-    float* __restrict__ state = g.state;
-    float x[NS], p[NP];
+    float* __restrict__ ring = g.ring + static_cast<size_t>(n) * c.R * RL + l;  // this node's row
+    // the record lives in shared memory, which the compiler must take to be
+    // written by the ring stores: what every step reads is copied here, so
+    // expressions of the constants are evaluated once per block
+    float Kc[16];
 #pragma unroll
-    for (int v = 0; v < NS; ++v) x[v] = state[(n * NS + v) * kLanes + l];
+    for (int v = 0; v < 16; ++v) Kc[v] = g.consts[v];
+    float sig[4];
 #pragma unroll
-    for (int v = 0; v < NP; ++v) p[v] = __ldg(g.nparam + (n * NP + v) * kLanes + l);
-    const float wsum = (CF == TVBG_CFUN_DIFF && g.wsum) ? __ldg(g.wsum + n) : 0.0f;
-    float bs = 0.0f, bF = 0.0f, bV = 0.0f, bQ = 0.0f;
-    if (bold) {
-        bs = g.bold[(0 * N + n) * kLanes + l];
-        bF = g.bold[(1 * N + n) * kLanes + l];
-        bV = g.bold[(2 * N + n) * kLanes + l];
-        bQ = g.bold[(3 * N + n) * kLanes + l];
-    }
-    float obs0 = M::obs(x, 0);
+    for (int v = 0; v < 4; ++v) sig[v] = g.sigma[v];
+    const float cf_b = g.cf_b, dt_bold = g.dt_bold;
+    const int bold_obs = g.bold_obs;
+    const uint32_t seed_lo = g.seed_lo, seed_hi = g.seed_hi;
+    float obs0 = M::obs(r.x, 0);
     float sn0 = 0.0f, cs0 = 0.0f;  // sin, cos of obs0 (Kuramoto coupling)
     if constexpr (NC == 2 && CF != TVBG_CFUN_LEMS_2) sincosf(obs0, &sn0, &cs0);
     float zz[4] = {0.0f, 0.0f, 0.0f, 0.0f};
     int b_next = mc.b_until, tr_next = mc.tr_until;
     int brow = mc.b_row, trow = mc.tr_row;
-#pragma unroll kUpdateUnroll
-    for (int k = 0; k < cnt; ++k) {
+    const int kend = c.t_end - tb < cnt ? static_cast<int>(c.t_end - tb) : cnt;  // this lane's steps
+    // one step; MON: trace and BOLD may be on; ALIGNED: tb % SPC == 0, so the
+    // step's place in its Philox call is k % SPC
+    auto step = [&](int k, auto mon, auto aligned) {
+        constexpr bool MON = decltype(mon)::value, ALIGNED = decltype(aligned)::value;
+
         const long long t = tb + k;
-        if (t >= c.t_end) break;
-        if (trace && k == tr_next) {
+        if (MON && trace && k == tr_next) {
             // a trace row holds the observables, then with TVBG_F_TRACE_CSUM
             // the raw coupling sum of the step (one-channel couplings)
             const bool csum = (c.flags & TVBG_F_TRACE_CSUM) != 0;
             const int tw = g.trace_nobs + (csum ? 1 : 0);
             float* dst = g.trace + ((static_cast<size_t>(trow) * N + n) * tw) * kLanes + l;
-            for (int o = 0; o < g.trace_nobs; ++o) dst[o * kLanes] = M::obs(x, o);
+            for (int o = 0; o < g.trace_nobs; ++o) dst[o * kLanes] = M::obs(r.x, o);
             if constexpr (NC == 1) {
                 if (csum) dst[g.trace_nobs * kLanes] = cs[k * stride];
             }
             tr_next += mc.tev;
             trow = trow + 1 == g.trace_len ? 0 : trow + 1;
         }
-        const float xbold = bold ? M::obs(x, g.bold_obs) : 0.0f;
+        const float xbold = (MON && bold) ? M::obs(r.x, bold_obs) : 0.0f;
         float cc, c2 = 0.0f;
         if constexpr (CF == TVBG_CFUN_LEMS_2) {
-            cc = M::coupling(cs[k * stride], x, p);
-            c2 = M::coupling2(cs[(K + k) * stride], x, p);
+            cc = M::coupling(cs[k * stride], r.x, r.p);
+            c2 = M::coupling2(cs[(K + k) * stride], r.x, r.p);
         } else if constexpr (NC == 2) {
             // sum_e w sin(x_j - x_i); Kuramoto: post = a * mean (coupling.py:119-121)
             const float S = cs0 * cs[k * stride] - sn0 * cs[(K + k) * stride];
             if constexpr (CF == TVBG_CFUN_LEMS_SC) {
-                cc = M::coupling(S, x, p);
+                cc = M::coupling(S, r.x, r.p);
             } else {
                 cc = c.cf_a * (S / static_cast<float>(N));
             }
         } else if constexpr (CF == TVBG_CFUN_LEMS) {
-            cc = M::coupling(cs[k * stride], x, p);
+            cc = M::coupling(cs[k * stride], r.x, r.p);
         } else {
-            cc = lane_post<CF>(cs[k * stride], obs0, wsum, c.cf_a, g.cf_b);
+            cc = lane_post<CF>(cs[k * stride], obs0, r.wsum, c.cf_a, cf_b);
         }
         float f[NS];
         if constexpr (CF == TVBG_CFUN_LEMS_2) {
-            M::drift2(x, cc, c2, p, g.consts, f);
+            M::drift2(r.x, cc, c2, r.p, Kc, f);
         } else {
-            M::drift(x, cc, p, g.consts, f);
+            M::drift(r.x, cc, r.p, Kc, f);
         }
 #pragma unroll
-        for (int v = 0; v < NS; ++v) x[v] = fmaf(dt, f[v], x[v]);
+        for (int v = 0; v < NS; ++v) r.x[v] = fmaf(dt, f[v], r.x[v]);
         if constexpr (Noise<M>::kOK) {
             if (noise) {
-                const int r0 = static_cast<int>(t & (SPC - 1));
-                if (k == 0 || r0 == 0) {
+                const int r0 = ALIGNED ? k % SPC : static_cast<int>(t & (SPC - 1));
+                if (ALIGNED ? r0 == 0 : (k == 0 || r0 == 0)) {
                     const u32x4 w = philox4x32_10(static_cast<uint32_t>(n), static_cast<uint32_t>(t / SPC),
-                                                  g.seed_hi, 0u, g.seed_lo, c.inst_id);
+                                                  seed_hi, 0u, seed_lo, c.inst_id);
                     box_muller_fast(w.v[0], w.v[1], zz[0], zz[1]);
                     box_muller_fast(w.v[2], w.v[3], zz[2], zz[3]);
                 }
 #pragma unroll
-                for (int v = 0; v < NS; ++v) x[v] = fmaf(sqrt_dt * pick4(zz, r0 * NS + v), g.sigma[v], x[v]);
+                for (int v = 0; v < NS; ++v) r.x[v] = fmaf(sqrt_dt * pick4(zz, r0 * NS + v), sig[v], r.x[v]);
             }
         } else if constexpr (WideNoise<M>::value) {
             if (noise) {
                 float z8[8];
 #pragma unroll
                 for (int b = 0; b < 2; ++b) {
-                    const u32x4 w = philox4x32_10(static_cast<uint32_t>(n), static_cast<uint32_t>(t), g.seed_hi,
-                                                  static_cast<uint32_t>(b), g.seed_lo, c.inst_id);
+                    const u32x4 w = philox4x32_10(static_cast<uint32_t>(n), static_cast<uint32_t>(t), seed_hi,
+                                                  static_cast<uint32_t>(b), seed_lo, c.inst_id);
                     box_muller_fast(w.v[0], w.v[1], z8[4 * b], z8[4 * b + 1]);
                     box_muller_fast(w.v[2], w.v[3], z8[4 * b + 2], z8[4 * b + 3]);
                 }
 #pragma unroll
                 for (int v = 0; v < NS; ++v)
-                    x[v] = fmaf(sqrt_dt * z8[v], g.sigma[0] * NoiseScale<M>::at(v), x[v]);
+                    r.x[v] = fmaf(sqrt_dt * z8[v], sig[0] * NoiseScale<M>::at(v), r.x[v]);
             }
         }
-        M::limit(x, c.flags);
-        obs0 = M::obs(x, 0);
+        M::limit(r.x, c.flags);
+        obs0 = M::obs(r.x, 0);
         const uint32_t pos = (static_cast<uint32_t>(t) + 1u) & mask;
-        const size_t idx = (static_cast<size_t>(n) * R + pos) * RL + l;
+        const uint32_t idx = pos * RL;
         if constexpr (NC == 2) {
             if constexpr (CF == TVBG_CFUN_LEMS_2) {
-                sn0 = M::ring_value(obs0, p);
-                cs0 = M::ring_value2(x[M::CVAR2], p);
+                sn0 = M::ring_value(obs0, r.p);
+                cs0 = M::ring_value2(r.x[M::CVAR2], r.p);
             } else {
                 sincosf(obs0, &sn0, &cs0);
             }
             ring[idx] = sn0;
             ring[idx + kLanes] = cs0;
             if (pos < kGhost) {
-                ring[idx + static_cast<size_t>(nh) * RL] = sn0;
-                ring[idx + static_cast<size_t>(nh) * RL + kLanes] = cs0;
+                ring[idx + nh * RL] = sn0;
+                ring[idx + nh * RL + kLanes] = cs0;
             }
         } else {
-            const float rv = ring_val<M, CF>(obs0, p);
+            const float rv = ring_val<M, CF>(obs0, r.p);
             ring[idx] = rv;
-            if (pos < kGhost) ring[idx + static_cast<size_t>(nh) * kLanes] = rv;
+            if (pos < kGhost) ring[idx + nh * RL] = rv;
         }
-        if (bold) {
-            Balloon::step(bs, bF, bV, bQ, xbold, g.dt_bold);
+        if (MON && bold) {
+            Balloon::step(r.bs, r.bF, r.bV, r.bQ, xbold, dt_bold);
             if (k == b_next) {
                 if (brow >= 0 && brow < g.bold_len)
-                    g.bold_out[(static_cast<size_t>(brow) * N + n) * kLanes + l] = Balloon::signal(bV, bQ);
+                    g.bold_out[(static_cast<size_t>(brow) * N + n) * kLanes + l] = Balloon::signal(r.bV, r.bQ);
                 b_next += mc.bper;
                 brow += 1;
             }
         }
-    }
+    };
+    // Whole blocks are unrolled: the generator and the addresses of later
+    // steps do not depend on the state, so they fill the waits of the earlier
+    // ones.  (The models with long drifts, or sincosf per step, stay rolled.)
+    if constexpr (NS <= 2 && NC == 1 && CF != TVBG_CFUN_LEMS) {
+        if (kend == K && (tb & (SPC - 1)) == 0) {
+            if (bold || trace) {
+#pragma unroll 1
+                for (int k0 = 0; k0 < K; k0 += kStepUnroll)
 #pragma unroll
-    for (int v = 0; v < NS; ++v) state[(n * NS + v) * kLanes + l] = x[v];
-    if (bold) {
-        g.bold[(0 * N + n) * kLanes + l] = bs;
-        g.bold[(1 * N + n) * kLanes + l] = bF;
-        g.bold[(2 * N + n) * kLanes + l] = bV;
-        g.bold[(3 * N + n) * kLanes + l] = bQ;
+                    for (int k = 0; k < kStepUnroll; ++k) step(k0 + k, Flag<true>{}, Flag<true>{});
+            } else {
+#pragma unroll 1
+                for (int k0 = 0; k0 < K; k0 += kStepUnroll)
+#pragma unroll
+                    for (int k = 0; k < kStepUnroll; ++k) step(k0 + k, Flag<false>{}, Flag<true>{});
+            }
+            return;
+        }
+    }
+#pragma unroll 1
+    for (int k = 0; k < kend; ++k) step(k, Flag<true>{}, Flag<false>{});
+}
+
+// Plain group run: per block, every thread gathers its node's sums and then
+// runs its updates; a slot takes several nodes in turn (rounds) where the
+// CTAs hold fewer slots than nodes.
+template <class M, int CF, int K, int BOUND>
+__device__ __forceinline__ void run_group(const tvbg_group& g, float* csum, EdgeStage& stage, int32_t* status) {
+    uint2* records = reinterpret_cast<uint2*>(csum + ring_channels<CF>() * K * blockDim.x);
+    const int N = g.N;
+    const uint32_t C = cluster_nranks();
+    const uint32_t rank = cluster_rank();
+    const bool cluster = C > 1;
+    if (!group_descriptor_ok<M, CF>(g)) {
+        if (threadIdx.x == 0) report(status, TVBG_EINVAL);
+        return;  // every CTA of the cluster reads the same descriptor and leaves here
+    }
+    const int l = threadIdx.x % kLanes;
+    const int P = blockDim.x / kLanes;
+    const int stride = static_cast<int>(C) * P;
+    const int rounds = (N + stride - 1) / stride;       // warp-uniform node loop
+    const int q0 = (threadIdx.x / kLanes) * static_cast<int>(C) + static_cast<int>(rank);
+    const GroupLane c = make_lane<M, CF, K>(g, l);
+    // with one node per slot the edge records are staged
+    const int n0 = q0 < N ? (g.nodes ? __ldg(g.nodes + q0) : q0) : 0;
+    const int lo0 = q0 < N ? __ldg(g.row + n0) : 0;
+    const int deg0 = q0 < N ? __ldg(g.row + n0 + 1) - lo0 : 0;
+    const uint2* edges0 = reinterpret_cast<const uint2*>(g.edges) + lo0;
+    if (rounds == 1) edges0 = stage_edges(g, stage, records, P, threadIdx.x, lo0, deg0);
+    for (int q = q0; q < N; q += stride) seed_node<M, CF>(g, c, g.nodes ? __ldg(g.nodes + q) : q);
+    group_barrier(cluster);
+    MonitorClock mc;
+    mc.init(g, c);
+    const long long t_stop = c.t0 + g.nsteps;
+    for (long long tb = c.t0; tb < t_stop; tb += K) {
+        const int cnt = (t_stop - tb) < K ? static_cast<int>(t_stop - tb) : K;
+        for (int r = 0; r < rounds; ++r) {
+            const int q = q0 + r * stride;
+            const bool valid = q < N;
+            int n = n0, deg = deg0;
+            const uint2* edges = edges0;
+            if (r > 0) {
+                n = valid ? (g.nodes ? __ldg(g.nodes + q) : q) : 0;
+                const int lo = valid ? __ldg(g.row + n) : 0;
+                deg = valid ? __ldg(g.row + n + 1) - lo : 0;
+                edges = reinterpret_cast<const uint2*>(g.edges) + lo;
+                __syncwarp();  // the last round's sums have been read
+            }
+            gather_node<M, CF, K, BOUND>(g, c, edges, deg, static_cast<uint32_t>(tb) & c.mask, csum + threadIdx.x - l,
+                                  blockDim.x);
+            __syncwarp();             // the slot's lanes read each other's sums
+            if (!valid) continue;
+            NodeRegs<M, CF> x;
+            x.load(g, c, n);
+            update_node<M, CF, K>(g, c, x, n, tb, cnt, csum + threadIdx.x, blockDim.x, mc);
+            x.store(g, c, n);
+        }
+        mc.advance(g, c, cnt);
+        group_barrier(cluster);
     }
 }
 
+// Phase counter of a cluster (pipelined kernel): every CTA's mbarrier takes
+// one arrival from each CTA of the cluster per phase.  One warp publishes a
+// phase (fence, then a remote arrive per CTA) and awaits it, in place of a
+// barrier.cluster with release and acquire by every thread, which cost
+// about 2300 cycles per block of 8 steps with nothing else to do.
+struct ClusterPhases {
+    unsigned long long bar;
+    int fail;             // a wait ran out in phase fail - 1: every thread leaves after that phase
+
+    __device__ __forceinline__ void init(uint32_t C) {  // one thread; cluster barrier before use
+        fail = 0;
+        mbar_init(smem_addr(&bar), C);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    // One warp, after a CTA barrier: what the CTA wrote before that barrier
+    // is visible to the cluster once this phase is awaited (the fence and the
+    // release are cumulative over the CTA barrier).
+    __device__ __forceinline__ void publish(uint32_t C) {
+        const uint32_t lane = threadIdx.x & 31u;
+        if (lane < C) {
+            asm volatile("fence.acq_rel.cluster;" ::: "memory");
+            uint32_t remote;
+            asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(smem_addr(&bar)), "r"(lane));
+            asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(remote) : "memory");
+        }
+        __syncwarp();
+    }
+    // One warp, in phase `now`: wait (bounded) for phase `ph` of every CTA.
+    __device__ __forceinline__ void await(uint32_t ph, uint32_t now) {
+        const uint32_t a = smem_addr(&bar);
+        uint32_t ok = 0;
+        for (int it = 0; it < (1 << 20) && !ok; ++it)
+            asm volatile(
+                "{\n\t.reg .pred p;\n\t"
+                "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
+                "selp.u32 %0, 1, 0, p;\n\t}"
+                : "=r"(ok)
+                : "r"(a), "r"(ph & 1u)
+                : "memory");
+        if (!ok) fail = static_cast<int>(now + 1);
+        __syncwarp();
+    }
+    // After the CTA barrier of phase `now`: the same answer in every thread.
+    __device__ __forceinline__ bool failed(uint32_t now) const {
+        const int f = *const_cast<const volatile int*>(&fail);
+        return f != 0 && static_cast<uint32_t>(f) <= now + 1;
+    }
+};
+
 // Pipelined group run: the CTA's warps form two teams of H = blockDim / 2
-// threads, both mapped onto the same (node, lane) pairs.  While the update
-// team runs the K steps of block b from the coupling sums in one shared
-// buffer, the gather team sums block b + 1 into the other; one (cluster)
-// barrier per block.  Block b + 1 reads ring slots up to
+// threads, both mapped onto the same (node, lane) pairs.  In phase b the
+// update team runs the K steps of block b from the coupling sums in one
+// shared buffer while the gather team sums block b + 1 into the other; a CTA
+// barrier ends the phase.  Block b + 1 reads ring slots up to
 // tb + 2K - 1 - d_min, so with d_min >= 2K - 1 every slot it reads was
-// written before block b started (ordered by the previous barrier), and
-// the newest slot written in block b (tb + K) is at most d_max < nh slots
-// ahead of the oldest read, so no read aliases a write.  Same arithmetic in
-// the same order as run_group, so the results are identical.  Needs one
-// node per slot (C * H / 8 >= N), K in {4, 8} and a 16-byte aligned ring.
-template <class M, int CF, int K>
-__device__ __forceinline__ void run_group_pipelined(const tvbg_group& g, float* csum, int32_t* status) {
+// written before block b started, and the newest slot written in block b
+// (tb + K) is at most d_max < nh slots ahead of the oldest read, so no read
+// aliases a write.  Same arithmetic in the same order as run_group, so the
+// results are identical.  Needs one node per slot (C * H / 8 >= N), K in
+// {4, 8} and a 16-byte aligned ring.
+//
+// Across the CTAs of a cluster a phase must not start before the writes it
+// reads have been published.  With d_min >= 3K - 1 (lag) the gather of phase
+// b reads nothing newer than block b - 2, so the phase that ends is
+// published by one warp during the next phase and awaited at that one's
+// end: no thread stands at a cluster-wide barrier.  A CTA may then be one
+// phase ahead of another, writing up to slot tb + 2K while tb + K - d_max is
+// read: K + d_max < nh, which nh >= d_max + 1 + K covers.  With shorter
+// delays the phase is awaited before the next one starts.
+template <class M, int CF, int K, int BOUND>
+__device__ __forceinline__ void run_group_pipelined(const tvbg_group& g, float* csum, EdgeStage& stage,
+                                                    ClusterPhases& phases, int32_t* status) {
     constexpr int NC = ring_channels<CF>();
     const int N = g.N;
     const uint32_t C = cluster_nranks();
@@ -895,80 +820,113 @@ __device__ __forceinline__ void run_group_pipelined(const tvbg_group& g, float* 
         if (threadIdx.x == 0) report(status, TVBG_EINVAL);
         return;  // uniform over the cluster: same descriptor, same launch shape
     }
+    const bool lag = g.dmin >= 3 * K - 1;
     const bool gather_team = static_cast<int>(threadIdx.x) >= H;
     const int tid = static_cast<int>(threadIdx.x) - (gather_team ? H : 0);
     const int l = tid % kLanes;
     const int q = (tid / kLanes) * static_cast<int>(C) + static_cast<int>(rank);
     const bool valid = q < N;
     const int n = valid ? (g.nodes ? __ldg(g.nodes + q) : q) : 0;
-    const GroupLane c = make_lane<M>(g, l);
+    const int lo = valid ? __ldg(g.row + n) : 0;
+    const int deg = valid ? __ldg(g.row + n + 1) - lo : 0;
+    const GroupLane c = make_lane<M, CF, K>(g, l);
     const int bufsz = NC * K * H;  // floats per coupling-sum buffer
+    if (threadIdx.x == 0) phases.init(C);
+    // the gather team's threads carry the slots (their tid is the scan's)
+    const int st_tid = gather_team ? tid : H + tid;
+    const uint2* edges = stage_edges(g, stage, reinterpret_cast<uint2*>(csum + 2 * bufsz), P, st_tid, lo, deg);
 
     if (!gather_team && valid) seed_node<M, CF>(g, c, n);
     group_barrier(cluster);
     // each team runs its own loop (disjoint live ranges); both meet at the
-    // same number of barriers: one after block 0's gather, one per block
+    // same barriers
     const long long t_stop = c.t0 + g.nsteps;
     if (gather_team) {
+        // the last gather warp, whose nodes have the fewest edges, keeps the phases
+        const bool keeper = cluster && tid >= H - 32;
         if (g.nsteps > 0)
-            gather_node<M, CF, K>(g, c, valid, n, static_cast<uint32_t>(c.t0) & c.mask, csum + tid, H);
-        group_barrier(cluster);
-        int buf = 1;
+            gather_node<M, CF, K, BOUND>(g, c, edges, deg, static_cast<uint32_t>(c.t0) & c.mask, csum + tid - l, H);
+        __syncthreads();
+        uint32_t ph = 0;  // phases ended
         for (long long tb = c.t0; tb < t_stop; tb += K) {
+            if (keeper && lag && ph > 0) phases.publish(C);
             if (tb + K < t_stop)
-                gather_node<M, CF, K>(g, c, valid, n, static_cast<uint32_t>(tb + K) & c.mask,
-                                      csum + buf * bufsz + tid, H);
-            buf ^= 1;
-            group_barrier(cluster);
+                gather_node<M, CF, K, BOUND>(g, c, edges, deg, static_cast<uint32_t>(tb + K) & c.mask,
+                                      csum + ((ph + 1) & 1u) * bufsz + tid - l, H);
+            if (keeper && lag && ph > 0) phases.await(ph - 1, ph);
+            __syncthreads();
+            if (cluster && !lag) {
+                if (keeper) {
+                    phases.publish(C);
+                    phases.await(ph, ph);
+                }
+                __syncthreads();
+            }
+            if (cluster && phases.failed(ph)) break;
+            ++ph;
         }
     } else {
-        group_barrier(cluster);
+        __syncthreads();
         MonitorClock mc;
         mc.init(g, c);
-        int buf = 0;
+        NodeRegs<M, CF> r;       // one node per thread: its state stays in registers
+        if (valid) r.load(g, c, n);
+        uint32_t ph = 0;
         for (long long tb = c.t0; tb < t_stop; tb += K) {
             const int cnt = (t_stop - tb) < K ? static_cast<int>(t_stop - tb) : K;
-            if (valid) update_node<M, CF, K>(g, c, n, tb, cnt, csum + buf * bufsz + tid, H, mc);
+            if (valid) update_node<M, CF, K>(g, c, r, n, tb, cnt, csum + (ph & 1u) * bufsz + tid, H, mc);
             mc.advance(g, c, cnt);
-            buf ^= 1;
-            group_barrier(cluster);
+            __syncthreads();
+            if (cluster && !lag) __syncthreads();
+            if (cluster && phases.failed(ph)) break;
+            ++ph;
         }
+        if (valid) r.store(g, c, n);
+    }
+    if (cluster) {
+        if (threadIdx.x == 0 && phases.fail) report(status, TVBG_ETIMEOUT);
+        group_barrier(true);  // no CTA leaves while another may still arrive on its phases
     }
 }
 
 // Dynamic shared memory of a pipelined group CTA: two coupling-sum buffers
-// of half the CTA each.
+// of half the CTA each, and the staged edge records.
 __host__ __device__ constexpr uint32_t group_pipelined_smem_bytes(int K, int threads, int nc) {
-    return static_cast<uint32_t>(4 * 2 * K * (threads / 2) * nc);
+    return static_cast<uint32_t>(4 * 2 * K * (threads / 2) * nc + stage_bytes(threads / 2));
 }
 
 // One group per CTA (or per cluster of CTAs): group index = order[cluster id].
-template <class M, int CF, int K>
-__global__ void __launch_bounds__(1024, 1)
+// BOUND: the largest CTA the instance is built for (its registers a thread).
+template <class M, int CF, int K, int BOUND = 1024>
+__global__ void __launch_bounds__(BOUND, 1)
     group_kernel(const tvbg_group* __restrict__ groups, int32_t n_groups,
                  const int32_t* __restrict__ order, int32_t* __restrict__ status) {
     __shared__ __align__(16) tvbg_group s_grp;
-    extern __shared__ float csum[];  // [channels][K][blockDim]: the block's coupling sums
+    __shared__ EdgeStage s_stage;
+    extern __shared__ __align__(16) float csum[];  // [channels][K][blockDim]: the block's sums; edge records
     const int cid = static_cast<int>(cluster_id_x());
     if (cid >= n_groups) return;  // uniform over the cluster
     const int idx = order ? __ldg(order + cid) : cid;
     stage_group(groups + idx, &s_grp);
-    run_group<M, CF, K>(s_grp, csum, status);
+    run_group<M, CF, K, BOUND>(s_grp, csum, s_stage, status);
 }
 
 // Pipelined variant (run_group_pipelined): blockDim = 2 teams x 8 lanes x
 // node slots; same tables and results as group_kernel.
-template <class M, int CF, int K>
-__global__ void __launch_bounds__(1024, 1)
+template <class M, int CF, int K, int BOUND = 1024>
+__global__ void __launch_bounds__(BOUND, 1)
     group_kernel_pipelined(const tvbg_group* __restrict__ groups, int32_t n_groups,
                            const int32_t* __restrict__ order, int32_t* __restrict__ status) {
     __shared__ __align__(16) tvbg_group s_grp;
-    extern __shared__ float csum[];  // [2][channels][K][blockDim / 2]
+    __shared__ EdgeStage s_stage;
+    __shared__ ClusterPhases s_phases;
+    static_assert(sizeof(EdgeStage) + sizeof(ClusterPhases) + 64 <= 640, "kGroupStaticBytes");
+    extern __shared__ __align__(16) float csum[];  // [2][channels][K][blockDim / 2]; edge records
     const int cid = static_cast<int>(cluster_id_x());
     if (cid >= n_groups) return;  // uniform over the cluster
     const int idx = order ? __ldg(order + cid) : cid;
     stage_group(groups + idx, &s_grp);
-    run_group_pipelined<M, CF, K>(s_grp, csum, status);
+    run_group_pipelined<M, CF, K, BOUND>(s_grp, csum, s_stage, s_phases, status);
 }
 
 }  // namespace tvbg

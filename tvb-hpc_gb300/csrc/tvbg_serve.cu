@@ -312,10 +312,10 @@ int plan(Request& r, const tvbg_serve_request& q) {
 // (cudaOccupancyMaxActiveClusters); the plain shape is used where not.
 bool pipelined_fits(const Request& r) {
     for (int k : r.k_list) {
-        GroupKernel kfn = lookup_group_kernel(r.model, r.cfun, k, true);
+        GroupKernel kfn = lookup_group_kernel(r.model, r.cfun, k, group_form(r.threads, r.cluster, true));
         if (!kfn) return false;
         const size_t smem = group_pipelined_smem_bytes(k, r.threads, group_channels(r.cfun));
-        if (smem + sizeof(tvbg_group) > 48u * 1024u &&
+        if (smem + kGroupStaticBytes > 48u * 1024u &&
             cudaFuncSetAttribute(reinterpret_cast<const void*>(kfn),
                                  cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  static_cast<int>(smem)) != cudaSuccess)
@@ -495,7 +495,9 @@ int launch_chunk(tvbg_serve& p, Request& r, int64_t steps) {
         cfg.d_status = reinterpret_cast<int32_t*>(r.dev + r.off_status);
         cfg.d_order = reinterpret_cast<const int32_t*>(r.dev + r.off_order) + r.k_start[i];
         const bool pipe = r.tpn == TVBG_GROUP_PIPELINED;
-        GroupKernel k = lookup_group_kernel(r.model, r.cfun, r.k_list[i], pipe);
+        GroupKernel k = lookup_group_kernel(
+            r.model, r.cfun, r.k_list[i],
+            group_form(r.threads, static_cast<long long>(r.k_count[i]) * r.cluster, pipe));
         if (!k) return set_error(TVBG_EUNSUPPORTED, "tvbg_serve: group kernel not built");
         const size_t smem =
             pipe ? group_pipelined_smem_bytes(cfg.block_k, cfg.threads, group_channels(cfg.cfun))
