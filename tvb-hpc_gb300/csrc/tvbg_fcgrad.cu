@@ -9,6 +9,7 @@
 // over the N nodes per sample (the loss's reductions over time, the FC
 // itself, stay FP64 in the caller).
 #include "tvbg_abi_internal.h"
+#include "tvbg_gram.cuh"
 
 namespace {
 
@@ -85,9 +86,8 @@ extern "C" int tvbg_fcfit_zgrad(const float* d_z, const float* d_a, float* d_out
 // X_b [T][N] (rows 0..T-2 from x, row T-1 from `last` when given), its
 // Pearson FC in FP64, the loss mean_{i<j} (FC_ij - F*_ij)^2 and
 // dL/dX = (Z A - Z diag(FC A)) / nrm, Z = (X - mean) / nrm, A = 2 (FC - F*) / P
-// with a zero diagonal (P = N (N - 1) / 2).  Kernels: FP64 means; the
-// centred Gram, upper triangle only (FP32 error-free transformations for
-// N <= 192, FP64 tiles above); per instance the norms from the Gram's
+// with a zero diagonal (P = N (N - 1) / 2).  Kernels: means and the centred
+// Gram to FP64 accuracy (tvbg_gram.cuh); per instance the norms from the Gram's
 // diagonal, FC, loss, A and diag(FC A) (the chain rule's time reduction
 // sum_t Z_ti (Z A)_ti, taken from FC in FP64); dL/dX in FP32 (Z A is a sum
 // over N nodes per sample, the precision of the backward).  The Pearson FC
@@ -97,243 +97,48 @@ extern "C" int tvbg_fcfit_zgrad(const float* d_z, const float* d_a, float* d_out
 
 namespace {
 
-// Instance b of a series lives in block b / lanes at lane b % lanes:
-// lanes = 1 for per-instance arrays, 8 for lane-interleaved groups.
-struct SeriesView {
-    const float* x;      // row s (s < T - 1, or every row without `last`):
-    int64_t xs;          //   x + (b / lanes) xs + b % lanes + (s N + i) lanes
-    const float* last;   // row T - 1: last + (b / lanes) ls + b % lanes + i lns, or NULL
-    int64_t ls, lns;
-    int T, N, lanes;
-    __device__ __forceinline__ float at(int b, int s, int i) const {
-        const int g = b / lanes, l = b % lanes;
-        if (last && s == T - 1) return __ldg(last + g * ls + l + static_cast<int64_t>(i) * lns);
-        return __ldg(x + g * xs + l + (static_cast<int64_t>(s) * N + i) * lanes);
+using tvbg::SeriesView;
+
+// FP64 means and the centred Gram (tvbg_gram.cuh), both triangles written.
+// Pass per adjoint at N = 84, 256 instances, 2000 samples: 1.54 ms with FP32
+// error-free products on the FP32 pipe and 0.31 for the means before.
+struct GramOut {
+    double* g;       // the instance's [N][N]
+    double* mean;    // the instance's [N]
+    int N;
+    __device__ __forceinline__ void put(int i, int j, double x, bool first) const {
+        double* p = g + static_cast<int64_t>(i) * N + j;
+        const double s = first ? x : *p + x;
+        *p = s;
+        g[static_cast<int64_t>(j) * N + i] = s;
     }
 };
 
-// FP64 mean of every (instance, node): the samples split into kMS slices
-// of consecutive samples, one thread each, the slices' sums added in slice
-// order.  CTA = 32 nodes x kMS slices of one instance (blockIdx.y).
-constexpr int kMS = 8;
-__global__ void __launch_bounds__(256) fcfit_mean_kernel(SeriesView v, double* mean) {
-    __shared__ double part[kMS][32];
-    const int b = blockIdx.y;
-    const int i = blockIdx.x * 32 + static_cast<int>(threadIdx.x);
-    const int per = (v.T + kMS - 1) / kMS;
-    const int t0 = static_cast<int>(threadIdx.y) * per;
-    const int t1 = t0 + per < v.T ? t0 + per : v.T;
-    double s = 0.0;
-    if (i < v.N)
-        for (int t = t0; t < t1; ++t) s += static_cast<double>(v.at(b, t, i));
-    part[threadIdx.y][threadIdx.x] = s;
-    __syncthreads();
-    if (threadIdx.y == 0 && i < v.N) {
-        double m = 0.0;
-#pragma unroll
-        for (int k = 0; k < kMS; ++k) m += part[k][threadIdx.x];
-        mean[static_cast<int64_t>(b) * v.N + i] = m / static_cast<double>(v.T);
-    }
-}
-
-// Error-free transformations in FP32 (Knuth's TwoSum and TwoProduct by FMA,
-// as used in Ogita, Rump and Oishi, "Accurate sum and dot
-// product", SIAM J. Sci. Comput. 26(6), 2005).  Every operation is an
-// explicitly rounded intrinsic: nothing is contracted or reordered.
-__device__ __forceinline__ void two_sum(float a, float b, float& s, float& e) {
-    s = __fadd_rn(a, b);
-    const float bb = __fsub_rn(s, a);
-    e = __fadd_rn(__fsub_rn(a, __fsub_rn(s, bb)), __fsub_rn(b, bb));
-}
-
-// Centred Gram G_ij = sum_t c_ti c_tj, c = x - mean, for N <= kTriMaxN,
-// all in FP32 arithmetic with error-free transformations (GB300 runs FP32
-// at about 64 times its FP64 rate; one DFMA per product took 4.2 ms per
-// adjoint pass at N = 84, 256 instances, 2000 samples).
-//
-// Work split: the exact upper triangle of 2 x 2 pair blocks (ceil(N/2)
-// (ceil(N/2) + 1) / 2 of them, row-major), kSplitBPT blocks per thread,
-// CTA = (instance blockIdx.x, part blockIdx.y), instances fastest so that
-// the lanes of a lane-interleaved group read the same sectors together.
-//
-// Centring: each mean (FP64) is split once into mh + ml (FP32 words); a
-// sample x becomes c = (x - mh) - ml as (hi, lo) with hi + lo = c up to
-// about 2^-48 (|c| + 2 |mean|): TwoSum(x, -mh) = (d, de), then
-// TwoSum(d, de - ml).  kTriL samples of every node staged per pass.
-//
-// Products: per pair and sample hi_i hi_j = p + e exactly (TwoProduct);
-// p is summed by TwoSum (rounding errors collected in a second word),
-// e + hi_i lo_j + lo_i hi_j (2^-24 of the product) in a third word; lo_i lo_j
-// (2^-48) is dropped.  Every kTriL samples the three words are added into
-// the pair's double-FP32 sum (TwoSum, then the small words, then TwoSum
-// again), converted to FP64 at the end.  The error is bounded by about kTriL^2 2^-48 sum_t |c_ti c_tj| (the
-// collected rounding errors of a pass summed in FP32), below 4e-12 of
-// ||c_i|| ||c_j||; typical errors are near 1e-14.  Both triangles of G
-// written.
-constexpr int kTriL = 32;
-constexpr int kTriMaxN = 192;   // staging (kTriL + 1) x N float2 <= 50.7 KB
-constexpr int kSplitBPT = 2;
-__global__ void __launch_bounds__(256) fcfit_gram_split_kernel(SeriesView v,
-                                                               const double* __restrict__ mean,
-                                                               double* G) {
-    extern __shared__ float2 sh[];  // [kTriL][Np] (hi, lo); then [Np] (mh, ml)
+// N <= ROWS: one CTA per instance.
+template <int ROWS>
+__global__ void __launch_bounds__(tvbg::kGramThreads) fcfit_gram_kernel(SeriesView v, double* mean, double* G) {
+    extern __shared__ __align__(16) unsigned char gram_smem[];
+    __shared__ tvbg::GramNode nodes[ROWS];
+    __shared__ double scale[ROWS];
     const int b = blockIdx.x;
-    const int N = v.N;
-    const int nb = (N + 1) / 2;
-    const int Np = 2 * nb;
-    float2* smean = sh + kTriL * Np;
-    const long long nblk = static_cast<long long>(nb) * (nb + 1) / 2;
-    int i0[kSplitBPT], j0[kSplitBPT];
-    bool act[kSplitBPT];
-#pragma unroll
-    for (int q = 0; q < kSplitBPT; ++q) {
-        const long long k =
-            (static_cast<long long>(blockIdx.y) * kSplitBPT + q) * blockDim.x + threadIdx.x;
-        act[q] = k < nblk;
-        int bi = 0, bj = 0;
-        if (act[q]) {
-            long long rem = k;
-            while (rem >= nb - bi) {
-                rem -= nb - bi;
-                ++bi;
-            }
-            bj = bi + static_cast<int>(rem);
-        }
-        i0[q] = 2 * bi;
-        j0[q] = 2 * bj;
-    }
-    const double* mb = mean + static_cast<int64_t>(b) * N;
-    for (int c = threadIdx.x; c < N; c += blockDim.x) {
-        const double m = mb[c];
-        const float mh = __double2float_rn(m);
-        smean[c] = make_float2(mh, __double2float_rn(m - static_cast<double>(mh)));
-    }
-    float ah[kSplitBPT][4], al[kSplitBPT][4];  // double-FP32 sums
-#pragma unroll
-    for (int q = 0; q < kSplitBPT; ++q)
-#pragma unroll
-        for (int m = 0; m < 4; ++m) ah[q][m] = al[q][m] = 0.0f;
-    __syncthreads();
-    for (int t0 = 0; t0 < v.T; t0 += kTriL) {
-        for (int e = threadIdx.x; e < kTriL * Np; e += blockDim.x) {
-            const int r = e / Np, c = e % Np;
-            const int t = t0 + r;
-            float2 hl = make_float2(0.0f, 0.0f);
-            if (t < v.T && c < N) {
-                const float2 m = smean[c];
-                float d, de;
-                two_sum(v.at(b, t, c), -m.x, d, de);
-                two_sum(d, __fsub_rn(de, m.y), hl.x, hl.y);
-            }
-            sh[e] = hl;
-        }
-        __syncthreads();
-#pragma unroll
-        for (int q = 0; q < kSplitBPT; ++q) {
-            if (!act[q]) continue;
-            float s[4] = {0.0f, 0.0f, 0.0f, 0.0f}, cp[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-            float sm[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-#pragma unroll 4
-            for (int r = 0; r < kTriL; ++r) {
-                const float2* row = sh + r * Np;
-                const float2 x[2] = {row[i0[q]], row[i0[q] + 1]};
-                const float2 y[2] = {row[j0[q]], row[j0[q] + 1]};
-#pragma unroll
-                for (int u = 0; u < 2; ++u)
-#pragma unroll
-                    for (int w = 0; w < 2; ++w) {
-                        const int m = 2 * u + w;
-                        const float p = __fmul_rn(x[u].x, y[w].x);
-                        const float e = __fmaf_rn(x[u].x, y[w].x, -p);  // hi hi - p, exact
-                        sm[m] = __fadd_rn(sm[m], __fmaf_rn(x[u].x, y[w].y, __fmaf_rn(x[u].y, y[w].x, e)));
-                        float t, err;
-                        two_sum(s[m], p, t, err);
-                        s[m] = t;
-                        cp[m] = __fadd_rn(cp[m], err);
-                    }
-            }
-#pragma unroll
-            for (int m = 0; m < 4; ++m) {  // (ah, al) += s + (cp + sm)
-                float hi, lo;
-                two_sum(ah[q][m], s[m], hi, lo);
-                lo = __fadd_rn(lo, __fadd_rn(al[q][m], __fadd_rn(cp[m], sm[m])));
-                two_sum(hi, lo, ah[q][m], al[q][m]);
-            }
-        }
-        __syncthreads();
-    }
-    double* gb = G + static_cast<int64_t>(b) * N * N;
-#pragma unroll
-    for (int q = 0; q < kSplitBPT; ++q) {
-        if (!act[q]) continue;
-#pragma unroll
-        for (int u = 0; u < 2; ++u)
-#pragma unroll
-            for (int w = 0; w < 2; ++w) {
-                const int i = i0[q] + u, j = j0[q] + w;
-                if (i < N && j < N && j >= i) {
-                    const double g = static_cast<double>(ah[q][2 * u + w]) +
-                                     static_cast<double>(al[q][2 * u + w]);
-                    gb[static_cast<int64_t>(i) * N + j] = g;
-                    gb[static_cast<int64_t>(j) * N + i] = g;
-                }
-            }
-    }
+    const GramOut out{G + static_cast<int64_t>(b) * v.N * v.N, mean + static_cast<int64_t>(b) * v.N, v.N};
+    tvbg::gram_whole<ROWS>(
+        v, b, [=](int i, double m) { out.mean[i] = m; },
+        [=](int i, int j, double g, bool first) { out.put(i, j, g, first); },
+        reinterpret_cast<__nv_bfloat16*>(gram_smem), nodes, scale);
 }
 
-constexpr int kGT = 32;   // Gram tile: 32 x 32 node pairs, 32 samples per stage
-
-// The centred Gram for larger N: one CTA per upper-triangle 32 x 32 tile
-// (blockIdx.y enumerates tiles with jt >= it; instance blockIdx.x), 256
-// threads of 2 x 2 pairs, samples in order; both triangles written.
-__global__ void __launch_bounds__(256) fcfit_gram_kernel(SeriesView v, const double* __restrict__ mean,
-                                                         double* G) {
-    __shared__ double sI[kGT][kGT + 1];
-    __shared__ double sJ[kGT][kGT + 1];
+// Larger N: one CTA per 64 x 64 tile of the upper triangle (blockIdx.y).
+__global__ void __launch_bounds__(tvbg::kGramThreads) fcfit_gram_tiles_kernel(SeriesView v, double* mean, double* G) {
+    extern __shared__ __align__(16) unsigned char gram_smem[];
+    __shared__ tvbg::GramNode nodes[128];
+    __shared__ double scale[128];
     const int b = blockIdx.x;
-    const int N = v.N;
-    const int nt = (N + kGT - 1) / kGT;
-    int it = 0, rem = blockIdx.y;
-    while (rem >= nt - it) {
-        rem -= nt - it;
-        ++it;
-    }
-    const int jt = it + rem;
-    const int i0 = it * kGT, j0 = jt * kGT;
-    const int tx = threadIdx.x % 16, ty = threadIdx.x / 16;
-    const double* mb = mean + static_cast<int64_t>(b) * N;
-    double acc[2][2] = {{0.0, 0.0}, {0.0, 0.0}};
-    for (int t0 = 0; t0 < v.T; t0 += kGT) {
-        for (int k = threadIdx.x; k < kGT * kGT; k += 256) {
-            const int r = k / kGT, c = k % kGT;   // r: sample, c: node within the tile
-            const int t = t0 + r;
-            const int ii = i0 + c, jj = j0 + c;
-            sI[r][c] = (t < v.T && ii < N) ? static_cast<double>(v.at(b, t, ii)) - mb[ii] : 0.0;
-            sJ[r][c] = (t < v.T && jj < N) ? static_cast<double>(v.at(b, t, jj)) - mb[jj] : 0.0;
-        }
-        __syncthreads();
-#pragma unroll 8
-        for (int r = 0; r < kGT; ++r) {
-            const double a0 = sI[r][2 * ty], a1 = sI[r][2 * ty + 1];
-            const double c0 = sJ[r][2 * tx], c1 = sJ[r][2 * tx + 1];
-            acc[0][0] = fma(a0, c0, acc[0][0]);
-            acc[0][1] = fma(a0, c1, acc[0][1]);
-            acc[1][0] = fma(a1, c0, acc[1][0]);
-            acc[1][1] = fma(a1, c1, acc[1][1]);
-        }
-        __syncthreads();
-    }
-    double* gb = G + static_cast<int64_t>(b) * N * N;
-#pragma unroll
-    for (int u = 0; u < 2; ++u)
-#pragma unroll
-        for (int w = 0; w < 2; ++w) {
-            const int i = i0 + 2 * ty + u, j = j0 + 2 * tx + w;
-            if (i < N && j < N && j >= i) {
-                gb[static_cast<int64_t>(i) * N + j] = acc[u][w];
-                gb[static_cast<int64_t>(j) * N + i] = acc[u][w];
-            }
-        }
+    const GramOut out{G + static_cast<int64_t>(b) * v.N * v.N, mean + static_cast<int64_t>(b) * v.N, v.N};
+    tvbg::gram_pair(
+        v, b, blockIdx.y, [=](int i, double m) { out.mean[i] = m; },
+        [=](int i, int j, double g, bool first) { out.put(i, j, g, first); },
+        reinterpret_cast<__nv_bfloat16*>(gram_smem), nodes, scale);
 }
 
 // Per instance (one CTA): nrm_i = sqrt(G_ii) (the centred sum of squares);
@@ -547,24 +352,18 @@ extern "C" int tvbg_fcfit_loss(const float* d_x, int64_t x_inst_stride, const fl
     SeriesView v{d_x, x_inst_stride, d_last, last_inst_stride, last_node_stride, T, N, lanes};
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     if ((T + 63) / 64 > 65535) return tvbg::set_error(TVBG_EINVAL, "tvbg_fcfit_loss: T too large");
-    const int nt = (N + kGT - 1) / kGT;
-    if (N > kTriMaxN && nt * (nt + 1) / 2 > 65535)
+    const int64_t nt = (N + 63) / 64;
+    if (N > 128 && nt * (nt + 1) / 2 > 65535)
         return tvbg::set_error(TVBG_EINVAL, "tvbg_fcfit_loss: N too large");
-    fcfit_mean_kernel<<<dim3((N + 31) / 32, n_inst), dim3(32, kMS), 0, st>>>(v, mean);
-    if (N <= kTriMaxN) {
-        const int nb = (N + 1) / 2;
-        const long long nblk = static_cast<long long>(nb) * (nb + 1) / 2;
-        const unsigned parts = static_cast<unsigned>((nblk + 256 * kSplitBPT - 1) / (256 * kSplitBPT));
-        const size_t smem = 8u * (kTriL + 1) * 2u * static_cast<size_t>(nb);
-        if (smem > 48u * 1024u) {
-            const cudaError_t e = cudaFuncSetAttribute(reinterpret_cast<const void*>(fcfit_gram_split_kernel),
-                                                       cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                       static_cast<int>(smem));
-            if (e != cudaSuccess) return tvbg::set_cuda_error(e, "tvbg_fcfit_loss: smem attribute");
-        }
-        fcfit_gram_split_kernel<<<dim3(n_inst, parts), 256, smem, st>>>(v, mean, fc);
-    } else {
-        fcfit_gram_kernel<<<dim3(n_inst, nt * (nt + 1) / 2), 256, 0, st>>>(v, mean, fc);
+    {
+        const bool whole = N <= 128, half = N <= 96;
+        auto kfn = half ? fcfit_gram_kernel<96> : whole ? fcfit_gram_kernel<128> : fcfit_gram_tiles_kernel;
+        const size_t smem = tvbg::gram_plane_bytes(half ? 96 : 128);
+        const cudaError_t e = cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                   static_cast<int>(smem));
+        if (e != cudaSuccess) return tvbg::set_cuda_error(e, "tvbg_fcfit_loss: smem attribute");
+        kfn<<<dim3(n_inst, whole ? 1 : static_cast<unsigned>(nt * (nt + 1) / 2)), tvbg::kGramThreads, smem, st>>>(
+            v, mean, fc);
     }
     fcfit_loss_kernel<<<n_inst, 256, 0, st>>>(fc, d_target, N, mean, nrm, d_loss, a32, zg, fsc);
     if (d_dx) {
