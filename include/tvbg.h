@@ -463,6 +463,15 @@ int tvbg_cov_update(const float *d_x, int64_t x_stride, int32_t n_inst,
                     int32_t N, int64_t n, double *d_mean, double *d_m2,
                     void *stream);
 
+/*
+ * The same for `rows` samples per instance in one call: sample r of instance
+ * b at d_x + b * x_stride + r * row_stride, folded in order r = 0, 1, ...;
+ * n: samples folded before the first of them.
+ */
+int tvbg_cov_update_rows(const float *d_x, int64_t x_stride, int64_t row_stride,
+                         int32_t rows, int32_t n_inst, int32_t N, int64_t n,
+                         double *d_mean, double *d_m2, void *stream);
+
 /* Pearson correlation of a streaming state: corr_ij = m2_ij / sqrt(m2_ii
  * m2_jj), float [n_inst][N][N].  Replaces refs/covar.c:73-109 (cov_to_corr). */
 int tvbg_cov_corr(const double *d_m2, int32_t n_inst, int32_t N, float *d_corr,

@@ -9,8 +9,9 @@
 //   m2_ij  += d_i (x_j - mean_j')          (mean' the updated mean)
 // so after n samples m2 is the co-moment sum_s (x_si - m_i)(x_sj - m_j) and
 // corr_ij = m2_ij / sqrt(m2_ii m2_jj) (covar.c:73-109, whose 1/n
-// normalisation cancels in the ratio).  One CTA per instance; the instance's
-// sample and means are staged in shared memory.
+// normalisation cancels in the ratio).  The increments are symmetric
+// (x_j - mean_j' = d_j n / (n + 1)), so the upper triangle is computed, in
+// 32 x 32 tiles, and written to both.
 #include <cuda_runtime.h>
 
 #include <cmath>
@@ -21,47 +22,163 @@
 namespace tvbg {
 
 constexpr int kCovThreads = 256;
+constexpr int kCovTile = 32;
 
+// Tile (ti <= tj) q of the upper triangle of nt x nt tiles, row-major.
+__device__ __forceinline__ void cov_tile(int q, int nt, int& ti, int& tj) {
+    ti = 0;
+    while (q >= nt - ti) {
+        q -= nt - ti;
+        ++ti;
+    }
+    tj = ti + q;
+}
+
+// `rows` samples folded in order, RC at a time: the samples' d and x - mean'
+// of every node in shared memory, then each entry of m2 takes the RC products
+// between one read and one write.  CTA (blockIdx.x of gridDim.x, instance
+// blockIdx.y) takes every gridDim.x-th tile; with one CTA per instance it also
+// stores the means, else cov_mean_kernel does after it.
+// FP64 products bound it (two per SM and clock): 8 samples of 256 x 84 nodes take
+// 7.3 M of them, 12 us, where a launch per sample took 8 x 11.3.
 __global__ void __launch_bounds__(kCovThreads)
-    cov_update_kernel(const float* __restrict__ x, long long x_stride, int N, long long n,
-                      double* __restrict__ mean, double* __restrict__ m2) {
-    extern __shared__ double sh[];  // d[N] | x[N] - mean'[N]
-    double* d = sh;
-    double* e = sh + N;
-    const long long b = blockIdx.x;
-    const float* xb = x + b * x_stride;
+    cov_update_kernel(const float* __restrict__ x, long long inst_stride, long long row_stride, int rows, int RC,
+                      int N, long long n, double* __restrict__ mean, double* __restrict__ m2) {
+    extern __shared__ double sh[];  // mean[N] | d[RC][N] | e[RC][N]
+    __shared__ double tr[kCovTile][kCovTile + 1];
+    double* m = sh;
+    double* d = sh + N;
+    double* e = d + static_cast<size_t>(RC) * N;
+    const long long b = blockIdx.y;
+    const float* xb = x + b * inst_stride;
     double* mb = mean + b * N;
     double* cb = m2 + b * static_cast<long long>(N) * N;
-    const double rn = 1.0 / static_cast<double>(n + 1);
-    for (int i = threadIdx.x; i < N; i += blockDim.x) {
-        const double xi = static_cast<double>(xb[i]);
-        const double m_old = n == 0 ? 0.0 : mb[i];
-        const double di = xi - m_old;
-        const double m_new = m_old + di * rn;
-        d[i] = di;
-        e[i] = xi - m_new;
-        mb[i] = m_new;
+    const int lane = threadIdx.x % 32, warp = threadIdx.x / 32;
+    const int nt = (N + kCovTile - 1) / kCovTile;
+    for (int i = threadIdx.x; i < N; i += kCovThreads) m[i] = n == 0 ? 0.0 : mb[i];
+    for (int r0 = 0; r0 < rows; r0 += RC) {
+        const int rc = rows - r0 < RC ? rows - r0 : RC;
+        for (int i = threadIdx.x; i < N; i += kCovThreads) {
+            double mi = m[i];
+            for (int r = 0; r < rc; ++r) {
+                const double xi = static_cast<double>(__ldg(xb + (r0 + r) * row_stride + i));
+                const double di = xi - mi;
+                mi = mi + di * (1.0 / static_cast<double>(n + r0 + r + 1));
+                d[r * N + i] = di;
+                e[r * N + i] = xi - mi;
+            }
+            m[i] = mi;
+        }
+        __syncthreads();
+        const bool start = n + r0 == 0;   // the first sample starts the co-moment
+        for (int q = blockIdx.x; q < nt * (nt + 1) / 2; q += gridDim.x) {
+            int ti, tj;
+            cov_tile(q, nt, ti, tj);
+            const int j = tj * kCovTile + lane;
+#pragma unroll
+            for (int u = 0; u < kCovTile / 8; ++u) {
+                const int k = warp + 8 * u, i = ti * kCovTile + k;
+                if (i < N && j < N && i <= j) {
+                    double* p = cb + static_cast<long long>(i) * N + j;
+                    double a = start ? 0.0 : *p;
+                    for (int r = 0; r < rc; ++r) a = fma(d[r * N + i], e[r * N + j], a);
+                    *p = a;
+                    tr[k][lane] = a;
+                }
+            }
+            __syncthreads();
+#pragma unroll
+            for (int u = 0; u < kCovTile / 8; ++u) {
+                const int k = warp + 8 * u;
+                const int i = ti * kCovTile + lane, jj = tj * kCovTile + k;   // entry (jj, i)
+                if (i < jj && jj < N) cb[static_cast<long long>(jj) * N + i] = tr[lane][k];
+            }
+            __syncthreads();
+        }
+    }
+    if (gridDim.x == 1)
+        for (int i = threadIdx.x; i < N; i += kCovThreads) mb[i] = m[i];
+}
+
+// The means after the same samples, the same arithmetic.
+__global__ void __launch_bounds__(kCovThreads)
+    cov_mean_kernel(const float* __restrict__ x, long long inst_stride, long long row_stride, int rows, int N,
+                    long long n, double* __restrict__ mean) {
+    const long long b = blockIdx.y;
+    const int i = blockIdx.x * kCovThreads + threadIdx.x;
+    if (i >= N) return;
+    double mi = n == 0 ? 0.0 : mean[b * N + i];
+    for (int r = 0; r < rows; ++r) {
+        const double di = static_cast<double>(__ldg(x + b * inst_stride + r * row_stride + i)) - mi;
+        mi = mi + di * (1.0 / static_cast<double>(n + r + 1));
+    }
+    mean[b * N + i] = mi;
+}
+
+// 32 x 32 tiles, a reciprocal square root per node of the tile and two
+// products per pair (a root and a division per entry took 72 us for 256 x 84
+// nodes).
+__global__ void __launch_bounds__(kCovThreads)
+    cov_corr_kernel(const double* __restrict__ m2, int N, float* __restrict__ corr) {
+    __shared__ float tile[kCovTile][kCovTile + 1];
+    __shared__ double ri[kCovTile], rj[kCovTile];
+    const long long b = blockIdx.y;
+    const double* cb = m2 + b * static_cast<long long>(N) * N;
+    float* ob = corr + b * static_cast<long long>(N) * N;
+    const int lane = threadIdx.x % 32, warp = threadIdx.x / 32;
+    int ti, tj;
+    cov_tile(blockIdx.x, (N + kCovTile - 1) / kCovTile, ti, tj);
+    const int i0 = ti * kCovTile, j0 = tj * kCovTile;
+    if (threadIdx.x < 2 * kCovTile) {
+        const int k = threadIdx.x % kCovTile, v = (threadIdx.x < kCovTile ? i0 : j0) + k;
+        (threadIdx.x < kCovTile ? ri : rj)[k] =
+            v < N ? 1.0 / sqrt(cb[static_cast<long long>(v) * N + v]) : 0.0;
     }
     __syncthreads();
-    const long long NN = static_cast<long long>(N) * N;
-    for (long long q = threadIdx.x; q < NN; q += blockDim.x) {
-        const int i = static_cast<int>(q / N), j = static_cast<int>(q % N);
-        const double inc = d[i] * e[j];
-        cb[q] = n == 0 ? inc : cb[q] + inc;   // n == 0 starts the co-moment (inc is 0)
+    for (int k = warp; k < kCovTile; k += 8) {
+        const int i = i0 + k, j = j0 + lane;
+        if (i <= j && j < N) {
+            const float r = static_cast<float>(cb[static_cast<long long>(i) * N + j] * (ri[k] * rj[lane]));
+            ob[static_cast<long long>(i) * N + j] = r;
+            tile[k][lane] = r;
+        }
+    }
+    __syncthreads();
+    for (int k = warp; k < kCovTile; k += 8) {
+        const int i = i0 + lane, j = j0 + k;   // entry (j, i)
+        if (i < j && j < N) ob[static_cast<long long>(j) * N + i] = tile[lane][k];
     }
 }
 
-__global__ void __launch_bounds__(kCovThreads)
-    cov_corr_kernel(const double* __restrict__ m2, int N, float* __restrict__ corr) {
-    const long long b = blockIdx.x;
-    const double* cb = m2 + b * static_cast<long long>(N) * N;
-    float* ob = corr + b * static_cast<long long>(N) * N;
-    const long long NN = static_cast<long long>(N) * N;
-    for (long long q = threadIdx.x; q < NN; q += blockDim.x) {
-        const int i = static_cast<int>(q / N), j = static_cast<int>(q % N);
-        const double den = sqrt(cb[static_cast<long long>(i) * N + i] * cb[static_cast<long long>(j) * N + j]);
-        ob[q] = static_cast<float>(cb[q] / den);
+// Launch over all instances (gridDim.y at most 65535 at a time).
+static int cov_rows(const float* x, int64_t inst_stride, int64_t row_stride, int rows, int n_inst, int N, int64_t n,
+                    double* mean, double* m2, cudaStream_t st) {
+    // samples per pass: their d and e in at most 192 KB, at least four
+    int RC = static_cast<int>(192 * 1024 / (16 * static_cast<int64_t>(N)));
+    RC = RC > 16 ? 16 : (RC < 4 ? 4 : RC);
+    if (RC > rows) RC = rows;
+    const size_t smem = sizeof(double) * static_cast<size_t>(N) * (1 + 2 * RC);
+    if (smem > 48u * 1024u) {
+        const cudaError_t e = cudaFuncSetAttribute(cov_update_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                   static_cast<int>(smem));
+        if (e != cudaSuccess) return set_cuda_error(e, "tvbg_cov_update: smem attribute");
     }
+    const int nt = (N + kCovTile - 1) / kCovTile, tiles = nt * (nt + 1) / 2;
+    // few instances: their tiles spread over about 1200 CTAs
+    int parts = n_inst >= 600 ? 1 : 1200 / n_inst;
+    parts = parts > tiles ? tiles : parts;
+    for (int b0 = 0; b0 < n_inst; b0 += 65535) {
+        const unsigned nb = static_cast<unsigned>(n_inst - b0 < 65535 ? n_inst - b0 : 65535);
+        const float* xb = x + b0 * inst_stride;
+        double* mb = mean + static_cast<int64_t>(b0) * N;
+        cov_update_kernel<<<dim3(static_cast<unsigned>(parts), nb), kCovThreads, smem, st>>>(
+            xb, inst_stride, row_stride, rows, RC, N, n, mb, m2 + static_cast<int64_t>(b0) * N * N);
+        if (parts > 1)
+            cov_mean_kernel<<<dim3(static_cast<unsigned>((N + kCovThreads - 1) / kCovThreads), nb), kCovThreads, 0,
+                              st>>>(xb, inst_stride, row_stride, rows, N, n, mb);
+    }
+    const cudaError_t e = cudaGetLastError();
+    return e == cudaSuccess ? TVBG_OK : set_cuda_error(e, "tvbg_cov_update launch");
 }
 
 }  // namespace tvbg
@@ -70,16 +187,18 @@ using namespace tvbg;
 
 extern "C" int tvbg_cov_update(const float* d_x, int64_t x_stride, int32_t n_inst, int32_t N,
                                int64_t n, double* d_mean, double* d_m2, void* stream) {
-    if (n_inst < 0 || N <= 0 || n < 0 || x_stride < N || (n_inst > 0 && (!d_x || !d_mean || !d_m2)))
+    return tvbg_cov_update_rows(d_x, x_stride, 0, 1, n_inst, N, n, d_mean, d_m2, stream);
+}
+
+extern "C" int tvbg_cov_update_rows(const float* d_x, int64_t x_stride, int64_t row_stride, int32_t rows,
+                                    int32_t n_inst, int32_t N, int64_t n, double* d_mean, double* d_m2,
+                                    void* stream) {
+    if (n_inst < 0 || rows < 0 || N <= 0 || n < 0 || x_stride < N || (n_inst > 0 && (!d_x || !d_mean || !d_m2)))
         return set_error(TVBG_EINVAL, "tvbg_cov_update: bad arguments");
     if (N > 3000) return set_error(TVBG_EINVAL, "tvbg_cov_update: N above 3000");
-    if (n_inst == 0) return TVBG_OK;
-    const size_t smem = 2u * sizeof(double) * static_cast<size_t>(N);
-    cov_update_kernel<<<n_inst, kCovThreads, smem, static_cast<cudaStream_t>(stream)>>>(
-        d_x, x_stride, N, n, d_mean, d_m2);
-    cudaError_t e = cudaGetLastError();
-    if (e != cudaSuccess) return set_cuda_error(e, "tvbg_cov_update launch");
-    return TVBG_OK;
+    if (n_inst == 0 || rows == 0) return TVBG_OK;
+    return cov_rows(d_x, x_stride, row_stride, rows, n_inst, N, n, d_mean, d_m2,
+                    static_cast<cudaStream_t>(stream));
 }
 
 extern "C" int tvbg_cov_corr(const double* d_m2, int32_t n_inst, int32_t N, float* d_corr,
@@ -87,7 +206,14 @@ extern "C" int tvbg_cov_corr(const double* d_m2, int32_t n_inst, int32_t N, floa
     if (n_inst < 0 || N <= 0 || (n_inst > 0 && (!d_m2 || !d_corr)))
         return set_error(TVBG_EINVAL, "tvbg_cov_corr: bad arguments");
     if (n_inst == 0) return TVBG_OK;
-    cov_corr_kernel<<<n_inst, kCovThreads, 0, static_cast<cudaStream_t>(stream)>>>(d_m2, N, d_corr);
+    const long long nt = (static_cast<long long>(N) + kCovTile - 1) / kCovTile, tiles = nt * (nt + 1) / 2;
+    if (tiles > 0x7fffffffLL) return set_error(TVBG_EINVAL, "tvbg_cov_corr: N too large");
+    for (int b0 = 0; b0 < n_inst; b0 += 65535) {
+        const unsigned nb = static_cast<unsigned>(n_inst - b0 < 65535 ? n_inst - b0 : 65535);
+        const int64_t off = static_cast<int64_t>(b0) * N * N;
+        cov_corr_kernel<<<dim3(static_cast<unsigned>(tiles), nb), kCovThreads, 0, static_cast<cudaStream_t>(stream)>>>(
+            d_m2 + off, N, d_corr + off);
+    }
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return set_cuda_error(e, "tvbg_cov_corr launch");
     return TVBG_OK;

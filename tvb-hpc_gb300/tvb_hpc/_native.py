@@ -261,6 +261,7 @@ SIGNATURES = {
     'tvbg_net_run': (ctypes.c_int, [ctypes.POINTER(tvbg_net), _i64, _i32,
                                     ctypes.POINTER(tvbg_launch), _vp]),
     'tvbg_cov_update': (ctypes.c_int, [_vp, _i64, _i32, _i32, _i64, _vp, _vp, _vp]),
+    'tvbg_cov_update_rows': (ctypes.c_int, [_vp, _i64, _i64, _i32, _i32, _i32, _i64, _vp, _vp, _vp]),
     'tvbg_cov_corr': (ctypes.c_int, [_vp, _i32, _i32, _vp, _vp]),
     'tvbg_pack_edges_group': (ctypes.c_int, [_i32, _i32, _vp, _vp, _vp, _vp, _i32, _vp]),
     'tvbg_group_run': (ctypes.c_int, [_vp, _i32, ctypes.POINTER(tvbg_launch), _vp]),

@@ -128,7 +128,22 @@ class StreamingFC:
         self.n += 1
 
     def update_rows(self, xs, rows, stream=None):
-        "Fold rows `rows` of xs [n_inst, T, N] in order."
+        """Fold rows `rows` of xs [n_inst, T, N] in order; evenly spaced rows
+        of a float32 tensor (a range, usually) in one call."""
+        rows = list(rows)
+        if (len(rows) > 1 and xs.dim() == 3 and xs.dtype == self.torch.float32 and xs.is_cuda
+                and (xs.shape[0], xs.shape[2]) == (self.n_inst, self.N)
+                and xs.stride(2) == 1 and xs.stride(0) >= self.N):
+            idx = [range(xs.shape[1])[r] for r in rows]     # negative rows, IndexError
+            step = idx[1] - idx[0]
+            if idx == list(range(idx[0], idx[0] + step * len(idx), step) if step else idx[:1] * len(idx)):
+                lib = nat.load()
+                nat.check(lib.tvbg_cov_update_rows(
+                    xs.data_ptr() + 4 * idx[0] * xs.stride(1), xs.stride(0), step * xs.stride(1),
+                    len(idx), self.n_inst, self.N, self.n, self.mean.data_ptr(), self.m2.data_ptr(),
+                    nat.stream_handle(stream)))
+                self.n += len(idx)
+                return
         for r in rows:
             self.update(xs[:, r, :], stream)
 
