@@ -450,6 +450,19 @@ int tvbg_net_run(const tvbg_net *net, int64_t t0, int32_t nsteps,
                  const tvbg_launch *cfg, void *stream);
 
 /*
+ * The same run, the same results, with blocks of 8 steps launched together:
+ * dmin = the smallest delay (0: not known), d_stage = device buffer of
+ * stage_floats floats.  With cfg->block_k = cfg->tpn = 8, J = 3 (dmin >= 23,
+ * stage_floats >= 24 N) or J = 2 (dmin >= 15, 16 N) blocks share a launch: an
+ * edge's run of 8 J slots and its record are read once, the new slots go to
+ * d_stage ([N][8 J]) and a copy launch writes them to the ring.  Otherwise as
+ * tvbg_net_run.  Graph-capturable.
+ */
+int tvbg_net_run_ex(const tvbg_net *net, int64_t t0, int32_t nsteps,
+                    const tvbg_launch *cfg, int32_t dmin, float *d_stage,
+                    int64_t stage_floats, void *stream);
+
+/*
  * Streaming covariance for long runs: fold one sample per instance into an
  * FP64 running state (Welford update).  d_x: sample of instance b at
  * d_x + b * x_stride (N floats); n: samples already folded (0 starts a new

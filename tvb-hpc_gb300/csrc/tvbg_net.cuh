@@ -225,6 +225,129 @@ __global__ void __launch_bounds__(256)
     (void)status;
 }
 
+// J blocks of 8 steps per launch, 8 lanes per node: lane k sums the steps
+// tb + k, tb + 8 + k, ..., so an edge reads one run of 8 J slots (32 J bytes) and
+// its record once.  A random source's run costs DRAM about (8 J + 15) / 16 chunks
+// of 64 bytes, so longer runs move fewer bytes a step: about 100 with J = 1, 67
+// with J = 2, 55 with J = 3, the edge records included.  Needs every delay >=
+// 8 J - 1.  The ring is not written: the new slots go to stage[n][8 J] and
+// net_copy_kernel puts them in place, so nh > d_max is enough (a run wraps at
+// nh slot by slot).  515 056 nodes, 64 edges a node, 24 steps: 2.62 ms with
+// one block per launch.
+template <class M, int CF, int J>
+__global__ void __launch_bounds__(256)
+    net_kernel_wide(const tvbg_net g, long long tb, int cnt, float* __restrict__ stage) {
+    constexpr int K = 8;
+    constexpr int NS = M::NS;
+    constexpr int NP = M::NP;
+    constexpr int SPC = Noise<M>::SPC;
+    constexpr int U = J == 1 ? 8 : (J == 2 ? 6 : 4);  // edges in flight per lane
+    const long long gid = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
+    const long long n = gid / K;
+    const int k = static_cast<int>(threadIdx.x & (K - 1));
+    if (n >= g.N) return;   // blockDim is a multiple of 32: a node's lanes leave together
+    const unsigned gmask = ((1u << K) - 1u) << ((threadIdx.x & 31u) & ~static_cast<unsigned>(K - 1));
+    const uint32_t nh = 1u << g.lognh;
+    const uint32_t mask = nh - 1u;
+    const uint32_t R = nh + kGhost;
+    const uint32_t tm = (static_cast<uint32_t>(tb) + static_cast<uint32_t>(k)) & mask;
+    const bool noise = (g.flags & TVBG_F_NOISE) != 0;
+    float acc[J];
+#pragma unroll
+    for (int j = 0; j < J; ++j) acc[j] = 0.0f;
+    const long long lo = __ldg(g.row + n), hi = __ldg(g.row + n + 1);
+    for (long long e = lo; e < hi; e += U) {
+        float v[U][J], w[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) {   // past the last edge: that edge again, its product dropped
+            const long long q = e + u < hi ? e + u : hi - 1;
+            const float* p = g.ring + static_cast<size_t>(__ldg(g.col + q)) * R;
+            const uint32_t pos = tm + __ldg(g.off + q);
+            w[u] = __ldg(g.w + q);
+#pragma unroll
+            for (int j = 0; j < J; ++j) v[u][j] = __ldg(p + ((pos + 8 * j) & mask));
+        }
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            if (e + u < hi) {
+#pragma unroll
+                for (int j = 0; j < J; ++j) acc[j] = fmaf(w[u], lane_pre<CF>(v[u][j], g.cf_p), acc[j]);
+            }
+        }
+    }
+    float x[NS], p[NP];
+#pragma unroll
+    for (int v = 0; v < NS; ++v) x[v] = g.state[n * NS + v];
+#pragma unroll
+    for (int v = 0; v < NP; ++v) p[v] = __ldg(g.nparam + n * NP + v);
+    const float wsum = (CF == TVBG_CFUN_DIFF && g.wsum) ? __ldg(g.wsum + n) : 0.0f;
+    float obs0 = M::obs(x, 0);
+#pragma unroll
+    for (int j = 0; j < J; ++j) {
+        // the normals of step tb + 8 j + k, drawn by lane k
+        float zk[NS];
+#pragma unroll
+        for (int v = 0; v < NS; ++v) zk[v] = 0.0f;
+        if constexpr (Noise<M>::kOK) {
+            if (noise && 8 * j + k < cnt) {
+                const long long t = tb + 8 * j + k;
+                const int r0 = static_cast<int>(t & (SPC - 1));
+                const u32x4 w = philox4x32_10(static_cast<uint32_t>(n), static_cast<uint32_t>(t / SPC),
+                                              g.seed_hi, 0u, g.seed_lo, 0u);
+                float zz[4];
+                box_muller_fast(w.v[0], w.v[1], zz[0], zz[1]);
+                box_muller_fast(w.v[2], w.v[3], zz[2], zz[3]);
+#pragma unroll
+                for (int v = 0; v < NS; ++v) zk[v] = pick4(zz, r0 * NS + v);
+            }
+        }
+        float mine = 0.0f;
+#pragma unroll
+        for (int s = 0; s < K; ++s) {
+            if (8 * j + s < cnt) {
+                const float S = __shfl_sync(gmask, acc[j], s, K);
+                const float c = lane_post<CF>(S, obs0, wsum, g.cf_a, g.cf_b);
+                float f[NS];
+                M::drift(x, c, p, g.consts, f);
+#pragma unroll
+                for (int v = 0; v < NS; ++v) x[v] = fmaf(g.dt, f[v], x[v]);
+                if constexpr (Noise<M>::kOK) {
+                    if (noise) {
+#pragma unroll
+                        for (int v = 0; v < NS; ++v) {
+                            const float zv = __shfl_sync(gmask, zk[v], s, K);
+                            x[v] = fmaf(g.sqrt_dt * zv, g.sigma[v], x[v]);
+                        }
+                    }
+                }
+                M::limit(x, g.flags);
+                obs0 = M::obs(x, 0);
+                if (k == s) mine = obs0;
+            }
+        }
+        stage[n * (8 * J) + 8 * j + k] = mine;
+    }
+    if (k == 0) {
+#pragma unroll
+        for (int v = 0; v < NS; ++v) g.state[n * NS + v] = x[v];
+    }
+}
+
+// Slots tb + 1 .. tb + cnt of every node from stage[n][W].
+__global__ void __launch_bounds__(256)
+    net_copy_kernel(const tvbg_net g, long long tb, int cnt, int W, const float* __restrict__ stage) {
+    const long long e = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
+    const long long n = e / W;
+    const int s = static_cast<int>(e - n * W);
+    if (n >= g.N || s >= cnt) return;
+    const uint32_t nh = 1u << g.lognh;
+    const uint32_t pos = (static_cast<uint32_t>(tb + s) + 1u) & (nh - 1u);
+    float* rrow = g.ring + static_cast<size_t>(n) * (nh + kGhost);
+    const float v = __ldg(stage + e);
+    rrow[pos] = v;
+    if (pos < kGhost) rrow[pos + nh] = v;
+}
+
 // Seed slot t0 of every node with obs0 of its state.
 template <class M>
 __global__ void net_seed_kernel(const tvbg_net g, long long t0) {

@@ -5,8 +5,9 @@ linear coupling, CSR connectivity), where instances cannot fill the GPU and
 the parallelism is over nodes.
 
 The history ring is node-major ([N][nh + 8]) so the K slots an edge reads
-in a block of K steps are contiguous; one kernel launch per block (the
-launch boundary is the grid-wide barrier).  Either K lanes per node (lane k
+in a block of K steps are contiguous; one kernel launch per block, or per
+two or three blocks where the delays allow (the launch boundary is the
+grid-wide barrier).  Either K lanes per node (lane k
 gathers step k, one contiguous load per edge across the lanes; the default)
 or one thread per node; both give bit-identical results.  The step is the
 CUDA-order step of the other kernels, and the noise is instance 0's Philox
@@ -96,6 +97,13 @@ class SingleNetwork:
         self.lanes = bool(lanes)
         self.t = int(t0)
         self.status = DeviceStatus()
+        # delays of 15 or 23 steps and more: 2 or 3 blocks of 8 steps per launch,
+        # their new slots staged here (tvbg_net_run_ex)
+        self.dmin = int(d.min()) if d.size else 0
+        blocks = (3 if self.dmin >= 23 else 2 if self.dmin >= 15 else 1) \
+            if self.lanes and self.block_k == 8 else 1
+        self._stage = (torch.empty(N * 8 * blocks, dtype=torch.float32, device=dev) if blocks > 1
+                       else None)
 
     def descriptor(self):
         d = nat.tvbg_net()
@@ -122,8 +130,10 @@ class SingleNetwork:
         cfg.tpn = self.block_k if self.lanes else 1
         cfg.d_status = self.status.t.data_ptr()
         d = self.descriptor()
-        nat.check(lib.tvbg_net_run(ctypes.byref(d), self.t, int(nsteps), ctypes.byref(cfg),
-                                   nat.stream_handle(stream)))
+        st = self._stage
+        nat.check(lib.tvbg_net_run_ex(ctypes.byref(d), self.t, int(nsteps), ctypes.byref(cfg),
+                                      self.dmin, nat.ptr(st), 0 if st is None else st.numel(),
+                                      nat.stream_handle(stream)))
         self.t += int(nsteps)
 
     def run(self, nsteps, stream=None, check=True):
