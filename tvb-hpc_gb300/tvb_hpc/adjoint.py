@@ -240,15 +240,13 @@ class FCFit:
 
     def _groups(self, G, eta, trace_len, trace_nobs, trace_csum):
         "Lane-interleaved groups of the I instances on the pipelined kernel."
-        from .groups import GroupSet, pipelined_shape, PIPELINED
+        from .groups import GroupSet, spread_shape, PIPELINED
         gs = GroupSet(self.model, self.cfun, self.scheme, self.conn, dt=self.dt,
                       couplings=np.asarray(G, np.float32), speeds=self.speed, state0=self.x0,
                       nparam=np.asarray(eta, np.float32).reshape(self.I, self.N, 1),
                       rounding=self.rounding, trace_every=1, trace_len=trace_len,
                       trace_nobs=trace_nobs, trace_csum=trace_csum)
-        sms = self.torch.cuda.get_device_properties(
-            self.torch.cuda.current_device()).multi_processor_count
-        shape = pipelined_shape(gs, min_ctas=sms)
+        shape = spread_shape(gs)
         assert shape[3] == PIPELINED
         gs.set_shape(*shape)
         return gs

@@ -218,7 +218,7 @@ def tune_group_batch(sets, nsteps, trial_max_steps=4096, passes=2, reps=2, verif
     if key in _GROUP_CACHE:
         return _GROUP_CACHE[key]
     small, scale = _scaled(nsteps, trial_max_steps)
-    default = [(s.threads, s.cluster, 0, 1) for s in sets]
+    default = [(s.threads, s.cluster, 0, s.tpn) for s in sets]
     snap = _snapshot(sets)
     trials = []
     try:

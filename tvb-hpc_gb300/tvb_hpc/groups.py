@@ -100,6 +100,68 @@ def group_shape(N, threads=None, cluster=None):
     return int(threads), int(cluster)
 
 
+def plain_shape(N, n_groups, sms, max_cluster=8):
+    """(threads, cluster) of the plain kernel for n_groups groups: group_shape,
+    spread over more CTAs of at least 192 threads while all of them fit one
+    per SM (measured, 400 steps: N = 84, up to 32 groups, 672 x 1 0.42 ms, 192 x 4
+    0.25, 96 x 8 0.30; N = 192, 768 x 2 0.51, 192 x 8 0.28; N = 400, 800 x 4 0.62,
+    416 x 8 0.42; at 128 groups of N = 84 one CTA each is as good)."""
+    threads, cluster = group_shape(N)
+    for c in range(cluster + 1, max_cluster + 1):
+        t = 32 * -(-(L * -(-N // c)) // 32)
+        if t >= 192 and n_groups * c <= sms and c in (2, 3, 4, 6, 8):
+            threads, cluster = t, c
+    return threads, cluster
+
+
+def spread_shape(gset, sms=None):
+    """
+    (threads, cluster, 0, tpn): the default launch shape of a set.  The
+    pipelined kernel where some delay table allows it:
+      - the largest cluster whose CTAs fit one per SM, all groups resident at
+        once (the chain of one group bounds the run: N = 84, 32 groups, 400
+        steps: 704 x 2 0.216 ms, 448 x 3 0.164, 384 x 4 0.150, and 0.170 for 256 x 6,
+        whose 192 CTAs share SMs; plain 672 x 1 0.427);
+      - with more groups the smallest cluster whose CTAs the build with more
+        registers takes (768 threads, 512 with two ring channels; clusters of
+        12 leave SMs of a GPC idle): throughput then depends little on the
+        shape (N = 84, 400 groups: 1.39 to 1.49 ms, plain 1.57; N = 192: 1024 x 3
+        4.44, 768 x 4 3.45, 512 x 6 3.28).
+    Two-channel rings whose CTAs exceed the 768-thread build stay on the plain
+    kernel (Kuramoto, N = 998, 10 groups: 1.97 ms against 2.36).
+    """
+    from .autotune import group_max_clusters
+    if sms is None:
+        sms = device_sms()
+    G = gset.n_groups
+    plain = plain_shape(gset.N, G, sms) + (0, 1)
+    if not (gset.can_pipeline and gset.pipelined_built):
+        return plain
+    shapes = []
+    for c in (1, 2, 3, 4, 6, 8, 12, 16):
+        t = pipelined_threads(gset.N, c)
+        if t and (not shapes or 256 <= t < shapes[-1][0]):
+            shapes.append((t, c, 0, PIPELINED))
+    if not shapes:
+        return plain
+    live = int(gset.pipe_tab[gset.gtab].sum())
+    for t, c, _, tpn in reversed(shapes):
+        if G * c <= sms and group_max_clusters(gset, t, c, tpn) >= live:
+            return (t, c, 0, PIPELINED)
+    limit = 768 if gset.channels == 1 else 512
+    fits = [s for s in shapes if s[0] <= limit and s[1] != 12]
+    if not fits and gset.channels == 2:
+        fits = [s for s in shapes if s[0] <= 768]
+        if not fits:
+            return plain
+    return fits[0] if fits else shapes[0]
+
+
+def device_sms():
+    torch = _torch()
+    return torch.cuda.get_device_properties(torch.cuda.current_device()).multi_processor_count
+
+
 def group_occupancy(cfg):
     lib = nat.load()
     per, sms = ctypes.c_int32(0), ctypes.c_int32(0)
@@ -124,7 +186,8 @@ class GroupSet:
       nsteps  : optional (I,) step counts, used to put instances of similar
                 length into the same group (longest first);
       block_k : 4 or 8 steps per barrier (default: 8 when d_min >= 7);
-      threads, cluster : launch shape (default: group_shape).
+      threads, cluster : plain launch shape (default: spread_shape, which
+                prefers the pipelined kernel; results do not depend on it).
     Couplings must be separable (Linear, Diff, Sigmoidal), or the Kuramoto
     coupling with the Kuramoto model (whose ring keeps sin and cos of the
     phase); the Track-A order runs on the per-instance kernels.
@@ -134,6 +197,7 @@ class GroupSet:
     """
 
     block_ks = (8, 4)     # block lengths the library's group kernels are built for
+    pipelined_built = True   # the library has the pipelined kernels
 
     def __init__(self, model, cfun, scheme, conn, dt, couplings, speeds=None, state0=None,
                  nparam=None, delays=None, rounding='ceil', seed=0, inst_ids=None,
@@ -302,6 +366,15 @@ class GroupSet:
         self.status = DeviceStatus()
         self._uploaded = None
         self._streams = None
+        # shape of the groups that stay on the plain kernel beside pipelined ones
+        self.plain = (self.threads, self.cluster)
+        if threads is None and cluster is None:
+            sms = device_sms()
+            self.plain = plain_shape(N, G, sms)
+            if self.trace_csum:    # asks for an explicit shape
+                self.threads, self.cluster = self.plain
+            else:
+                self.threads, self.cluster, _, self.tpn = spread_shape(self, sms)
 
     def bold_obs(self):
         """Observable feeding the balloon: sin(theta) for Kuramoto, V for G2DO
@@ -340,12 +413,8 @@ class GroupSet:
         """Zero history (every slot holds the observable 0): zeros, or with the
         Kuramoto coupling (sin 0, cos 0) = (0, 1) in every slot."""
         self.ring.zero_()
-        if self.channels == 2:
-            N = self.N
-            for g in range(self.n_groups):
-                R = int(self.R[g])
-                o = int(self.ring_off[g])
-                self.ring[o:o + N * R * L * 2].view(N, R, 2, L)[:, :, 1, :] = 1.0
+        if self.channels == 2:    # every group's ring is [N][R][2][8]
+            self.ring.view(-1, 2, L)[:, 1, :] = 1.0
 
     def fill_history(self):
         "Every ring slot of every lane holds obs0 of the current state."
@@ -449,7 +518,7 @@ class GroupSet:
         priority (0 = the stream's; lower numbers are dispatched first) and
         tpn = 2 for the pipelined kernel (threads then count both teams;
         needs one node per slot and a table with d_min >= 2 K - 1; groups of
-        the other tables keep the plain kernel on group_shape)."""
+        the other tables keep the plain kernel on their own shape)."""
         tpn = int(tpn)
         if tpn == PIPELINED:
             if not self.can_pipeline:
@@ -480,7 +549,7 @@ class GroupSet:
         cfg = nat.tvbg_launch()
         cfg.model, cfg.cfun = self.model_id, self.cfun_id
         if plain and self.tpn == PIPELINED:
-            cfg.threads, cfg.cluster = group_shape(self.N)
+            cfg.threads, cfg.cluster = self.plain
             cfg.tpn = 1
         else:
             cfg.threads, cfg.cluster = self.threads, self.cluster

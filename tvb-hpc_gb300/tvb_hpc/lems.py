@@ -1072,6 +1072,7 @@ class LemsGroupSet(GroupSet):
     """
 
     block_ks = (8, 4, 2, 1)   # the generated libraries build every block length
+    pipelined_built = False
 
     def __init__(self, m, conn, dt, params, state0=None, noise=None, single=False, **kwargs):
         self.lems = LemsLibrary(m, single)
