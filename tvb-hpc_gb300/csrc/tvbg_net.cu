@@ -113,7 +113,7 @@ extern "C" int tvbg_net_run_ex(const tvbg_net* net, int64_t t0, int32_t nsteps, 
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return set_cuda_error(e, "tvbg_net_run: seed launch");
     int J = 1;
-    if (d_stage && lanes == 8)
+    if (d_stage && lanes == 8 && cfg->threads <= 256)
         for (int j = 3; j >= 2 && J == 1; --j)
             if (dmin >= 8 * j - 1 && stage_floats >= net->N * static_cast<int64_t>(8 * j)) J = j;
     const WideKernel wfn = J > 1 ? lookup_wide(net->model, net->cfun, J) : nullptr;
