@@ -40,12 +40,14 @@ static StepKernel lookup(int model, int cfun, int tpn) {
     }
 }
 
-static BlockedKernel lookup_blocked(int model, int cfun, int tpn, int k) {
+static BlockedKernel lookup_blocked(int model, int cfun, int tpn, int k, int threads, size_t smem) {
+    // two CTAs do not fit one SM: registers are free
+    const bool wide = threads <= 512 && smem > 113u * 1024u;
     switch (model) {
-        case TVBG_MODEL_G2DO: return blocked_kernel_g2do(cfun, tpn, k);
-        case TVBG_MODEL_MPR: return blocked_kernel_mpr(cfun, tpn, k);
-        case TVBG_MODEL_LINEAR: return blocked_kernel_linear(cfun, tpn, k);
-        case TVBG_MODEL_G2DOSC: return blocked_kernel_g2dosc(cfun, tpn, k);
+        case TVBG_MODEL_G2DO: return blocked_kernel_g2do(cfun, tpn, k, wide);
+        case TVBG_MODEL_MPR: return blocked_kernel_mpr(cfun, tpn, k, wide);
+        case TVBG_MODEL_LINEAR: return blocked_kernel_linear(cfun, tpn, k, wide);
+        case TVBG_MODEL_G2DOSC: return blocked_kernel_g2dosc(cfun, tpn, k, wide);
         default: return nullptr;
     }
 }
@@ -71,12 +73,12 @@ static int launch_step(int model, int cfun, const tvbg_instance* d_inst, int32_t
     BlockedKernel kb = nullptr;
     size_t smem = 0;
     if (blocked) {
-        kb = lookup_blocked(model, cfun, cfg->tpn, cfg->block_k);
+        smem = static_cast<size_t>(cfg->smem_ring) + blocked_aux_bytes(model, cfg->block_k, nmax);
+        kb = lookup_blocked(model, cfun, cfg->tpn, cfg->block_k, cfg->threads, smem);
         if (!kb)
             return set_error(TVBG_EUNSUPPORTED,
                              "time-blocked kernel not built for this model/coupling/tpn/block_k");
         kfn = reinterpret_cast<const void*>(kb);
-        smem = static_cast<size_t>(cfg->smem_ring) + blocked_aux_bytes(model, cfg->block_k, nmax);
     } else {
         k1 = lookup(model, cfun, cfg->tpn);
         if (!k1) return set_error(TVBG_EUNSUPPORTED, "model/coupling pair not built into the library");
@@ -157,10 +159,10 @@ int tvbg_occupancy(const tvbg_launch* cfg, int32_t* ctas_per_sm, int32_t* sms) {
     const void* kfn = nullptr;
     size_t smem = 0;
     if (blocked) {
-        BlockedKernel kb = lookup_blocked(cfg->model, cfg->cfun, cfg->tpn, cfg->block_k);
+        smem = static_cast<size_t>(cfg->smem_ring) + blocked_aux_bytes(cfg->model, cfg->block_k, nmax);
+        BlockedKernel kb = lookup_blocked(cfg->model, cfg->cfun, cfg->tpn, cfg->block_k, cfg->threads, smem);
         if (!kb) return set_error(TVBG_EUNSUPPORTED, "time-blocked kernel not built");
         kfn = reinterpret_cast<const void*>(kb);
-        smem = static_cast<size_t>(cfg->smem_ring) + blocked_aux_bytes(cfg->model, cfg->block_k, nmax);
     } else {
         StepKernel k1 = lookup(cfg->model, cfg->cfun, cfg->tpn);
         if (!k1) return set_error(TVBG_EUNSUPPORTED, "model/coupling pair not built");

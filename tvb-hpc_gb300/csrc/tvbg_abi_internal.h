@@ -30,11 +30,13 @@ StepKernel step_kernel_linear(int cfun, int tpn);
 StepKernel step_kernel_g2dosc(int cfun, int tpn);
 StepKernel step_kernel_rww(int cfun, int tpn);
 StepKernel step_kernel_jansenrit(int cfun, int tpn);
-// Per-model lookup of the time-blocked kernel for (cfun, tpn, K); nullptr if not built.
-BlockedKernel blocked_kernel_g2do(int cfun, int tpn, int k);
-BlockedKernel blocked_kernel_mpr(int cfun, int tpn, int k);
-BlockedKernel blocked_kernel_linear(int cfun, int tpn, int k);
-BlockedKernel blocked_kernel_g2dosc(int cfun, int tpn, int k);
+// Per-model lookup of the time-blocked kernel for (cfun, tpn, K); wide: the
+// build for CTAs of at most 512 threads that have an SM to themselves (128
+// registers a thread); nullptr if not built.
+BlockedKernel blocked_kernel_g2do(int cfun, int tpn, int k, bool wide);
+BlockedKernel blocked_kernel_mpr(int cfun, int tpn, int k, bool wide);
+BlockedKernel blocked_kernel_linear(int cfun, int tpn, int k, bool wide);
+BlockedKernel blocked_kernel_g2dosc(int cfun, int tpn, int k, bool wide);
 // Builds of a lane-interleaved group kernel: plain or pipelined, by the
 // largest CTA they take (registers a thread: 64, 80, 128).
 enum GroupForm { kPlain1024, kPlain768, kPipe1024, kPipe768, kPipe512 };

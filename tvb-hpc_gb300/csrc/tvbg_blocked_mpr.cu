@@ -5,30 +5,30 @@
 
 namespace tvbg {
 
-template <int CF, int K>
+template <int CF, int K, int BOUND>
 static BlockedKernel pick_tpn_b(int tpn) {
     switch (tpn) {
-        case 2: return blocked_kernel<MPR, CF, 2, K>;
-        case 4: return blocked_kernel<MPR, CF, 4, K>;
-        case 8: return blocked_kernel<MPR, CF, 8, K>;
+        case 2: return blocked_kernel<MPR, CF, 2, K, BOUND>;
+        case 4: return blocked_kernel<MPR, CF, 4, K, BOUND>;
+        case 8: return blocked_kernel<MPR, CF, 8, K, BOUND>;
         default: return nullptr;
     }
 }
 
 template <int CF>
-static BlockedKernel pick_k(int tpn, int k) {
+static BlockedKernel pick_k(int tpn, int k, bool wide) {
     switch (k) {
-        case 4: return pick_tpn_b<CF, 4>(tpn);
-        case 8: return pick_tpn_b<CF, 8>(tpn);
+        case 4: return wide ? pick_tpn_b<CF, 4, 512>(tpn) : pick_tpn_b<CF, 4, 1024>(tpn);
+        case 8: return wide ? pick_tpn_b<CF, 8, 512>(tpn) : pick_tpn_b<CF, 8, 1024>(tpn);
         default: return nullptr;
     }
 }
 
-BlockedKernel blocked_kernel_mpr(int cfun, int tpn, int k) {
+BlockedKernel blocked_kernel_mpr(int cfun, int tpn, int k, bool wide) {
     switch (cfun) {
-        case TVBG_CFUN_LINEAR: return pick_k<TVBG_CFUN_LINEAR>(tpn, k);
-        case TVBG_CFUN_DIFF: return pick_k<TVBG_CFUN_DIFF>(tpn, k);
-        case TVBG_CFUN_SIGMOIDAL: return pick_k<TVBG_CFUN_SIGMOIDAL>(tpn, k);
+        case TVBG_CFUN_LINEAR: return pick_k<TVBG_CFUN_LINEAR>(tpn, k, wide);
+        case TVBG_CFUN_DIFF: return pick_k<TVBG_CFUN_DIFF>(tpn, k, wide);
+        case TVBG_CFUN_SIGMOIDAL: return pick_k<TVBG_CFUN_SIGMOIDAL>(tpn, k, wide);
         default: return nullptr;
     }
 }

@@ -340,6 +340,11 @@ class InstanceSet:
         cap = max_smem()
         self.ring_bytes = N * self.stride * 4
         self.smem_cap = cap
+        # staged rings of more than half the shared memory leave one CTA per SM:
+        # the blocked kernel then takes 512 threads, mostly gathering warps
+        # (results do not depend on it)
+        self._one_cta = any(2 * r > cap and r <= self.smem_ring_limit(0, k)
+                            for r, k in set(zip(self.ring_bytes.tolist(), self.block_k.tolist())) if k)
         self.table = None
         self.table_dev = None
 
@@ -360,7 +365,7 @@ class InstanceSet:
         if blocked_k and self.warps:
             return min(1024, max(own + 32, 32 * int(self.warps)))
         if blocked_k:
-            return min(1024, max(own + 32, 256))
+            return min(1024, max(own + 32, 512 if self._one_cta else 256))
         return own
 
     def smem_ring_limit(self, threads, blocked_k=0):
