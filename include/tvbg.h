@@ -491,6 +491,18 @@ int tvbg_cov_corr(const double *d_m2, int32_t n_inst, int32_t N, float *d_corr,
                   void *stream);
 
 /*
+ * Rings of the per-instance kernels from a time buffer (the executor's obsrv,
+ * transforms.py:30-42): slot t of node j of instance b takes
+ * d_obs[t mod ntime][b][j][0] ([ntime][n_inst][N][nobs] floats) for t in
+ * [t_lo, t_hi), every other slot 0; d_ring: [n_inst][N << lognh], skewed
+ * node-major (slot t of node j at j nh + ((t + j) & (nh - 1))).  Needs
+ * t_hi - t_lo <= nh.
+ */
+int tvbg_ring_from_obs(const float *d_obs, int32_t ntime, int32_t n_inst,
+                       int32_t N, int32_t nobs, int64_t t_lo, int64_t t_hi,
+                       int32_t lognh, float *d_ring, void *stream);
+
+/*
  * Fill d_out[0..n) with standard normals from Philox4x32-10 (Salmon et al.
  * 2011) + Box-Muller: key = (seed_lo, stream_id), counter = (i/4, 0,
  * seed_hi, 0) for output i.  Replaces tvb_hpc/rng.py:30-96 (RNG.fill).

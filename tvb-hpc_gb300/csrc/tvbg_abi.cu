@@ -118,6 +118,28 @@ __global__ void philox_normal_kernel(uint32_t k0, uint32_t k1, uint32_t c2, floa
     }
 }
 
+// Skewed node-major rings from rows of a time buffer: slot t of node j of
+// instance b holds obs[t mod ntime][b][j][0] for t in [t_lo, t_hi), 0 elsewhere.
+__global__ void __launch_bounds__(256)
+    ring_from_obs_kernel(const float* __restrict__ obs, int ntime, int n_inst, int N, int nobs, long long t_lo,
+                         int rows, int lognh, long long total, float* __restrict__ ring) {
+    const long long e = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
+    if (e >= total) return;
+    const int nh = 1 << lognh;
+    const long long bj = e >> lognh;
+    const int j = static_cast<int>(bj % N);
+    const long long b = bj / N;
+    const int slot = (static_cast<int>(e & (nh - 1)) - j) & (nh - 1);
+    const int k = (slot - static_cast<int>(t_lo & (nh - 1))) & (nh - 1);   // t = t_lo + k
+    float v = 0.0f;
+    if (k < rows) {
+        long long r = (t_lo + k) % ntime;
+        if (r < 0) r += ntime;
+        v = __ldg(obs + ((r * n_inst + b) * N + j) * nobs);
+    }
+    ring[e] = v;
+}
+
 __global__ void philox_u32_kernel(uint32_t k0, uint32_t k1, uint32_t c1, uint32_t c2, uint32_t c3,
                                   uint32_t* __restrict__ out, long long nb) {
     for (long long b = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; b < nb;
@@ -274,6 +296,20 @@ int tvbg_batch_run(const tvbg_instance* d_inst, int32_t n_inst, const tvbg_launc
     if (rc) return rc;
     if (n_inst == 0) return TVBG_OK;
     return launch_step(cfg->model, cfg->cfun, d_inst, n_inst, cfg, true, stream);
+}
+
+int tvbg_ring_from_obs(const float* d_obs, int32_t ntime, int32_t n_inst, int32_t N, int32_t nobs,
+                       int64_t t_lo, int64_t t_hi, int32_t lognh, float* d_ring, void* stream) {
+    if (!d_obs || !d_ring || ntime < 1 || n_inst < 1 || N < 1 || nobs < 1 || lognh < 2 || lognh > 30 ||
+        t_hi < t_lo || t_hi - t_lo > (1LL << lognh))
+        return set_error(TVBG_EINVAL, "tvbg_ring_from_obs: bad arguments");
+    const long long total = (static_cast<long long>(n_inst) * N) << lognh;
+    const long long blocks = (total + 255) / 256;
+    if (blocks > 0x7fffffffLL) return set_error(TVBG_EINVAL, "tvbg_ring_from_obs: rings too large");
+    ring_from_obs_kernel<<<static_cast<unsigned>(blocks), 256, 0, static_cast<cudaStream_t>(stream)>>>(
+        d_obs, ntime, n_inst, N, nobs, t_lo, static_cast<int>(t_hi - t_lo), lognh, total, d_ring);
+    const cudaError_t e = cudaGetLastError();
+    return e == cudaSuccess ? TVBG_OK : set_cuda_error(e, "tvbg_ring_from_obs launch");
 }
 
 int tvbg_philox_normal(uint64_t seed, uint32_t stream_id, float* d_out, int64_t n, void* stream) {

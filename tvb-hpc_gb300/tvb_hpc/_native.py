@@ -255,6 +255,7 @@ SIGNATURES = {
     'tvbg_adjoint_mpr_ex': (ctypes.c_int, [_vp, _i32, _i32, _i32, _vp]),
     'tvbg_adjoint_group_size': (_sz, []),
     'tvbg_adjoint_mpr_groups': (ctypes.c_int, [_vp, _i32, _i32, _i32, _i32, _i32, _vp, _vp]),
+    'tvbg_ring_from_obs': (ctypes.c_int, [_vp, _i32, _i32, _i32, _i32, _i64, _i64, _i32, _vp, _vp]),
     'tvbg_philox_u32': (ctypes.c_int, [_u32, _u32, _u32, _u32, _u32, _vp, _i64, _vp]),
     'tvbg_group_size': (_sz, []),
     'tvbg_net_run_ex': (ctypes.c_int, [ctypes.POINTER(tvbg_net), _i64, _i32, ctypes.POINTER(tvbg_launch), _i32, _vp,

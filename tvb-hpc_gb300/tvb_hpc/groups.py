@@ -568,23 +568,27 @@ class GroupSet:
         CTAs of long groups first.  Returns the launch list."""
         torch = self.torch
         tab, gmax = self.build_table(nsteps)
-        dev = torch.from_numpy(tab.view(np.uint8).copy()).cuda()
         prio = (np.full(self.n_groups, self.priority, np.int64) if priorities is None
                 else np.asarray(priorities, np.int64))
         pipe = self.pipe_tab[self.gtab] if self.tpn == PIPELINED else np.ones(self.n_groups, bool)
         if self.trace_csum and (self.tpn != PIPELINED or not pipe.all()):
             raise ValueError('trace_csum: every group on the pipelined kernel (set_shape tpn=2, '
                              'delays >= 2 K - 1)')
-        launches = []
+        parts = []
         for k in sorted(set(self.block_k.tolist())):
             for pk in (True, False):
                 sel = (self.block_k == k) & (pipe == pk)
                 for pr in sorted(set(prio[sel].tolist())):
                     idx = np.nonzero(sel & (prio == pr))[0]
-                    idx = idx[np.argsort(-gmax[idx], kind='stable')].astype(np.int32)
-                    order = torch.from_numpy(idx).cuda()
-                    launches.append((dev, order, int(idx.size),
-                                     self.launch_cfg(k, order, pr, plain=not pk)))
+                    parts.append((idx[np.argsort(-gmax[idx], kind='stable')].astype(np.int32), k, pk, pr))
+        # the table and the launch orders in one upload
+        dev = torch.from_numpy(np.concatenate(
+            [tab.view(np.uint8).reshape(-1)] + [p[0].view(np.uint8) for p in parts])).cuda()
+        launches, o = [], tab.nbytes
+        for idx, k, pk, pr in parts:
+            order = dev[o:o + idx.nbytes].view(torch.int32)
+            o += idx.nbytes
+            launches.append((dev, order, int(idx.size), self.launch_cfg(k, order, pr, plain=not pk)))
         self._uploaded = (launches, gmax)
         return launches, gmax
 
