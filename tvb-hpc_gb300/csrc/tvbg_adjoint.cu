@@ -17,35 +17,61 @@ namespace tvbg {
 // the same numbers.  adj_mu_r: mu_r(t+1) = lambda_r(t+1), masked where the
 // rate update of step t was clamped at 0 (rpre as MPR::drift computes it).
 struct AdjMpr {
-    float Delta, J, tau, dt;
+    float J, tau, dt;
+    float f0, itau, c2;   // Delta / (pi tau), 1 / tau, 2 pi^2 tau^2
+    double c;             // dt / tau
+
+    __device__ __forceinline__ AdjMpr(const float* consts, float dt_) : J(consts[1]), tau(consts[2]), dt(dt_) {
+        const float pi = 3.14159265358979323846f;
+        f0 = consts[0] / (pi * tau);
+        itau = 1.0f / tau;
+        c2 = __fmul_rn(__fmul_rn(__fmul_rn(__fmul_rn(2.0f, pi), pi), tau), tau);
+        c = static_cast<double>(__fdiv_rn(dt, tau));
+    }
 
     __device__ __forceinline__ float mu_r(float r, float V, float lr) const {
-        const float pi = 3.14159265358979323846f;
-        const float fr = (Delta / (pi * tau) + 2.0f * r * V) * (1.0f / tau);  // as MPR::drift
-        const float rpre = fmaf(dt, fr, r);
+        const float fr = __fmul_rn(__fmaf_rn(__fmul_rn(2.0f, r), V, f0), itau);  // as MPR::drift
+        const float rpre = __fmaf_rn(dt, fr, r);
         return rpre >= 0.0f ? lr : 0.0f;
     }
 
     // lambda(t) from mu(t+1) = (mr, mv), the coupling gather and dL/dr(t).
     // Every rounding is spelled out (no contraction left to the compiler), so
-    // both kernels produce the same bits.
-    __device__ __forceinline__ void update(float r, float V, float S, float mr, float mv, float coup,
-                                           float cG, float drt, float& lr, float& lv, double& deta,
-                                           double& dG) const {
-        const float pi = 3.14159265358979323846f;
-        const float dfr_dr = __fdiv_rn(__fmul_rn(2.0f, V), tau);  // = dfV_dV
-        const float dfr_dV = __fdiv_rn(__fmul_rn(2.0f, r), tau);
-        const float c2 = __fmul_rn(__fmul_rn(__fmul_rn(__fmul_rn(2.0f, pi), pi), tau), tau);
-        const float dfV_dr = __fdiv_rn(__fsub_rn(__fmul_rn(J, tau), __fmul_rn(c2, r)), tau);
+    // both kernels produce the same bits.  UNIT: tau = 1 (the model's
+    // default), where x / tau is x and the three divisions of a step, each a
+    // reciprocal with its correction, go.
+    template <bool UNIT>
+    __device__ __forceinline__ void update(float r, float V, float mr, float mv, float coup,
+                                           float cG, float drt, float& lr, float& lv) const {
+        const auto over_tau = [&](float x) { return UNIT ? x : __fdiv_rn(x, tau); };
+        const float dfr_dr = over_tau(__fmul_rn(2.0f, V));  // = dfV_dV
+        const float dfr_dV = over_tau(__fmul_rn(2.0f, r));
+        const float dfV_dr = over_tau(__fsub_rn(__fmul_rn(J, tau), __fmul_rn(c2, r)));
         float nlr = __fmaf_rn(dt, __fmaf_rn(mv, dfV_dr, __fmul_rn(mr, dfr_dr)), mr);
         nlr = __fmaf_rn(cG, coup, nlr);
         const float nlv = __fmaf_rn(dt, __fmaf_rn(mv, dfr_dr, __fmul_rn(mr, dfr_dV)), mv);
-        const double c = static_cast<double>(__fdiv_rn(dt, tau));
-        const double cm = __dmul_rn(c, static_cast<double>(mv));
-        deta = __dadd_rn(deta, cm);
-        dG = __fma_rn(cm, static_cast<double>(S), dG);
         lr = __fadd_rn(nlr, drt);
         lv = nlv;
+    }
+};
+
+// Partial sums of dL/deta and dL/dG over steps, without their common factor
+// dt / tau, which add() applies in one FMA: two FP64 operations a step (the
+// FP64 pipe does two a cycle and SM, 100 cycles for each operation of 21
+// nodes; with the factor in every step the group kernel took 987 us where it
+// takes 880, 84 nodes, 256 instances, 2000 steps).
+struct AdjSums {
+    double m = 0.0, mS = 0.0;
+
+    __device__ __forceinline__ void step(float mv, float S) {
+        const double d = static_cast<double>(mv);
+        m = __dadd_rn(m, d);
+        mS = __fma_rn(d, static_cast<double>(S), mS);
+    }
+    __device__ __forceinline__ void add(double c, double* deta, double* dG) {
+        *deta = __fma_rn(c, m, *deta);
+        *dG = __fma_rn(c, mS, *dG);
+        m = mS = 0.0;
     }
 };
 
@@ -74,10 +100,10 @@ __device__ __forceinline__ void adjoint_segment(const tvbg_adjoint& a, AdjRing<S
     const bool own = j < N;
     const uint32_t lognh = static_cast<uint32_t>(a.lognh);
     const uint32_t mask = (1u << lognh) - 1u;
-    const AdjMpr m{a.consts[0], a.consts[1], a.consts[2], a.dt};
+    const AdjMpr m(a.consts, a.dt);
     const float cG = a.dt * a.G / a.consts[2];
     float lr = 0.f, lv = 0.f;
-    double deta = 0.0, dG = 0.0;
+    AdjSums sums;
     int lo = 0, hi = 0;
     if (own) {
         lr = a.lam[2 * j];
@@ -121,16 +147,15 @@ __device__ __forceinline__ void adjoint_segment(const tvbg_adjoint& a, AdjRing<S
                 const uint2 ew = __ldg(edges + e);
                 coup = fmaf(__uint_as_float(ew.y), ring.ld(((tm + ew.x) & mask) | (ew.x & ~mask)), coup);
             }
-            m.update(r, V, S, mr, mv, coup, cG, a.dr[static_cast<long long>(k) * N + j], lr, lv, deta,
-                     dG);
+            m.update<false>(r, V, mr, mv, coup, cG, a.dr[static_cast<long long>(k) * N + j], lr, lv);
+            sums.step(mv, S);
         }
         __syncthreads();
     }
     if (own) {
         a.lam[2 * j] = lr;
         a.lam[2 * j + 1] = lv;
-        a.deta[j] += deta;
-        a.dG[j] += dG;
+        sums.add(m.c, a.deta + j, a.dG + j);
     }
 }
 
@@ -156,82 +181,41 @@ __global__ void __launch_bounds__(1024, 1)
 // Lane-interleaved groups, time-blocked
 // ---------------------------------------------------------------------------
 
-// Out-edge sums of node slot (lanes l = 0..7) for the K reverse steps of a
-// block: lane l loads ring positions tm + d + (l % K) of NI instances
-// (32 contiguous bytes for K = 8) and accumulates pairs of instances with
-// the packed FMA (each half rounded as fmaf), edges in out-edge order.  The
-// sum of step ks, instance m lands at cs[ks * stride + m] (cs: the slot's
-// first thread).  U edges per iteration: 8 loads of 16 bytes in flight.
-template <int K>
-__device__ __forceinline__ void adj_gather(const float* __restrict__ ring_g,
-                                           const uint2* __restrict__ edges, int lo, int hi,
-                                           uint32_t tm, uint32_t mask, uint32_t R, int l, float* cs,
-                                           int stride) {
-    static_assert(K == 4 || K == 8, "adjoint group gather: K = 4 or 8");
-    constexpr int NI = K == 8 ? 8 : 4;  // instances per lane
-    constexpr int NV = NI / 4;          // 16-byte loads per edge
-    constexpr int U = 8 / NV;
-    const int ks = l % K;
-    const int m0 = (l / K) * NI;
-    const float* __restrict__ ring = ring_g + m0;
-    float2 acc[NI / 2];
-#pragma unroll
-    for (int i = 0; i < NI / 2; ++i) acc[i] = make_float2(0.0f, 0.0f);
-    for (int e = lo; e < hi; e += U) {
-        float4 v[U][NV];
-        float w[U];
-#pragma unroll
-        for (int u = 0; u < U; ++u) {
-            if (e + u < hi) {
-                const uint2 ed = __ldg(edges + e + u);
-                const float4* p = reinterpret_cast<const float4*>(
-                    ring + (static_cast<size_t>(ed.x >> 16) * R + (((tm + (ed.x & 0xffffu)) & mask) + ks)) * kLanes);
-                w[u] = __uint_as_float(ed.y);
-#pragma unroll
-                for (int j = 0; j < NV; ++j) v[u][j] = __ldcg(p + j);
-            }
-        }
-#pragma unroll
-        for (int u = 0; u < U; ++u) {
-            if (e + u < hi) {
-                const float2 ww = make_float2(w[u], w[u]);
-#pragma unroll
-                for (int j = 0; j < NV; ++j) {
-                    acc[2 * j] = __ffma2_rn(ww, make_float2(v[u][j].x, v[u][j].y), acc[2 * j]);
-                    acc[2 * j + 1] = __ffma2_rn(ww, make_float2(v[u][j].z, v[u][j].w), acc[2 * j + 1]);
-                }
-            }
-        }
-    }
-#pragma unroll
-    for (int i = 0; i < NI / 2; ++i) {
-        cs[ks * stride + m0 + 2 * i] = acc[i].x;
-        cs[ks * stride + m0 + 2 * i + 1] = acc[i].y;
-    }
-}
-
 // One group per CTA (or cluster of C CTAs): thread t of CTA r is lane
 // l = t % 8 of node slot q = (t / 8) C + r.  Per block of K reverse steps
 // (tb, tb - 1, ..., tb - K + 1): the gather of all K steps (reads slots
 // t + 1 + d >= tb + 2, written by earlier blocks since d >= K), then the K
 // updates from registers, each writing mu_V(t + 1) to slot t + 1, then one
 // barrier.  A slot written in a block aliases slot + nh, which no read of
-// the block reaches (nh >= d_max + K).
+// the block reaches (nh >= d_max + K).  The gather is the forward group
+// kernel's (gather_run over records staged in shared memory): the out-edge
+// records of a node are the in-edge records of the transposed network.
 //
 // PIPE: two thread teams of blockDim / 2 on the same (node slot, lane)
 // pairs; the update team runs block b from one coupling-sum buffer while
-// the gather team sums block b + 1 into the other, and the cluster meets at
-// one barrier per block.  Block b + 1 reads slots >= tb - 2K + 2 + d_min,
-// all written before block b started when d_min >= 2K; the slots block b
-// writes ([tb - K + 2, tb + 1]) alias none of them (nh > d_max - 1).  Each
-// team runs its own loop; both meet at the same number of barriers.  Same
-// per-step code and gather order: the same results.
+// the gather team sums block b + 1 into the other.  Block b + 1 reads slots
+// >= tb - 2K + 2 + d_min, all written before block b started when
+// d_min >= 2K; the slots block b writes ([tb - K + 2, tb + 1]) alias none of
+// them (nh > d_max - 1).  The CTAs of a cluster meet by ClusterPhases.  With
+// d_min >= 3K (lag) the gather of phase b reads nothing newer than block
+// b - 2, so a phase is published by one warp during the next one and awaited
+// at that one's end.  A CTA may then be one phase ahead, writing slots down
+// to tb - 2K + 2 while another reads up to tb - K + 1 + d_max: nh >= d_max + K
+// keeps them apart.  Same per-step code and gather order: the same results.
+//
+// What bounds it: the steps of the update team, their serial chain and FP64
+// sums (without the coupling gather the kernel takes the same time).  The
+// trace and dL/dr of a step come from DRAM; each step reads those of the
+// same step of the next block into the registers it has just used, so that
+// they have a block's time to arrive.
 template <int K, bool PIPE>
 __global__ void __launch_bounds__(512, 1)
     adjoint_group_kernel(const tvbg_adjoint_group* __restrict__ adj, int32_t n_groups,
                          int32_t* __restrict__ status) {
     __shared__ __align__(16) tvbg_adjoint_group s;
-    extern __shared__ __align__(16) float csum[];  // [(PIPE ? 2 : 1)][K][team threads]: out-edge sums
+    __shared__ EdgeStage stage;
+    __shared__ ClusterPhases phases;
+    extern __shared__ __align__(16) float csum[];  // [(PIPE ? 2 : 1)][K][team threads]: out-edge sums; records
     const int cid = static_cast<int>(cluster_id_x());
     if (cid >= n_groups) return;  // uniform over the cluster
     {
@@ -255,6 +239,7 @@ __global__ void __launch_bounds__(512, 1)
         if (threadIdx.x == 0) report(status, TVBG_EINVAL);
         return;  // uniform over the cluster: same record, same launch shape
     }
+    const bool lag = s.dmin >= 3 * K;
     const bool gather_team = PIPE && static_cast<int>(threadIdx.x) >= H;
     const int tid = static_cast<int>(threadIdx.x) - (gather_team ? H : 0);
     const int l = tid % kLanes;
@@ -265,94 +250,151 @@ __global__ void __launch_bounds__(512, 1)
     const uint32_t nh = 1u << s.lognh;
     const uint32_t mask = nh - 1u;
     const uint32_t R = nh + K;
+    float* const ring = s.ring;
     float* cs = csum + (tid - l);
     const int bufsz = K * H;
-    const uint2* __restrict__ edges = reinterpret_cast<const uint2*>(s.edges_t);
     const long long t0 = s.t0;
-    const long long top = t0 + s.len - 1;
-    int lo = 0, hi = 0;
-    if (!PIPE || gather_team) {
-        lo = valid ? __ldg(s.row_t + n) : 0;
-        hi = valid ? __ldg(s.row_t + n + 1) : 0;
-    }
+    const int len = s.len;
+    const long long top = t0 + len - 1;
+    const int lo = valid ? __ldg(s.row_t + n) : 0;
+    const int deg = valid ? __ldg(s.row_t + n + 1) - lo : 0;
+    if (PIPE && threadIdx.x == 0) phases.init(C);
+    // the gathering threads carry the slots (their tid is the scan's)
+    const uint2* edges = stage_edges(reinterpret_cast<const uint2*>(s.edges_t), stage,
+                                     reinterpret_cast<uint2*>(csum + (PIPE ? 2 : 1) * bufsz), P,
+                                     PIPE && !gather_team ? H + tid : tid, lo, deg);
+    const bool vec = run_vec<K, 1>(ring, N, R);
+    // out-edge sums of the K steps tb - K + 1 .. tb of this thread's slot
+    const auto gather = [&](long long tb, float* dst) {
+        const uint32_t tm = static_cast<uint32_t>(tb - K + 2) & mask;
+        if (vec)
+            gather_run<TVBG_CFUN_LINEAR, K, 1, true, PIPE ? 64 : 32>(ring, nullptr, edges, deg, tm, mask, R, l, dst, H);
+        else
+            gather_run_any<TVBG_CFUN_LINEAR, K, 1>(ring, nullptr, edges, deg, tm, mask, R, l, dst, H);
+    };
+    if (PIPE) group_barrier(cluster);  // the phases are initialised
     if (gather_team) {
-        if (s.len > 0)
-            adj_gather<K>(s.ring, edges, lo, hi, static_cast<uint32_t>(top - K + 2) & mask, mask, R, l, cs,
-                          H);
-        group_barrier(cluster);
-        int buf = 1;
+        // the last gather warp, whose nodes have the fewest edges, keeps the phases
+        const bool keeper = cluster && tid >= H - 32;
+        if (len > 0) gather(top, cs);
+        __syncthreads();
+        uint32_t ph = 0;  // phases ended
         for (long long tb = top; tb >= t0; tb -= K) {
-            if (tb - K >= t0)
-                adj_gather<K>(s.ring, edges, lo, hi, static_cast<uint32_t>(tb - 2 * K + 2) & mask, mask, R,
-                              l, cs + buf * bufsz, H);
-            buf ^= 1;
-            group_barrier(cluster);
+            if (keeper && lag && ph > 0) phases.publish(C);
+            if (tb - K >= t0) gather(tb - K, cs + ((ph + 1) & 1u) * bufsz);
+            if (keeper && lag && ph > 0) phases.await(ph - 1, ph);
+            __syncthreads();
+            if (cluster && !lag) {
+                if (keeper) {
+                    phases.publish(C);
+                    phases.await(ph, ph);
+                }
+                __syncthreads();
+            }
+            if (cluster && phases.failed(ph)) break;
+            ++ph;
         }
-        return;
-    }
-    const AdjMpr m{s.consts[0], s.consts[1], s.consts[2], s.dt};
-    const float cG = s.dt * s.G[l] / s.consts[2];
-    float lr = 0.0f, lv = 0.0f;
-    if (live) {
-        lr = s.lam[2LL * N * l + 2 * n];
-        lv = s.lam[2LL * N * l + 2 * n + 1];
-    }
-    double deta = 0.0, dG = 0.0;
-    float* __restrict__ ring_n = s.ring + static_cast<size_t>(n) * R * kLanes + l;
-    const float* __restrict__ seg_n = s.seg + static_cast<size_t>(n) * 3 * kLanes + l;
-    const float* __restrict__ dr_n = s.dr + s.dr_stride * l + n;
-    if (PIPE) group_barrier(cluster);  // block 0's sums
-    // partial sums of deta and dG go to memory after each step t with
-    // t % flush_every == 0 (the grouping of one launch per segment)
-    const long long fe = s.flush_every > 0 ? s.flush_every : 0;
-    long long next_flush = fe ? top - (top % fe) : t0 - 1;
-    bool pending = false;
-    int buf = 0;
-    for (long long tb = top; tb >= t0; tb -= K) {
-        const int cnt = (tb - t0 + 1) < K ? static_cast<int>(tb - t0 + 1) : K;
-        if (!PIPE) {
-            adj_gather<K>(s.ring, edges, lo, hi, static_cast<uint32_t>(tb - K + 2) & mask, mask, R, l, cs,
-                          H);
-            __syncwarp();
+    } else {
+        const AdjMpr m(s.consts, s.dt);
+        const float cG = s.dt * s.G[l] / s.consts[2];
+        float lr = 0.0f, lv = 0.0f;
+        if (live) {
+            lr = s.lam[2LL * N * l + 2 * n];
+            lv = s.lam[2LL * N * l + 2 * n + 1];
         }
-        const float* csb = cs + buf * bufsz;
+        AdjSums sums;
+        double* const deta_n = s.deta + static_cast<long long>(N) * l + n;
+        double* const dG_n = s.dG + static_cast<long long>(N) * l + n;
+        float* __restrict__ ring_n = ring + static_cast<size_t>(n) * R * kLanes + l;
+        // step t0 + k of this thread: r, V and S at seg_k, dL/dr at dr_k;
+        // read in the order of the steps, a block ahead of their use
+        const long long seg_row = 3LL * kLanes * N;
+        int kload = len - 1;
+        const float* __restrict__ seg_k = s.seg + (static_cast<size_t>(n) * 3 * kLanes + l) + kload * seg_row;
+        const float* __restrict__ dr_k = s.dr + s.dr_stride * l + n + static_cast<long long>(kload) * N;
+        float r[K], V[K], S[K], drt[K];
+        const auto load = [&](int i) {
+            if (kload >= 0) {
+                r[i] = __ldg(seg_k);
+                V[i] = __ldg(seg_k + kLanes);
+                S[i] = __ldg(seg_k + 2 * kLanes);
+                if (live) drt[i] = __ldg(dr_k);
+            }
+            seg_k -= seg_row;
+            dr_k -= N;
+            --kload;
+        };
 #pragma unroll
         for (int i = 0; i < K; ++i) {
-            if (i < cnt) {
-                const long long k = tb - i - t0;
-                const float* x = seg_n + static_cast<size_t>(k) * N * 3 * kLanes;
-                const float r = x[0], V = x[kLanes], S = x[2 * kLanes];
-                const float drt = live ? dr_n[k * N] : 0.0f;
-                const float mr = m.mu_r(r, V, lr);
+            r[i] = V[i] = S[i] = drt[i] = 0.0f;
+            load(i);
+        }
+        if (PIPE) __syncthreads();  // block 0's sums
+        // partial sums go to memory after each step t with
+        // t % flush_every == 0 (the grouping of one launch per segment):
+        // after `until` more steps
+        const int fe = s.flush_every > 0 ? s.flush_every : 0;
+        int until = fe ? static_cast<int>(top % fe) : -1;
+        bool pending = false;
+        const auto block = [&](auto unit, auto whole, long long tb, int cnt, const float* csb) {
+#pragma unroll
+            for (int i = 0; i < K; ++i) {
+                if (!whole.value && i >= cnt) break;
+                const float mr = m.mu_r(r[i], V[i], lr);
                 const float mv = lv;
                 if (valid) {
                     const uint32_t pos = static_cast<uint32_t>(tb - i + 1) & mask;
                     ring_n[pos * kLanes] = mv;
                     if (pos < static_cast<uint32_t>(K)) ring_n[(pos + nh) * kLanes] = mv;
                 }
-                m.update(r, V, S, mr, mv, csb[(K - 1 - i) * H + l], cG, drt, lr, lv, deta, dG);
+                m.update<decltype(unit)::value>(r[i], V[i], mr, mv, csb[(K - 1 - i) * H + l], cG, drt[i], lr, lv);
+                sums.step(mv, S[i]);
+                load(i);
                 pending = true;
-                if (tb - i == next_flush) {
-                    if (live) {
-                        s.deta[static_cast<long long>(N) * l + n] += deta;
-                        s.dG[static_cast<long long>(N) * l + n] += dG;
-                    }
-                    deta = dG = 0.0;
+                if (until-- == 0) {
+                    if (live) sums.add(m.c, deta_n, dG_n);
+                    sums = AdjSums();
                     pending = false;
-                    next_flush -= fe;
+                    until = fe - 1;
                 }
             }
+        };
+        const auto run = [&](auto unit) {
+            uint32_t ph = 0;
+            for (long long tb = top; tb >= t0; tb -= K) {
+                const int cnt = (tb - t0 + 1) < K ? static_cast<int>(tb - t0 + 1) : K;
+                if (!PIPE) {
+                    gather(tb, cs);
+                    __syncwarp();
+                }
+                const float* csb = PIPE ? cs + (ph & 1u) * bufsz : cs;
+                if (cnt == K)
+                    block(unit, Flag<true>{}, tb, K, csb);
+                else
+                    block(unit, Flag<false>{}, tb, cnt, csb);
+                if (PIPE) {
+                    __syncthreads();
+                    if (cluster && !lag) __syncthreads();
+                    if (cluster && phases.failed(ph)) break;
+                } else {
+                    group_barrier(cluster);
+                }
+                ++ph;
+            }
+        };
+        if (m.tau == 1.0f)
+            run(Flag<true>{});
+        else
+            run(Flag<false>{});
+        if (live) {
+            s.lam[2LL * N * l + 2 * n] = lr;
+            s.lam[2LL * N * l + 2 * n + 1] = lv;
+            if (pending) sums.add(m.c, deta_n, dG_n);
         }
-        if (PIPE) buf ^= 1;
-        group_barrier(cluster);
     }
-    if (live) {
-        s.lam[2LL * N * l + 2 * n] = lr;
-        s.lam[2LL * N * l + 2 * n + 1] = lv;
-        if (pending) {
-            s.deta[static_cast<long long>(N) * l + n] += deta;
-            s.dG[static_cast<long long>(N) * l + n] += dG;
-        }
+    if (PIPE && cluster) {
+        if (threadIdx.x == 0 && phases.fail) report(status, TVBG_ETIMEOUT);
+        group_barrier(true);  // no CTA leaves while another may still arrive on its phases
     }
 }
 
@@ -373,7 +415,8 @@ extern "C" int tvbg_adjoint_mpr_groups(const tvbg_adjoint_group* d_adj, int32_t 
     using Fn = void (*)(const tvbg_adjoint_group*, int32_t, int32_t*);
     const Fn kfn = pipelined ? (block_k == 8 ? adjoint_group_kernel<8, true> : adjoint_group_kernel<4, true>)
                              : (block_k == 8 ? adjoint_group_kernel<8, false> : adjoint_group_kernel<4, false>);
-    const size_t smem = 4u * static_cast<size_t>(block_k) * static_cast<size_t>(threads);
+    const size_t smem = 4u * static_cast<size_t>(block_k) * static_cast<size_t>(threads) +
+                        static_cast<size_t>(stage_bytes(pipelined ? threads / 2 : threads));
     cudaError_t e = cudaSuccess;
     if (cluster > 8) {
         e = cudaFuncSetAttribute(reinterpret_cast<const void*>(kfn),

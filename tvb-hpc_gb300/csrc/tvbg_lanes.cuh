@@ -170,13 +170,14 @@ __device__ __forceinline__ void ldcg_run(const float* p, float v[W]) {
 // VEC: run_vec holds (every ring of the Python layer); otherwise W scalar
 // loads and 64-bit indices.
 template <int CF, int K, int NC, bool VEC, int FLOATS>
-__device__ __forceinline__ void gather_run(const tvbg_group& g, const uint2* edges, int deg, uint32_t tm,
-                                           uint32_t mask, uint32_t R, int l, float* cs_slot, int stride) {
+__device__ __forceinline__ void gather_run(const float* __restrict__ ring_g, const float* cf_p, const uint2* edges,
+                                           int deg, uint32_t tm, uint32_t mask, uint32_t R, int l, float* cs_slot,
+                                           int stride) {
     constexpr int F = K * NC;               // floats of a run per lane
     constexpr int W = F < 8 ? F : 8;        // floats per load
     constexpr int NJ = F / W;               // loads per edge and lane
     constexpr int U = !VEC ? 1 : (FLOATS / F < 8 ? FLOATS / F : 8);  // edges in flight
-    const float* __restrict__ ring = g.ring + l * W;
+    const float* __restrict__ ring = ring_g + l * W;
     float2 acc[NJ][(W + 1) / 2];
 #pragma unroll
     for (int j = 0; j < NJ; ++j)
@@ -213,13 +214,13 @@ __device__ __forceinline__ void gather_run(const tvbg_group& g, const uint2* edg
 #pragma unroll
                 for (int j = 0; j < NJ; ++j) {
                     if constexpr (W == 1) {
-                        acc[j][0].x = fmaf(w[u], lane_pre<CF>(v[u][j][0], g.cf_p), acc[j][0].x);
+                        acc[j][0].x = fmaf(w[u], lane_pre<CF>(v[u][j][0], cf_p), acc[j][0].x);
                     } else {
 #pragma unroll
                         for (int i = 0; i < W / 2; ++i)
                             acc[j][i] = __ffma2_rn(ww,
-                                                   make_float2(lane_pre<CF>(v[u][j][2 * i], g.cf_p),
-                                                               lane_pre<CF>(v[u][j][2 * i + 1], g.cf_p)),
+                                                   make_float2(lane_pre<CF>(v[u][j][2 * i], cf_p),
+                                                               lane_pre<CF>(v[u][j][2 * i + 1], cf_p)),
                                                    acc[j][i]);
                     }
                 }
@@ -246,9 +247,10 @@ __device__ __forceinline__ void gather_run(const tvbg_group& g, const uint2* edg
 // gather_run for a ring of any alignment, out of line: its registers stay
 // out of the callers' loops.
 template <int CF, int K, int NC>
-__device__ __noinline__ void gather_run_any(const tvbg_group& g, const uint2* edges, int deg, uint32_t tm,
-                                            uint32_t mask, uint32_t R, int l, float* cs_slot, int stride) {
-    gather_run<CF, K, NC, false, 16>(g, edges, deg, tm, mask, R, l, cs_slot, stride);
+__device__ __noinline__ void gather_run_any(const float* ring, const float* cf_p, const uint2* edges, int deg,
+                                            uint32_t tm, uint32_t mask, uint32_t R, int l, float* cs_slot,
+                                            int stride) {
+    gather_run<CF, K, NC, false, 16>(ring, cf_p, edges, deg, tm, mask, R, l, cs_slot, stride);
 }
 
 // Whether a ring takes gather_run's vector loads and 32-bit row indices.
@@ -383,9 +385,10 @@ __device__ __forceinline__ void gather_node(const tvbg_group& g, const GroupLane
                                             uint32_t tm, float* cs_slot, int stride) {
     constexpr int NC = ring_channels<CF>();
     if (c.vec)
-        gather_run<CF, K, NC, true, gather_floats(BOUND)>(g, edges, deg, tm, c.mask, c.R, c.l, cs_slot, stride);
+        gather_run<CF, K, NC, true, gather_floats(BOUND)>(g.ring, g.cf_p, edges, deg, tm, c.mask, c.R, c.l, cs_slot,
+                                                          stride);
     else
-        gather_run_any<CF, K, NC>(g, edges, deg, tm, c.mask, c.R, c.l, cs_slot, stride);
+        gather_run_any<CF, K, NC>(g.ring, g.cf_p, edges, deg, tm, c.mask, c.R, c.l, cs_slot, stride);
 }
 
 // In-edge records of the CTA's node slots, staged in shared memory for the
@@ -402,8 +405,8 @@ struct EdgeStage {
 // All threads of the CTA; threads [0, 8 P) are the lanes of the P slots,
 // with the degree deg of their slot's node and its first edge lo.  Returns
 // the slot's records (valid for threads < 8 P).  Ends with a barrier.
-__device__ __forceinline__ const uint2* stage_edges(const tvbg_group& g, EdgeStage& st, uint2* records, int P,
-                                                    int tid, int lo, int deg) {
+__device__ __forceinline__ const uint2* stage_edges(const uint2* edges, EdgeStage& st, uint2* records,
+                                                    int P, int tid, int lo, int deg) {
     const int slot = tid / kLanes, l = tid % kLanes;
     if (slot < P && l == 0) st.off[slot + 1] = deg;
     __syncthreads();
@@ -423,7 +426,7 @@ __device__ __forceinline__ const uint2* stage_edges(const tvbg_group& g, EdgeSta
         if (tid == 0) st.off[0] = 0;
     }
     __syncthreads();
-    const uint2* src = reinterpret_cast<const uint2*>(g.edges) + lo;
+    const uint2* src = edges + lo;
     const uint2* out = src;
     if (st.off[P] <= P * kStageEdges) {
         if (slot < P) {
@@ -702,7 +705,7 @@ __device__ __forceinline__ void run_group(const tvbg_group& g, float* csum, Edge
     const int lo0 = q0 < N ? __ldg(g.row + n0) : 0;
     const int deg0 = q0 < N ? __ldg(g.row + n0 + 1) - lo0 : 0;
     const uint2* edges0 = reinterpret_cast<const uint2*>(g.edges) + lo0;
-    if (rounds == 1) edges0 = stage_edges(g, stage, records, P, threadIdx.x, lo0, deg0);
+    if (rounds == 1) edges0 = stage_edges(reinterpret_cast<const uint2*>(g.edges), stage, records, P, threadIdx.x, lo0, deg0);
     for (int q = q0; q < N; q += stride) seed_node<M, CF>(g, c, g.nodes ? __ldg(g.nodes + q) : q);
     group_barrier(cluster);
     MonitorClock mc;
@@ -834,7 +837,8 @@ __device__ __forceinline__ void run_group_pipelined(const tvbg_group& g, float* 
     if (threadIdx.x == 0) phases.init(C);
     // the gather team's threads carry the slots (their tid is the scan's)
     const int st_tid = gather_team ? tid : H + tid;
-    const uint2* edges = stage_edges(g, stage, reinterpret_cast<uint2*>(csum + 2 * bufsz), P, st_tid, lo, deg);
+    const uint2* edges = stage_edges(reinterpret_cast<const uint2*>(g.edges), stage,
+                                     reinterpret_cast<uint2*>(csum + 2 * bufsz), P, st_tid, lo, deg);
 
     if (!gather_team && valid) seed_node<M, CF>(g, c, n);
     group_barrier(cluster);

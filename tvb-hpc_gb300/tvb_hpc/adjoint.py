@@ -112,12 +112,10 @@ def plan_windows(S, per_segment, budget, window=None):
 
 def adjoint_group_shape(N, pipelined=False, slots=16, max_threads=512, max_cluster=16):
     """(threads, cluster, pipelined) of tvbg_adjoint_mpr_groups for N
-    nodes: about `slots` node slots per CTA (measured at N = 84, 256
-    instances: 16 slots x 6 CTAs 9.15 ms per backward, 44 x 2 9.5 ms), as
-    many CTAs as that takes up to max_cluster, node slots a multiple of 4
-    (each team's threads a multiple of 32); threads = 8 (16 with the two
-    pipelined teams) per slot, at most max_threads; None when N does not
-    fit."""
+    nodes: about `slots` node slots per CTA, as many CTAs as that takes up to
+    max_cluster, node slots a multiple of 4 (each team's threads a multiple
+    of 32); threads = 8 (16 with the two pipelined teams) per slot, at most
+    max_threads; None when N does not fit."""
     per = 16 if pipelined else 8
     c0 = min(max_cluster, max(-(-N // slots), -(-N // (max_threads // per)), 1))
     for c in range(c0, max_cluster + 1):
@@ -126,6 +124,23 @@ def adjoint_group_shape(N, pipelined=False, slots=16, max_threads=512, max_clust
         if per * p <= max_threads:
             return per * p, c, int(bool(pipelined))
     return None
+
+
+def adjoint_spread_shape(N, groups, sms):
+    """Shape of the two-team reverse kernel for `groups` groups.  Its time
+    grows with the node slots an SM holds (about 440 us + 18 us per slot for
+    2000 steps), so: the smallest CTAs of at least 16 slots that all find an
+    SM of their own (clusters leave about 0.15 of the SMs unused).  N = 84,
+    32 groups: 24 slots x 4 CTAs 881 us, 16 x 6 985 us, 28 x 3 965 us; N = 40,
+    63 groups: 20 x 2 799 us, 16 x 3 958 us; N = 130, 13 groups: 16 x 9 895
+    us, 24 x 6 981 us.  More groups than that take several waves, and two
+    CTAs of 16 slots per SM are the best: N = 84, 125 groups: 16 x 6 3438 us,
+    28 x 3 3646 us, 24 x 4 4132 us."""
+    for slots in range(16, 33, 4):
+        shape = adjoint_group_shape(N, pipelined=True, slots=slots)
+        if shape and groups * shape[1] <= 0.85 * sms:
+            return shape
+    return adjoint_group_shape(N, pipelined=True)
 
 
 class FCFit:
@@ -165,7 +180,7 @@ class FCFit:
         # forward and recomputation sweeps: the pipelined lane-interleaved
         # group kernel where it applies (delays >= 2 K - 1, N <= 1024), else
         # the per-instance step kernel
-        from .groups import plan_group, pipelined_threads
+        from .groups import plan_group, pipelined_threads, device_sms
         k, _ = plan_group(int(d.min()), int(d.max()))
         self.layout = ('groups' if int(d.min()) >= 2 * k - 1 and pipelined_threads(self.N, 16)
                        else 'instances')
@@ -177,7 +192,7 @@ class FCFit:
         # the two-team reverse kernel where every delay is >= 2 K
         self.adjoint_shape = None
         if self.adj_k:
-            self.adjoint_shape = (adjoint_group_shape(self.N, pipelined=True)
+            self.adjoint_shape = (adjoint_spread_shape(self.N, -(-self.I // 8), device_sms())
                                   if self.dmin >= 2 * self.adj_k else None) or \
                 adjoint_group_shape(self.N)
         self.adjoint_kernel = ('groups' if self.layout == 'groups' and self.adjoint_shape
