@@ -790,9 +790,10 @@ class LemsStep:
 
 
 class AdjointStep:
-    """One bench step of the adjoint fit: FCFit.forward (checkpointed forward
-    sweep, FP64 FC loss) and FCFit.backward (recomputation + reverse-time
-    kernel per segment, FP64 gradient accumulation)."""
+    """One bench step of the adjoint fit: FCFit.forward (forward sweep with the
+    whole trace, or checkpoints where it does not fit; FC loss to FP64 accuracy)
+    and FCFit.backward (reverse-time kernel, over checkpoints with the
+    recomputation; FP64 gradient accumulation)."""
 
     def __init__(self, wl, torch):
         from tvb_hpc import adjoint
@@ -804,11 +805,14 @@ class AdjointStep:
         self.tpn = 2
         self.status = None
         self.grads = None
-        self.path = ('%s forward with checkpoints every %d steps; FC-fit loss '
-                     'path on the device (tvbg_fcfit_loss: FP64 FC and loss, no library GEMM); '
-                     'per segment: recomputation + reverse-time kernel (%s); FP64 gradients'
+        traced = self.prob.layout == 'groups' and self.prob._traced()
+        self.path = ('%s forward %s; FC-fit loss '
+                     'path on the device (tvbg_fcfit_loss: FP64-accurate FC and loss, no library GEMM); '
+                     '%sreverse-time kernel (%s); FP64 gradients'
                      % ('pipelined group kernel' if self.prob.layout == 'groups'
-                        else 'per-step kernel', wl['ckpt'],
+                        else 'per-step kernel',
+                        'with the whole trace' if traced else 'with checkpoints every %d steps' % wl['ckpt'],
+                        '' if traced else 'recomputation and ',
                         'lane-interleaved groups, time-blocked%s, %d threads x %d CTAs'
                         % ((', two thread teams' if self.prob.adjoint_shape[2] else '',)
                            + tuple(self.prob.adjoint_shape[:2]))
@@ -830,8 +834,14 @@ class AdjointStep:
         return ([(e0, e1)] if time_kernels else []), None
 
     def launches_per_step(self):
+        # forward, Gram, loss, dL/dr, reverse-time kernel; over checkpoints, a
+        # forward per segment, and a recomputation and a reverse per window
+        if self.prob.layout == 'groups' and self.prob._traced():
+            return 5
         segs = -(-self.wl['nsteps'] // self.wl['ckpt'])
-        return 3 * segs        # forward segment, recomputation, reverse-time kernel
+        if self.prob.layout == 'groups' and self.prob.adjoint_kernel == 'groups':
+            return segs + 3 + 2 * len(self.prob._windows()[1])
+        return 3 * segs + 3
 
     def grad_error(self, n_check=4):
         "Max-norm relative error of dL/dG and dL/deta vs the FP64 oracle on a sample."

@@ -656,10 +656,9 @@ int tvbg_fcfit_zgrad(const float *d_z, const float *d_a, float *d_out, int32_t n
  * groups): row s < T - 1 at d_x + g * x_inst_stride + l + (s * N + i) *
  * lanes, row T - 1 at d_last + g * last_inst_stride + l + i *
  * last_node_stride (or from d_x too when d_last is NULL).  Computes the
- * Pearson FC to FP64 accuracy (two-pass: FP64 means, then the centred Gram,
- * upper triangle only, in FP32 error-free arithmetic for N <= 192 -- every
- * product exact, sums carried in two FP32 words, error below 4e-12 of
- * ||c_i|| ||c_j|| -- and in FP64 above; norms from its diagonal; into
+ * Pearson FC to FP64 accuracy (two-pass: means, then the centred Gram, upper
+ * triangle only, from exact products of 8-bit digits of the centred samples,
+ * about 2^-53 of each node's largest deviation; norms from its diagonal; into
  * d_fc [n_inst][N][N] when not NULL), d_loss[b] = mean_{i<j}
  * (FC_ij - target_ij)^2 (FP64) and, when d_dx is not NULL, dL/dX (FP32) at
  * d_dx + b * dx_inst_stride + s * N + i.  target [N][N] FP64; d_scratch of
@@ -673,6 +672,15 @@ int tvbg_fcfit_loss(const float *d_x, int64_t x_inst_stride, const float *d_last
                     int32_t n_inst, int32_t T, int32_t N, const double *d_target,
                     double *d_loss, float *d_dx, int64_t dx_inst_stride, double *d_fc,
                     void *d_scratch, void *stream);
+/* The same for a trace with x_cols values per node and sample, the series
+ * being the first: row s < T - 1 at d_x + g * x_inst_stride + l +
+ * (s * N + i) * x_cols * lanes. */
+int tvbg_fcfit_loss_ex(const float *d_x, int64_t x_inst_stride, int32_t x_cols,
+                       const float *d_last, int64_t last_inst_stride,
+                       int64_t last_node_stride, int32_t lanes, int32_t n_inst,
+                       int32_t T, int32_t N, const double *d_target, double *d_loss,
+                       float *d_dx, int64_t dx_inst_stride, double *d_fc,
+                       void *d_scratch, void *stream);
 
 /*
  * Region mapping (tvb_hpc/network.py:179-202).  to_avg: d_roi[i][j] = sum

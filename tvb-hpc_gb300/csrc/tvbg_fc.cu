@@ -201,7 +201,7 @@ extern "C" int tvbg_fc_ex(const float* d_x, int32_t n_inst, int32_t T, int32_t N
     if ((d_target == nullptr) != (d_err == nullptr))
         return set_error(TVBG_EINVAL, "tvbg_fc: d_target and d_err go together");
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    const SeriesView v{d_x, inst_stride, nullptr, 0, 0, T, N, 1};
+    const SeriesView v{d_x, inst_stride, nullptr, 0, 0, T, N, 1, 1};
     if (fc_small_path(N)) {
         const bool half = N <= 96;
         const size_t smem = gram_plane_bytes(half ? 96 : 128) + sizeof(double) * (static_cast<size_t>(N) * (N + 1) / 2);
@@ -223,7 +223,7 @@ extern "C" int tvbg_fc_ex(const float* d_x, int32_t n_inst, int32_t T, int32_t N
         const int ncta = static_cast<int>(norms < N ? norms : N);   // one error part each
         for (int b0 = 0; b0 < n_inst; b0 += 65535) {   // gridDim.y
             const int nb = n_inst - b0 < 65535 ? n_inst - b0 : 65535;
-            const SeriesView vb{d_x + b0 * inst_stride, inst_stride, nullptr, 0, 0, T, N, 1};
+            const SeriesView vb{d_x + b0 * inst_stride, inst_stride, nullptr, 0, 0, T, N, 1, 1};
             double* gb = gram + static_cast<long long>(b0) * N * N;
             fc_gram_kernel<<<dim3(static_cast<unsigned>(tiles), nb), kGramThreads, smem, st>>>(vb, gb);
             double* parts = d_err ? d_scratch + static_cast<long long>(b0) * N : nullptr;

@@ -336,8 +336,17 @@ extern "C" int tvbg_fcfit_loss(const float* d_x, int64_t x_inst_stride, const fl
                                int32_t n_inst, int32_t T, int32_t N, const double* d_target,
                                double* d_loss, float* d_dx, int64_t dx_inst_stride, double* d_fc,
                                void* d_scratch, void* stream) {
+    return tvbg_fcfit_loss_ex(d_x, x_inst_stride, 1, d_last, last_inst_stride, last_node_stride, lanes, n_inst, T,
+                              N, d_target, d_loss, d_dx, dx_inst_stride, d_fc, d_scratch, stream);
+}
+
+extern "C" int tvbg_fcfit_loss_ex(const float* d_x, int64_t x_inst_stride, int32_t x_cols, const float* d_last,
+                                  int64_t last_inst_stride, int64_t last_node_stride, int32_t lanes,
+                                  int32_t n_inst, int32_t T, int32_t N, const double* d_target,
+                                  double* d_loss, float* d_dx, int64_t dx_inst_stride, double* d_fc,
+                                  void* d_scratch, void* stream) {
     if (!d_x || !d_target || !d_loss || !d_scratch || n_inst <= 0 || n_inst > 65535 || T < 2 ||
-        N < 2 || x_inst_stride < 0 || lanes < 1 || lanes > 8 ||
+        N < 2 || x_inst_stride < 0 || x_cols < 1 || x_cols > 1024 || lanes < 1 || lanes > 8 ||
         (d_dx && dx_inst_stride < static_cast<int64_t>(T) * N))
         return tvbg::set_error(TVBG_EINVAL, "tvbg_fcfit_loss: bad arguments (need T >= 2, N >= 2)");
     const int64_t nn = static_cast<int64_t>(N) * N, in = static_cast<int64_t>(n_inst);
@@ -349,7 +358,7 @@ extern "C" int tvbg_fcfit_loss(const float* d_x, int64_t x_inst_stride, const fl
     double* fc = d_fc ? d_fc : reinterpret_cast<double*>(s + 3 * al(in * N * 8));
     float* a32 = reinterpret_cast<float*>(s + 3 * al(in * N * 8) + al(in * nn * 8));
     float* fsc = reinterpret_cast<float*>(s + 3 * al(in * N * 8) + al(in * nn * 8) + al(in * nn * 4));
-    SeriesView v{d_x, x_inst_stride, d_last, last_inst_stride, last_node_stride, T, N, lanes};
+    SeriesView v{d_x, x_inst_stride, d_last, last_inst_stride, last_node_stride, T, N, lanes, x_cols};
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     if ((T + 63) / 64 > 65535) return tvbg::set_error(TVBG_EINVAL, "tvbg_fcfit_loss: T too large");
     const int64_t nt = (N + 63) / 64;

@@ -40,14 +40,15 @@ namespace tvbg {
 // lanes = 1 for per-instance arrays, 8 for lane-interleaved groups.
 struct SeriesView {
     const float* x;      // row s (s < T - 1, or every row without `last`):
-    int64_t xs;          //   x + (b / lanes) xs + b % lanes + (s N + i) lanes
+    int64_t xs;          //   x + (b / lanes) xs + b % lanes + (s N + i) cols lanes
     const float* last;   // row T - 1: last + (b / lanes) ls + b % lanes + i lns, or NULL
     int64_t ls, lns;
     int T, N, lanes;
+    int cols;            // values of a node and sample in x; the series is the first
     __device__ __forceinline__ float at(int b, int s, int i) const {
         const int g = b / lanes, l = b % lanes;
         if (last && s == T - 1) return __ldg(last + g * ls + l + static_cast<int64_t>(i) * lns);
-        return __ldg(x + g * xs + l + (static_cast<int64_t>(s) * N + i) * lanes);
+        return __ldg(x + g * xs + l + (static_cast<int64_t>(s) * N + i) * (lanes * cols));
     }
 };
 
@@ -59,8 +60,8 @@ struct SeriesRow {
     int end;
     __device__ __forceinline__ SeriesRow(const SeriesView& v, int b, int i) {
         const int g = b / v.lanes, l = b % v.lanes;
-        p = v.x + g * v.xs + l + static_cast<int64_t>(i) * v.lanes;
-        stride = static_cast<int64_t>(v.N) * v.lanes;
+        p = v.x + g * v.xs + l + static_cast<int64_t>(i) * (v.lanes * v.cols);
+        stride = static_cast<int64_t>(v.N) * (v.lanes * v.cols);
         last = v.last ? v.last + g * v.ls + l + static_cast<int64_t>(i) * v.lns : nullptr;
         end = v.last ? v.T - 1 : v.T;
     }

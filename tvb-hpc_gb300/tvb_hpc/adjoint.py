@@ -7,24 +7,26 @@ Problem (one connectome, I instances, T steps, deterministic):
   S_i(t) = sum_e w_e r_{j_e}(t - d_e)           (zero history)
   X_b[s] = r_b(s + 1),  FC_b = Pearson(X_b),  loss_b = mean_{i<j}(FC_b,ij - F*_ij)^2
 
-``FCFit.forward`` runs the sweep in chunks of `checkpoint_every` steps --
-on the pipelined lane-interleaved group kernel where the delays allow
-(every delay >= 2 K - 1), else on the per-instance step kernel -- keeping
-the state and the history ring at every chunk start (checkpoints) and the
-rate series for the FC; tvbg_fcfit_loss then takes the FC (FP64 means, a
-centred upper-triangle Gram in FP32 error-free arithmetic), the loss and
-dL/dr on the device in one call, no library GEMM.
+``FCFit.forward`` runs the sweep on the pipelined lane-interleaved group
+kernel where the delays allow (every delay >= 2 K - 1), else on the
+per-instance step kernel.  The backward needs the state and the coupling sum
+of every step.  Where `trace_budget` holds them for all T steps, the grouped
+forward traces them itself, in one launch (the group kernel's
+TVBG_F_TRACE_CSUM column), and nothing is computed twice.  Else it runs in
+chunks of `checkpoint_every` steps, keeping the state and the history ring
+at every chunk start (checkpoints) and the rate series.  tvbg_fcfit_loss_ex
+then takes the FC (tvbg_gram.cuh), the loss and dL/dr on the device in one
+call, no library GEMM.
 
-``FCFit.backward`` walks the chunks backwards.  On the grouped layout the
-chunks are recomputed in windows (as many as `trace_budget` holds, one
-launch per window: every chunk from a working copy of its checkpoint, on
-the forward's kernel, so bit-identical), the last window already at the end
-of forward on a side stream; the recomputation traces the state and the
-coupling sums (the group kernel's TVBG_F_TRACE_CSUM column).  The
-reverse-time recursion then runs over each window in one launch, on
-lane-interleaved groups of 8 instances, time-blocked, with two thread teams
-where every delay is >= 2 K (tvbg_adjoint_mpr_groups), carrying the adjoint
-state and an adjoint ring of mu_V between windows.  Elsewhere (delays under
+``FCFit.backward`` runs the reverse-time recursion over the whole trace in
+one launch, on lane-interleaved groups of 8 instances, time-blocked, with two
+thread teams where every delay is >= 2 K (tvbg_adjoint_mpr_groups).  Over
+checkpoints it goes by windows of chunks, last first (as many as
+`trace_budget` holds, one launch per window to recompute them, every chunk
+from a working copy of its checkpoint, on the forward's kernel, so
+bit-identical), the last window already at the end of forward on a side
+stream, carrying the adjoint state and an adjoint ring of mu_V between
+windows.  Elsewhere (delays under
 4 steps, N > 1024, the per-instance layout) chunk by chunk per instance
 (tvbg_adjoint_mpr; through tvbg_adjoint.seg_lanes on a group trace).
 dL/dG and dL/deta accumulate in FP64, their partial sums grouped per chunk
@@ -198,7 +200,8 @@ class FCFit:
         self.adjoint_kernel = ('groups' if self.layout == 'groups' and self.adjoint_shape
                                else 'instances')
         # device buffers and group sets reused across calls (built on first use)
-        self._fw_gs = self._rec_gs = None
+        self._fw_gs = self._rec_gs = self._tr_gs = None
+        self._side = None
         self._ck = None
         self._bufs = None
         self._adj_ring = None
@@ -206,13 +209,14 @@ class FCFit:
         self._eager = None
         self._tables = []
         self._deferred = []      # status words of earlier calls, copied to the host
-        # the recomputation on the grouped layout runs in windows of segments,
-        # one launch per window, their traces (r, V, S) and working copies of
-        # the checkpoints within trace_budget bytes; the last window is
+        # the grouped forward keeps the trace (r, V, S) of all steps where it
+        # fits trace_budget bytes (_traced).  Else the recomputation runs in
+        # windows of segments, one launch per window, their traces and working
+        # copies of the checkpoints within trace_budget; the last window is
         # recomputed at the end of forward() (side stream, overlapping the
         # loss path) when eager_recompute
         self.trace_budget = 2 << 30
-        self.recompute_window = None   # segments per window (None: from trace_budget)
+        self.recompute_window = None   # segments per window (None: by trace_budget, or none at all)
         self.eager_recompute = True
         if self.adjoint_kernel == 'groups':
             self.lognh_g = max(1, int(np.ceil(np.log2(self.dmax + self.adj_k))))
@@ -297,66 +301,94 @@ class FCFit:
             return self._forward_groups(G, eta)
         return self._forward_instances(G, eta)
 
-    def _group_sets(self, G, eta):
-        """The forward's and the recomputation's GroupSets (one-column r
-        trace of T rows; r, V and the coupling sum over one segment), built
-        on the first call and given this call's couplings, eta and initial
-        state after that."""
+    def _traced(self):
+        """Whether the forward keeps the whole trace in place of checkpoints:
+        it fits trace_budget, and no smaller windows were asked for.  (84
+        nodes, 256 instances, 2000 steps: 516 MB; recomputing it took 0.87 ms
+        of a 6.0 ms pass, the checkpoints' copies 0.51 ms.)"""
+        S = -(-self.T // self.C)
+        if self.recompute_window is not None and self.recompute_window < S:
+            return False
+        return 4 * (-(-self.I // 8)) * 8 * self.T * self.N * 3 <= self.trace_budget
+
+    def _group_sets(self, G, eta, traced):
+        """The forward's and the recomputation's GroupSets, built on first use
+        and given this call's couplings, eta and initial state after that:
+        traced, one set with r, V and the coupling sum of T rows; else the
+        forward's (one-column r trace of T rows) and the recomputation's (r, V
+        and the coupling sum over one segment)."""
         from .groups import pipelined_shape
         torch = self.torch
-        if self._fw_gs is None:
-            self._fw_gs = self._groups(G, eta, self.T, 1, False)
-            # the recomputation set: its tables, flags and parameters serve the
-            # windows (many groups per launch: the smallest pipelined cluster)
-            self._rec_gs = self._groups(G, eta, self.C, 2, True)
-            self._rec_gs.set_shape(*pipelined_shape(self._rec_gs))
+        if self._side is None:
             self._x0_dev = torch.from_numpy(self.x0).cuda()
             self._side = torch.cuda.Stream()
+        # an earlier call's recomputation (side stream) may still read the
+        # checkpoints and buffers that this forward overwrites or gives back
+        torch.cuda.current_stream().wait_stream(self._side)
+        self._tables, self._eager = [], None
+        if traced:
+            self._fw_gs = self._rec_gs = self._ck = self._win = None
+            old = (self._tr_gs, )
+            if self._tr_gs is None:
+                self._tr_gs = self._groups(G, eta, self.T, 2, True)
+            fw = self._tr_gs
         else:
-            for gs in (self._fw_gs, self._rec_gs):
+            self._tr_gs = None
+            old = (self._fw_gs, self._rec_gs)
+            if self._fw_gs is None:
+                self._fw_gs = self._groups(G, eta, self.T, 1, False)
+                # the recomputation set: its tables, flags and parameters serve
+                # the windows (many groups per launch: the smallest pipelined
+                # cluster)
+                self._rec_gs = self._groups(G, eta, self.C, 2, True)
+                self._rec_gs.set_shape(*pipelined_shape(self._rec_gs))
+            fw = self._fw_gs
+        if old[0] is not None:
+            for gs in old:
                 gs.set_couplings(G)
                 gs.set_nparam(eta)
-            fw = self._fw_gs
             fw.set_state(self._x0_dev)
             fw.clear_history()
             fw.t[:] = 0
-        return self._fw_gs, self._rec_gs
+        return fw
 
     def _forward_groups(self, G, eta):
-        """Forward on the pipelined group kernel: segments of C steps, the
-        group state and ring copied at each segment start, the r trace
-        lane-interleaved ([G][T][N][1][8]); the loss path reads it in place."""
+        """Forward on the pipelined group kernel: traced, one launch with r, V
+        and S lane-interleaved ([G][T][N][3][8]); else segments of C steps,
+        the group state and ring copied at each segment start, and the r trace
+        ([G][T][N][1][8]).  The loss path reads the trace in place."""
         torch = self.torch
-        fw, _ = self._group_sets(G, eta)
-        # an earlier call's recomputation (side stream) may still read the
-        # checkpoints this forward overwrites
-        torch.cuda.current_stream().wait_stream(self._side)
-        self._tables = []
+        traced = self._traced()
+        fw = self._group_sets(G, eta, traced)
         segs = [(t, min(self.C, self.T - t)) for t in range(0, self.T, self.C)]
-        plans = fw.prepare_segments(segs)
-        if self._ck is None:
-            self._ck = (torch.empty((len(segs), ) + tuple(fw.gstate.shape), dtype=torch.float32,
-                                    device='cuda'),
-                        torch.empty((len(segs), fw.ring.numel()), dtype=torch.float32, device='cuda'))
-        self.ckpt = []
-        for s, ((t0, n), launches) in enumerate(zip(segs, plans)):
-            self._ck[0][s].copy_(fw.gstate)
-            self._ck[1][s].copy_(fw.ring)
-            self.ckpt.append((t0, n, self._ck[0][s], self._ck[1][s]))
-            fw.launch(launches)
-        fw.t[:] = self.T
-        self.fw = fw
         I, N, T = self.I, self.N, self.T
         L = 8
-        self._eager = None
-        if self.adjoint_kernel == 'groups' and self.eager_recompute:
+        if traced:
+            self.ckpt = [(t0, n, None, None) for t0, n in segs]
+            fw.launch(fw.prepare_segments([(0, T)])[0])
+        else:
+            plans = fw.prepare_segments(segs)
+            if self._ck is None:
+                self._ck = (torch.empty((len(segs), ) + tuple(fw.gstate.shape), dtype=torch.float32,
+                                        device='cuda'),
+                            torch.empty((len(segs), fw.ring.numel()), dtype=torch.float32, device='cuda'))
+            self.ckpt = []
+            for s, ((t0, n), launches) in enumerate(zip(segs, plans)):
+                self._ck[0][s].copy_(fw.gstate)
+                self._ck[1][s].copy_(fw.ring)
+                self.ckpt.append((t0, n, self._ck[0][s], self._ck[1][s]))
+                fw.launch(launches)
+        fw.t[:] = T
+        self.fw = fw
+        if not traced and self.adjoint_kernel == 'groups' and self.eager_recompute:
             # the last window's recomputation overlaps the loss path
             self._windows()
             side = self._side
             side.wait_stream(torch.cuda.current_stream())
             self._eager = self._recompute_window(0, side)
-        loss = self._loss(fw.gtrace.data_ptr() + 4 * N * L, T * N * L, fw.gstate.data_ptr(),
-                          N * 2 * L, 2 * L, L)
+        cols = fw.gtrace.shape[3]
+        loss = self._loss(fw.gtrace.data_ptr() + 4 * N * cols * L, T * N * cols * L, fw.gstate.data_ptr(),
+                          N * 2 * L, 2 * L, L, cols)
         # this call's status copied without waiting; the earlier calls' checked
         # now that this call's work is queued behind theirs
         n_prev = len(self._deferred)
@@ -364,8 +396,8 @@ class FCFit:
         self.check(n_prev)
         return loss
 
-    def _loss(self, x, xs, last, ls, lns, lanes):
-        """tvbg_fcfit_loss on the series at x (rows 1..T-1) and last (row T):
+    def _loss(self, x, xs, last, ls, lns, lanes, cols=1):
+        """tvbg_fcfit_loss_ex on the series at x (rows 1..T-1) and last (row T):
         FP64 FC and loss; dL/dr(t) = dL/dX[t-1] into self.dr[:, 1:]."""
         torch = self.torch
         I, N, T = self.I, self.N, self.T
@@ -379,9 +411,10 @@ class FCFit:
                           torch.empty(int(nb.value), dtype=torch.uint8, device='cuda'))
         self.dr, self.fc, scratch = self._bufs
         loss = torch.empty(I, dtype=torch.float64, device='cuda')
-        nat.check(lib.tvbg_fcfit_loss(x, xs, last, ls, lns, lanes, I, T, N, self.target.data_ptr(),
-                                      loss.data_ptr(), self.dr.data_ptr() + 4 * N, (T + 1) * N,
-                                      self.fc.data_ptr(), scratch.data_ptr(), nat.stream_handle()))
+        nat.check(lib.tvbg_fcfit_loss_ex(x, xs, cols, last, ls, lns, lanes, I, T, N,
+                                         self.target.data_ptr(), loss.data_ptr(),
+                                         self.dr.data_ptr() + 4 * N, (T + 1) * N, self.fc.data_ptr(),
+                                         scratch.data_ptr(), nat.stream_handle()))
         return loss
 
     def _forward_instances(self, G, eta):
@@ -425,7 +458,13 @@ class FCFit:
         b = np.arange(I, dtype=np.int64)
         if grouped and self.adjoint_kernel == 'groups':
             return self._reverse_windows(lam, deta, dGn)
-        if grouped:
+        traced = grouped and rev[0][2] is None
+        if traced:
+            # the forward's trace, read in place
+            seg_ptr = self.fw.gtrace.data_ptr() + 4 * ((b // 8) * T * N * 3 * 8 + b % 8)
+            seg_lanes = 8
+            plans = [None] * len(rev)
+        elif grouped:
             # recomputation on the same pipelined group kernel (bit-identical
             # to the forward) with r, V and the coupling sum S traced,
             # lane-interleaved [G][C][N][3][8]; the adjoint reads it in place
@@ -447,7 +486,7 @@ class FCFit:
             tk = tab[k]
             tk['edges_t'] = self.edges_t.data_ptr()
             tk['row_t'] = self.row_t.data_ptr()
-            tk['seg'] = seg_ptr
+            tk['seg'] = seg_ptr + (4 * t0 * N * 3 * 8 if traced else 0)
             tk['seg_lanes'] = seg_lanes
             tk['dr'] = dr.data_ptr() + 4 * (b * (T + 1) * N + t0 * N)
             tk['lam'] = lam.data_ptr() + 4 * b * N * 2
@@ -473,7 +512,9 @@ class FCFit:
         smem = ring_b if (self.adjoint_smem == 'auto' and ring_b + 4096 <= max_smem()
                           and I <= sms) else 0
         for k, ((t0, n, st, rg), pl) in enumerate(zip(rev, plans)):
-            if grouped:
+            if traced:
+                pass
+            elif grouped:
                 rec.gstate.copy_(st)
                 rec.ring.copy_(rg)
                 rec.launch(pl)
@@ -484,7 +525,7 @@ class FCFit:
             nat.check(lib.tvbg_adjoint_mpr_ex(dev.data_ptr() + k * row_bytes, I, threads, smem,
                                               nat.stream_handle()))
         torch.cuda.synchronize()
-        (rec if grouped else sw).status.check()
+        (self.fw if traced else rec if grouped else sw).status.check()
         return dGn.sum(1), deta
 
 
@@ -551,8 +592,9 @@ class FCFit:
         return ev
 
     def _reverse_windows(self, lam, deta, dGn):
-        """Windows last first: each window recomputed in one launch (side
-        stream; the last window at the end of forward when eager_recompute),
+        """The forward's whole trace as one window, or windows last first: each
+        recomputed in one launch (side stream; the last window at the end of
+        forward when eager_recompute),
         then tvbg_adjoint_mpr_groups over the whole window in one launch,
         reading the window's traces in place.  The recomputation of window
         w + 1 overlaps the reverse kernel of window w; events order each
@@ -571,7 +613,12 @@ class FCFit:
         threads, cluster, pipe = self.adjoint_shape
         if pipe and self.dmin < 2 * K:
             raise ValueError('pipelined reverse kernel: every delay >= 2 K')
-        W, wins, bufs, _ = self._windows()
+        traced = self.ckpt[0][2] is None
+        if traced:
+            wins, bufs, rows = [(0, len(self.ckpt))], [(self.fw.gtrace, )], T
+        else:
+            W, wins, bufs, _ = self._windows()
+            rows = W * self.C
         nw = len(wins)
         g = np.arange(Gn, dtype=np.int64)[None, :]           # [1, Gn]
         t0s = np.array([wins[w][0] * self.C for w in range(nw)], np.int64)[:, None]
@@ -584,7 +631,7 @@ class FCFit:
         tab['edges_t'] = self.edges_tg.data_ptr()
         tab['row_t'] = self.row_t.data_ptr()
         tab['nodes'] = self.nodes_t.data_ptr()
-        tab['seg'] = tr0 + 4 * g * W * self.C * N * 3 * 8
+        tab['seg'] = tr0 + 4 * g * rows * N * 3 * 8
         tab['dr'] = self.dr.data_ptr() + 4 * (8 * g * (T + 1) * N + t0s * N)
         tab['lam'] = lam.data_ptr() + 4 * 8 * g * N * 2
         tab['ring'] = ring.data_ptr() + 4 * g * N * R * 8
@@ -605,27 +652,34 @@ class FCFit:
         row_bytes = Gn * nat.ADJOINT_GROUP_DTYPE.itemsize
         status = DeviceStatus()
         main, side = torch.cuda.current_stream(), self._side
-        side.wait_stream(main)
-        ready = [None] * nw
-        done = [None] * nw
-        ready[0], self._eager = self._eager, None
-        if ready[0] is None:
-            ready[0] = self._recompute_window(0, side)
-        for w in range(nw):
-            if w + 1 < nw:
-                if w >= 1:
-                    side.wait_event(done[w - 1])       # buffer (w + 1) % 2 last read by window w - 1
-                ready[w + 1] = self._recompute_window(w + 1, side)
-            main.wait_event(ready[w])
+
+        def reverse(w):
             nat.check(lib.tvbg_adjoint_mpr_groups(dev.data_ptr() + w * row_bytes, Gn, threads,
                                                   cluster, K, pipe, status.t.data_ptr(),
                                                   main.cuda_stream))
-            done[w] = torch.cuda.Event()
-            done[w].record(main)
-        main.wait_stream(side)
+
+        if traced:
+            reverse(0)
+        else:
+            side.wait_stream(main)
+            ready = [None] * nw
+            done = [None] * nw
+            ready[0], self._eager = self._eager, None
+            if ready[0] is None:
+                ready[0] = self._recompute_window(0, side)
+            for w in range(nw):
+                if w + 1 < nw:
+                    if w >= 1:
+                        side.wait_event(done[w - 1])       # buffer (w + 1) % 2 last read by window w - 1
+                    ready[w + 1] = self._recompute_window(w + 1, side)
+                main.wait_event(ready[w])
+                reverse(w)
+                done[w] = torch.cuda.Event()
+                done[w].record(main)
+            main.wait_stream(side)
         dG = dGn.sum(1)
         n_prev = len(self._deferred)
-        self._defer(self._rec_gs.status, status)
+        self._defer(*((status, ) if traced else (self._rec_gs.status, status)))
         self.check(n_prev)
         return dG, deta
 
