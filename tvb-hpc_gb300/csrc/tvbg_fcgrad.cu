@@ -86,8 +86,9 @@ extern "C" int tvbg_fcfit_zgrad(const float* d_z, const float* d_a, float* d_out
 // X_b [T][N] (rows 0..T-2 from x, row T-1 from `last` when given), its
 // Pearson FC in FP64, the loss mean_{i<j} (FC_ij - F*_ij)^2 and
 // dL/dX = (Z A - Z diag(FC A)) / nrm, Z = (X - mean) / nrm, A = 2 (FC - F*) / P
-// with a zero diagonal (P = N (N - 1) / 2).  Kernels: means and the centred
-// Gram to FP64 accuracy (tvbg_gram.cuh); per instance the norms from the Gram's
+// with a zero diagonal (P = N (N - 1) / 2).  Kernels: FP64 means and the
+// centred Gram (FP32 error-free transformations for N <= 192, digit products
+// above); per instance the norms from the Gram's
 // diagonal, FC, loss, A and diag(FC A) (the chain rule's time reduction
 // sum_t Z_ti (Z A)_ti, taken from FC in FP64); dL/dX in FP32 (Z A is a sum
 // over N nodes per sample, the precision of the backward).  The Pearson FC
@@ -99,9 +100,253 @@ namespace {
 
 using tvbg::SeriesView;
 
-// FP64 means and the centred Gram (tvbg_gram.cuh), both triangles written.
-// Pass per adjoint at N = 84, 256 instances, 2000 samples: 1.54 ms with FP32
-// error-free products on the FP32 pipe and 0.31 for the means before.
+// FP64 mean of every (instance, node): the samples split into kMS slices
+// of consecutive samples, one thread each, the slices' sums added in slice
+// order.  CTA = 32 (node, lane) pairs x kMS slices of one block of instances
+// (blockIdx.y), lanes fastest: a warp reads whole sectors of a
+// lane-interleaved series (256 x 84 series of 2000 samples: 187 us; 223 with one
+// lane per CTA).
+constexpr int kMS = 8;
+__global__ void __launch_bounds__(256) fcfit_mean_kernel(SeriesView v, int n_inst, double* mean) {
+    __shared__ double part[kMS][32];
+    const int q = blockIdx.x * 32 + static_cast<int>(threadIdx.x);
+    const int i = q / v.lanes;
+    const int b = static_cast<int>(blockIdx.y) * v.lanes + q % v.lanes;
+    const bool own = i < v.N && b < n_inst;
+    const int per = (v.T + kMS - 1) / kMS;
+    const int t0 = static_cast<int>(threadIdx.y) * per;
+    const int t1 = t0 + per < v.T ? t0 + per : v.T;
+    double s = 0.0;
+    if (own) {
+        const tvbg::SeriesRow row(v, b, i);
+#pragma unroll 8
+        for (int t = t0; t < t1; ++t) s += static_cast<double>(row.at(t));
+    }
+    part[threadIdx.y][threadIdx.x] = s;
+    __syncthreads();
+    if (threadIdx.y == 0 && own) {
+        double m = 0.0;
+#pragma unroll
+        for (int k = 0; k < kMS; ++k) m += part[k][threadIdx.x];
+        mean[static_cast<int64_t>(b) * v.N + i] = m / static_cast<double>(v.T);
+    }
+}
+
+// Centred Gram G_ij = sum_t c_ti c_tj, c = x - mean, for N <= kSplitMaxN,
+// all in FP32 arithmetic with error-free transformations: Knuth's TwoSum and
+// TwoProduct by FMA, as in Ogita, Rump and Oishi, "Accurate sum and dot
+// product", SIAM J. Sci. Comput. 26(6), 2005.  Every operation is an
+// explicitly rounded intrinsic: nothing is contracted or reordered.
+//
+// A, 1 / nrm and zg / nrm are rounded to FP32 from this Gram, and the backward
+// carries those roundings into dL/deta: two Grams that differ by 1e-14 give
+// gradients that differ by up to 5e-8.  So these sums keep one arithmetic
+// (the digit products of tvbg_gram.cuh are as accurate, but not the same bits).
+//
+// Work split: tiles of RB x 4 pairs of the upper triangle, one per thread,
+// CTA = (instance blockIdx.x, part blockIdx.y of the tiles), instances
+// fastest so that the lanes of a lane-interleaved group read the same
+// sectors together.
+//
+// Centring: each mean (FP64) is split once into mh + ml (FP32 words); a
+// sample x becomes c = (x - mh) - ml as (hi, lo) with hi + lo = c up to
+// about 2^-48 (|c| + 2 |mean|): TwoSum(x, -mh) = (d, de), then
+// TwoSum(d, de - ml).  kSplitL samples of every node staged per pass.
+//
+// Products: per pair and sample hi_i hi_j = p + e exactly (TwoProduct);
+// p is summed by TwoSum (rounding errors collected in a second word),
+// e + hi_i lo_j + lo_i hi_j (2^-24 of the product) in a third word; lo_i lo_j
+// (2^-48) is dropped.  Every kSplitL samples the three words are added into
+// the pair's double-FP32 sum (TwoSum, then the small words, then TwoSum
+// again), converted to FP64 at the end.  The error is bounded by about
+// kSplitL^2 2^-48 sum_t |c_ti c_tj| (the collected rounding errors of a pass
+// summed in FP32), below 4e-12 of ||c_i|| ||c_j||; typical errors are near
+// 1e-14.  Both triangles of G written.
+//
+// What bounds it: 12 FP32 operations per pair and sample, 256 x 84 nodes x 2000
+// samples 1.28 ms (1.52 with 2 x 2 blocks of pairs and a division per staged
+// sample; scalar operations 1.34).  They run two pairs at a time on the packed instructions; a subtraction is an FMA by -1 (the
+// same rounding), and the third word is kept negated, which lets
+// e = hi_i hi_j - p come from -hi_i.
+constexpr int kSplitL = 32;
+constexpr int kSplitMaxN = 192;   // staging (kSplitL + 1) x N pairs of words <= 50.7 KB
+constexpr int kSplitThreads = 128;
+constexpr int kSplitWarps = kSplitThreads / 32;
+
+__device__ __forceinline__ float2 sub2(float2 a, float2 b) { return __ffma2_rn(b, make_float2(-1.0f, -1.0f), a); }
+__device__ __forceinline__ void two_sum2(float2 a, float2 b, float2& s, float2& e) {
+    s = __fadd2_rn(a, b);
+    const float2 bb = sub2(s, a);
+    e = __fadd2_rn(sub2(a, sub2(s, bb)), sub2(b, bb));
+}
+
+// Tiles of row block bi: column blocks from its first pair on or above the
+// diagonal.
+template <int RB>
+__host__ __device__ __forceinline__ int split_tiles(int N) {
+    int n = 0;
+    for (int i = 0; i < N; i += RB) n += (N + 3) / 4 - i / 4;
+    return n;
+}
+
+template <int RB>
+__global__ void __launch_bounds__(kSplitThreads, 4) fcfit_gram_split_kernel(SeriesView v, const double* __restrict__ mean,
+                                                                         int per_part, double* G) {
+    extern __shared__ __align__(16) float sh[];  // [kSplitL][Np] hi, [kSplitL][Np] lo, [Np] mh, [Np] ml
+    const int b = blockIdx.x;
+    const int N = v.N;
+    const int nc = (N + 3) / 4;
+    const int Np = 4 * nc;
+    const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
+    float* const shi = sh;
+    float* const slo = sh + kSplitL * Np;
+    float* const smh = sh + 2 * kSplitL * Np;
+    float* const sml = smh + Np;
+    const int first = static_cast<int>(blockIdx.y) * per_part;
+    int i0 = 0, j0 = 0;
+    bool act = false;
+    if (static_cast<int>(threadIdx.x) < per_part) {
+        int rem = first + static_cast<int>(threadIdx.x);
+        while (i0 < N && rem >= nc - i0 / 4) {
+            rem -= nc - i0 / 4;
+            i0 += RB;
+        }
+        act = i0 < N;
+        j0 = act ? 4 * (i0 / 4 + rem) : 0;
+        if (!act) i0 = 0;
+    }
+    const double* mb = mean + static_cast<int64_t>(b) * N;
+    for (int c = threadIdx.x; c < Np; c += kSplitThreads) {
+        const double m = c < N ? mb[c] : 0.0;
+        const float mh = __double2float_rn(m);
+        smh[c] = mh;
+        sml[c] = __double2float_rn(m - static_cast<double>(mh));
+    }
+    float2 ah[RB][2], al[RB][2];  // double-FP32 sums
+#pragma unroll
+    for (int u = 0; u < RB; ++u)
+#pragma unroll
+        for (int w = 0; w < 2; ++w) ah[u][w] = al[u][w] = make_float2(0.0f, 0.0f);
+    __syncthreads();
+    for (int t0 = 0; t0 < v.T; t0 += kSplitL) {
+        // a warp takes whole rows of samples, its lanes the nodes
+        for (int c = lane; c < Np; c += 32) {
+            const tvbg::SeriesRow row(v, b, c < N ? c : 0);
+            const float mh = smh[c], ml = sml[c];
+            float x[kSplitL / kSplitWarps];
+#pragma unroll
+            for (int k = 0; k < kSplitL / kSplitWarps; ++k) {
+                const int t = t0 + warp + k * kSplitWarps;
+                x[k] = c < N && t < v.T ? row.at(t) : 0.0f;
+            }
+#pragma unroll
+            for (int k = 0; k < kSplitL / kSplitWarps; ++k) {
+                const int r = warp + k * kSplitWarps;
+                float hi = 0.0f, lo = 0.0f;
+                if (c < N && t0 + r < v.T) {
+                    float d, de;
+                    tvbg::gram_two_sum(x[k], -mh, d, de);
+                    tvbg::gram_two_sum(d, __fsub_rn(de, ml), hi, lo);
+                }
+                shi[r * Np + c] = hi;
+                slo[r * Np + c] = lo;
+            }
+        }
+        __syncthreads();
+        if (act) {
+            float2 s[RB][2], cp[RB][2], nm[RB][2];  // nm: the small words, negated
+#pragma unroll
+            for (int u = 0; u < RB; ++u)
+#pragma unroll
+                for (int w = 0; w < 2; ++w) s[u][w] = cp[u][w] = nm[u][w] = make_float2(0.0f, 0.0f);
+#pragma unroll 1
+            for (int r = 0; r < kSplitL; ++r) {
+                const float* const xh = shi + r * Np + i0;
+                const float* const xl = slo + r * Np + i0;
+                const float4 yh4 = *reinterpret_cast<const float4*>(shi + r * Np + j0);
+                const float4 yl4 = *reinterpret_cast<const float4*>(slo + r * Np + j0);
+                const float2 yh[2] = {make_float2(yh4.x, yh4.y), make_float2(yh4.z, yh4.w)};
+                const float2 yl[2] = {make_float2(yl4.x, yl4.y), make_float2(yl4.z, yl4.w)};
+                float h[RB], q[RB];
+                if constexpr (RB == 4) {
+                    *reinterpret_cast<float4*>(h) = *reinterpret_cast<const float4*>(xh);
+                    *reinterpret_cast<float4*>(q) = *reinterpret_cast<const float4*>(xl);
+                } else if constexpr (RB == 2) {
+                    *reinterpret_cast<float2*>(h) = *reinterpret_cast<const float2*>(xh);
+                    *reinterpret_cast<float2*>(q) = *reinterpret_cast<const float2*>(xl);
+                } else {
+                    h[0] = *xh;
+                    q[0] = *xl;
+                }
+#pragma unroll
+                for (int u = 0; u < RB; ++u) {
+                    const float2 hh = make_float2(h[u], h[u]), nh = make_float2(-h[u], -h[u]);
+                    const float2 nq = make_float2(-q[u], -q[u]);
+#pragma unroll
+                    for (int w = 0; w < 2; ++w) {
+                        const float2 p = __fmul2_rn(hh, yh[w]);
+                        const float2 ne = __ffma2_rn(nh, yh[w], p);  // p - hi hi, exact
+                        nm[u][w] = __fadd2_rn(nm[u][w], __ffma2_rn(nh, yl[w], __ffma2_rn(nq, yh[w], ne)));
+                        float2 t, err;
+                        two_sum2(s[u][w], p, t, err);
+                        s[u][w] = t;
+                        cp[u][w] = __fadd2_rn(cp[u][w], err);
+                    }
+                }
+            }
+#pragma unroll
+            for (int u = 0; u < RB; ++u)
+#pragma unroll
+                for (int w = 0; w < 2; ++w) {  // (ah, al) += s + (cp + small words)
+                    float2 hi, lo;
+                    two_sum2(ah[u][w], s[u][w], hi, lo);
+                    lo = __fadd2_rn(lo, __fadd2_rn(al[u][w], sub2(cp[u][w], nm[u][w])));
+                    two_sum2(hi, lo, ah[u][w], al[u][w]);
+                }
+        }
+        __syncthreads();
+    }
+    if (!act) return;
+    double* gb = G + static_cast<int64_t>(b) * N * N;
+#pragma unroll
+    for (int u = 0; u < RB; ++u)
+#pragma unroll
+        for (int w = 0; w < 4; ++w) {
+            const int i = i0 + u, j = j0 + w;
+            if (i < N && j < N && j >= i) {
+                const double g = w % 2 ? static_cast<double>(ah[u][w / 2].y) + static_cast<double>(al[u][w / 2].y)
+                                       : static_cast<double>(ah[u][w / 2].x) + static_cast<double>(al[u][w / 2].x);
+                gb[static_cast<int64_t>(i) * N + j] = g;
+                gb[static_cast<int64_t>(j) * N + i] = g;
+            }
+        }
+}
+
+template <int RB>
+int launch_gram_split(SeriesView v, const double* mean, double* G, int n_inst, cudaStream_t st) {
+    const int tiles = split_tiles<RB>(v.N);
+    const int parts = (tiles + kSplitThreads - 1) / kSplitThreads;
+    const size_t smem = 8u * (kSplitL + 1) * 4u * static_cast<size_t>((v.N + 3) / 4);
+    if (smem > 48u * 1024u) {
+        const cudaError_t e = cudaFuncSetAttribute(fcfit_gram_split_kernel<RB>,
+                                                   cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+        if (e != cudaSuccess) return tvbg::set_cuda_error(e, "tvbg_fcfit_loss: smem attribute");
+    }
+    fcfit_gram_split_kernel<RB><<<dim3(n_inst, parts), kSplitThreads, smem, st>>>(v, mean, (tiles + parts - 1) / parts, G);
+    return TVBG_OK;
+}
+
+// The tallest tiles that put a warp on every scheduler: 4 x 4 read the least
+// from shared memory, 1 x 4 are four times as many.  Whole loss path, us, with
+// 4 x 4 and 2 x 4 tiles: 256 x 84 nodes x 2000 samples 2070 and 2100, 64 x 84 x 1500
+// 668 and 632, 4 x 84 x 2000 756 and 629, 200 x 31 x 700 328 and 244.
+template <int RB>
+bool split_fills(int n_inst, int N) {
+    return static_cast<int64_t>(n_inst) * split_tiles<RB>(N) >= 152 * kSplitThreads;
+}
+
+// N > kSplitMaxN: FP64 means and Gram by digit products (tvbg_gram.cuh), both
+// triangles written.
 struct GramOut {
     double* g;       // the instance's [N][N]
     double* mean;    // the instance's [N]
@@ -114,21 +359,7 @@ struct GramOut {
     }
 };
 
-// N <= ROWS: one CTA per instance.
-template <int ROWS>
-__global__ void __launch_bounds__(tvbg::kGramThreads) fcfit_gram_kernel(SeriesView v, double* mean, double* G) {
-    extern __shared__ __align__(16) unsigned char gram_smem[];
-    __shared__ tvbg::GramNode nodes[ROWS];
-    __shared__ double scale[ROWS];
-    const int b = blockIdx.x;
-    const GramOut out{G + static_cast<int64_t>(b) * v.N * v.N, mean + static_cast<int64_t>(b) * v.N, v.N};
-    tvbg::gram_whole<ROWS>(
-        v, b, [=](int i, double m) { out.mean[i] = m; },
-        [=](int i, int j, double g, bool first) { out.put(i, j, g, first); },
-        reinterpret_cast<__nv_bfloat16*>(gram_smem), nodes, scale);
-}
-
-// Larger N: one CTA per 64 x 64 tile of the upper triangle (blockIdx.y).
+// N > kSplitMaxN: one CTA per 64 x 64 tile of the upper triangle (blockIdx.y).
 __global__ void __launch_bounds__(tvbg::kGramThreads) fcfit_gram_tiles_kernel(SeriesView v, double* mean, double* G) {
     extern __shared__ __align__(16) unsigned char gram_smem[];
     __shared__ tvbg::GramNode nodes[128];
@@ -362,17 +593,22 @@ extern "C" int tvbg_fcfit_loss_ex(const float* d_x, int64_t x_inst_stride, int32
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     if ((T + 63) / 64 > 65535) return tvbg::set_error(TVBG_EINVAL, "tvbg_fcfit_loss: T too large");
     const int64_t nt = (N + 63) / 64;
-    if (N > 128 && nt * (nt + 1) / 2 > 65535)
+    if (N > kSplitMaxN && nt * (nt + 1) / 2 > 65535)
         return tvbg::set_error(TVBG_EINVAL, "tvbg_fcfit_loss: N too large");
-    {
-        const bool whole = N <= 128, half = N <= 96;
-        auto kfn = half ? fcfit_gram_kernel<96> : whole ? fcfit_gram_kernel<128> : fcfit_gram_tiles_kernel;
-        const size_t smem = tvbg::gram_plane_bytes(half ? 96 : 128);
-        const cudaError_t e = cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    if (N <= kSplitMaxN) {
+        fcfit_mean_kernel<<<dim3((N * lanes + 31) / 32, (n_inst + lanes - 1) / lanes), dim3(32, kMS), 0, st>>>(
+            v, n_inst, mean);
+        const int rc = split_fills<4>(n_inst, N)   ? launch_gram_split<4>(v, mean, fc, n_inst, st)
+                       : split_fills<2>(n_inst, N) ? launch_gram_split<2>(v, mean, fc, n_inst, st)
+                                                   : launch_gram_split<1>(v, mean, fc, n_inst, st);
+        if (rc != TVBG_OK) return rc;
+    } else {
+        const size_t smem = tvbg::gram_plane_bytes(128);
+        const cudaError_t e = cudaFuncSetAttribute(fcfit_gram_tiles_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                                    static_cast<int>(smem));
         if (e != cudaSuccess) return tvbg::set_cuda_error(e, "tvbg_fcfit_loss: smem attribute");
-        kfn<<<dim3(n_inst, whole ? 1 : static_cast<unsigned>(nt * (nt + 1) / 2)), tvbg::kGramThreads, smem, st>>>(
-            v, mean, fc);
+        fcfit_gram_tiles_kernel<<<dim3(n_inst, static_cast<unsigned>(nt * (nt + 1) / 2)), tvbg::kGramThreads, smem,
+                                  st>>>(v, mean, fc);
     }
     fcfit_loss_kernel<<<n_inst, 256, 0, st>>>(fc, d_target, N, mean, nrm, d_loss, a32, zg, fsc);
     if (d_dx) {
