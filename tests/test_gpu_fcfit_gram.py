@@ -19,7 +19,8 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize('I,T,N', [(100, 70, 85), (45, 33, 83), (1, 31, 2), (3, 32, 3), (9, 65, 31),
-                                   (1300, 34, 18)])
+                                   (1300, 34, 18), (2, 127, 32), (1, 128, 33), (2, 129, 64), (1, 257, 65),
+                                   (2, 64, 96), (1, 65, 97), (2, 63, 128), (1, 64, 129)])
 def test_fcfit_loss_tiles(cuda, I, T, N):
     from tvb_hpc import _native as nat
     torch = cuda

@@ -479,74 +479,95 @@ __global__ void __launch_bounds__(256)
 }
 
 // The same product for N <= 16 WN, whole rows: CTA = (instance blockIdx.x,
-// 64 samples blockIdx.y), A_b [N][16 WN] and the Z tile [64][N + 1] staged
-// in shared memory once; thread (tx, ty) of 16 x 16 owns samples 4 ty .. +3
-// and nodes tx + 16 w.  Sums over k in order, as fcfit_dx_kernel: the same
-// results.
-template <int WN>
-__global__ void __launch_bounds__(256)
+// 8 TY samples blockIdx.y), A_b [N][16 WN] and the Z tile, transposed, staged
+// in shared memory once; thread (tx, ty) of 16 x TY owns samples 8 ty .. + 7
+// and nodes 2 tx + 32 w, + 1.  Sums over k in order, as fcfit_dx_kernel: the
+// same results.  Bound by shared memory and the FP32 pipe: 2 + WN / 2 loads for
+// 4 WN packed FMAs per k; with 4 samples per thread and a load for each operand
+// (10 for 24 FMAs) it took 460 us for 256 x 84 series of 2000 samples, 268 now.
+template <int WN, int TY>
+__global__ void __launch_bounds__(16 * TY)
     fcfit_dx_rows_kernel(SeriesView v, const float* __restrict__ fs, const float* __restrict__ A,
                          float* __restrict__ dx, int64_t dxs) {
-    extern __shared__ float sm[];
-    constexpr int NP = 16 * WN;
+    extern __shared__ __align__(16) float sm[];
+    constexpr int NP = 16 * WN, TS = 8 * TY, ZS = TS + 4;
     const int b = blockIdx.x;
     const int T = v.T, N = v.N;
-    const int t0 = blockIdx.y * 64;
+    const int t0 = blockIdx.y * TS;
     float* sA = sm;             // [N][NP]
-    float* sZ = sm + N * NP;    // [64][N + 1]
-    const int zs = N + 1;
+    float* sZ = sm + N * NP;    // [N][ZS]
     const float* fb = fs + static_cast<int64_t>(b) * N * 3;
     const float* Ab = A + static_cast<size_t>(b) * N * N;
-    for (int e = threadIdx.x; e < N * NP; e += 256) {
-        const int k = e / NP, j = e % NP;
-        sA[e] = j < N ? __ldg(Ab + static_cast<size_t>(k) * N + j) : 0.0f;
-    }
-    for (int e = threadIdx.x; e < 64 * N; e += 256) {
-        const int r = e / N, k = e % N;
-        const int t = t0 + r;
-        sZ[r * zs + k] = t < T ? (v.at(b, t, k) - fb[3 * k]) * fb[3 * k + 1] : 0.0f;
+    const int lane = threadIdx.x % 32, warp = threadIdx.x / 32;
+    constexpr int kWarps = TY / 2;
+    for (int k = warp; k < N; k += kWarps)
+#pragma unroll
+        for (int j = lane; j < NP; j += 32) sA[k * NP + j] = j < N ? __ldg(Ab + static_cast<size_t>(k) * N + j) : 0.0f;
+    for (int k = lane; k < N; k += 32) {   // a warp takes whole samples, its lanes the nodes
+        const tvbg::SeriesRow row(v, b, k);
+        const float mean = fb[3 * k], inv = fb[3 * k + 1];
+#pragma unroll
+        for (int r0 = 0; r0 < TS; r0 += 8 * kWarps) {
+            float x[8];
+#pragma unroll
+            for (int u = 0; u < 8; ++u) {
+                const int t = t0 + r0 + u * kWarps + warp;
+                x[u] = t < T ? row.at(t) : mean;
+            }
+#pragma unroll
+            for (int u = 0; u < 8; ++u) sZ[k * ZS + r0 + u * kWarps + warp] = (x[u] - mean) * inv;
+        }
     }
     __syncthreads();
     const int tx = threadIdx.x % 16, ty = threadIdx.x / 16;
-    float acc[4][WN] = {};
+    float2 acc[8][WN / 2];
+#pragma unroll
+    for (int u = 0; u < 8; ++u)
+#pragma unroll
+        for (int w = 0; w < WN / 2; ++w) acc[u][w] = make_float2(0.0f, 0.0f);
+#pragma unroll 2
     for (int k = 0; k < N; ++k) {
-        float z[4], a[WN];
+        float z[8];
+        *reinterpret_cast<float4*>(z) = *reinterpret_cast<const float4*>(sZ + k * ZS + 8 * ty);
+        *reinterpret_cast<float4*>(z + 4) = *reinterpret_cast<const float4*>(sZ + k * ZS + 8 * ty + 4);
+        float2 a[WN / 2];
 #pragma unroll
-        for (int u = 0; u < 4; ++u) z[u] = sZ[(ty * 4 + u) * zs + k];
+        for (int w = 0; w < WN / 2; ++w) a[w] = *reinterpret_cast<const float2*>(sA + k * NP + 2 * tx + 32 * w);
 #pragma unroll
-        for (int w = 0; w < WN; ++w) a[w] = sA[k * NP + tx + 16 * w];
+        for (int u = 0; u < 8; ++u)
 #pragma unroll
-        for (int u = 0; u < 4; ++u)
-#pragma unroll
-            for (int w = 0; w < WN; ++w) acc[u][w] = fmaf(z[u], a[w], acc[u][w]);
+            for (int w = 0; w < WN / 2; ++w) acc[u][w] = __ffma2_rn(make_float2(z[u], z[u]), a[w], acc[u][w]);
     }
 #pragma unroll
-    for (int u = 0; u < 4; ++u) {
-        const int t = t0 + ty * 4 + u;
-        if (t >= T) continue;
+    for (int w = 0; w < WN / 2; ++w)
 #pragma unroll
-        for (int w = 0; w < WN; ++w) {
-            const int j = tx + 16 * w;
+        for (int c = 0; c < 2; ++c) {
+            const int j = 2 * tx + 32 * w + c;
             if (j >= N) continue;
-            const float z = sZ[(ty * 4 + u) * zs + j];
-            dx[b * dxs + static_cast<int64_t>(t) * N + j] =
-                fmaf(-z, fb[3 * j + 2], acc[u][w] * fb[3 * j + 1]);
+            const float inv = fb[3 * j + 1], zg = fb[3 * j + 2];
+#pragma unroll
+            for (int u = 0; u < 8; ++u) {
+                const int t = t0 + ty * 8 + u;
+                if (t < T)
+                    dx[b * dxs + static_cast<int64_t>(t) * N + j] =
+                        fmaf(-sZ[j * ZS + ty * 8 + u], zg, (c ? acc[u][w].y : acc[u][w].x) * inv);
+            }
         }
-    }
 }
 
 template <int WN>
 int launch_dx_rows(SeriesView v, const float* fs, const float* A, float* dx, int64_t dxs, int n_inst,
                    cudaStream_t st) {
-    const size_t smem = 4u * (static_cast<size_t>(v.N) * 16 * WN + 64u * (v.N + 1));
+    constexpr int TY = WN < 8 ? 16 : 8;   // two CTAs per SM at the largest N
+    const size_t smem = 4u * static_cast<size_t>(v.N) * (16 * WN + 8 * TY + 4);
     if (smem > 48u * 1024u) {
-        const cudaError_t e = cudaFuncSetAttribute(reinterpret_cast<const void*>(fcfit_dx_rows_kernel<WN>),
+        const cudaError_t e = cudaFuncSetAttribute(reinterpret_cast<const void*>(fcfit_dx_rows_kernel<WN, TY>),
                                                    cudaFuncAttributeMaxDynamicSharedMemorySize,
                                                    static_cast<int>(smem));
         if (e != cudaSuccess) return tvbg::set_cuda_error(e, "tvbg_fcfit_loss: smem attribute");
     }
-    const dim3 grid(static_cast<unsigned>(n_inst), static_cast<unsigned>((v.T + 63) / 64));
-    fcfit_dx_rows_kernel<WN><<<grid, 256, smem, st>>>(v, fs, A, dx, dxs);
+    const dim3 grid(static_cast<unsigned>(n_inst), static_cast<unsigned>((v.T + 8 * TY - 1) / (8 * TY)));
+    fcfit_dx_rows_kernel<WN, TY><<<grid, 16 * TY, smem, st>>>(v, fs, A, dx, dxs);
     return TVBG_OK;
 }
 
