@@ -23,6 +23,8 @@ namespace tvbg {
 
 constexpr int kCovThreads = 256;
 constexpr int kCovTile = 32;
+// static shared memory of cov_update_kernel: its transposing tile
+constexpr size_t kCovStaticBytes = sizeof(double) * kCovTile * (kCovTile + 1);
 
 // Tile (ti <= tj) q of the upper triangle of nt x nt tiles, row-major.
 __device__ __forceinline__ void cov_tile(int q, int nt, int& ti, int& tj) {
@@ -158,7 +160,7 @@ static int cov_rows(const float* x, int64_t inst_stride, int64_t row_stride, int
     RC = RC > 16 ? 16 : (RC < 4 ? 4 : RC);
     if (RC > rows) RC = rows;
     const size_t smem = sizeof(double) * static_cast<size_t>(N) * (1 + 2 * RC);
-    if (smem > 48u * 1024u) {
+    if (smem + kCovStaticBytes > 48u * 1024u) {   // the kernel's own tile counts too
         const cudaError_t e = cudaFuncSetAttribute(cov_update_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                                    static_cast<int>(smem));
         if (e != cudaSuccess) return set_cuda_error(e, "tvbg_cov_update: smem attribute");
