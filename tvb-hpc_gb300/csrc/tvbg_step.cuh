@@ -101,10 +101,14 @@ struct SmemPlan {
 };
 
 // Stage `bytes` from global `src` into shared `dst` with bulk copies, waiting
-// on the mbarrier with a bounded poll.  Returns false on timeout.
+// on the mbarrier with a bounded poll.  Returns false on timeout.  Called after
+// a CTA barrier; what the CTA stored to `dst` by ordinary stores before it (the
+// instance before this one, in a persistent launch) is ordered before the
+// copies, which write through the async proxy, by the fence.
 __device__ __forceinline__ bool tma_load(uint32_t dst, const void* src, uint32_t bytes,
                                          uint32_t bar, uint32_t& phase) {
     if (threadIdx.x == 0) {
+        fence_proxy_async();
         mbar_expect_tx(bar, bytes);
         constexpr uint32_t kChunk = 32768;
         for (uint32_t off = 0; off < bytes; off += kChunk) {
