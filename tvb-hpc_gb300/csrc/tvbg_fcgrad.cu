@@ -173,13 +173,6 @@ constexpr int kSplitMaxN = 192;   // staging (kSplitL + 1) x N pairs of words <=
 constexpr int kSplitThreads = 128;
 constexpr int kSplitWarps = kSplitThreads / 32;
 
-__device__ __forceinline__ float2 sub2(float2 a, float2 b) { return __ffma2_rn(b, make_float2(-1.0f, -1.0f), a); }
-__device__ __forceinline__ void two_sum2(float2 a, float2 b, float2& s, float2& e) {
-    s = __fadd2_rn(a, b);
-    const float2 bb = sub2(s, a);
-    e = __fadd2_rn(sub2(a, sub2(s, bb)), sub2(b, bb));
-}
-
 // Tiles of row block bi: column blocks from its first pair on or above the
 // diagonal.
 template <int RB>
@@ -288,7 +281,7 @@ __global__ void __launch_bounds__(kSplitThreads, 4) fcfit_gram_split_kernel(Seri
                         const float2 ne = __ffma2_rn(nh, yh[w], p);  // p - hi hi, exact
                         nm[u][w] = __fadd2_rn(nm[u][w], __ffma2_rn(nh, yl[w], __ffma2_rn(nq, yh[w], ne)));
                         float2 t, err;
-                        two_sum2(s[u][w], p, t, err);
+                        tvbg::gram_two_sum2(s[u][w], p, t, err);
                         s[u][w] = t;
                         cp[u][w] = __fadd2_rn(cp[u][w], err);
                     }
@@ -299,9 +292,9 @@ __global__ void __launch_bounds__(kSplitThreads, 4) fcfit_gram_split_kernel(Seri
 #pragma unroll
                 for (int w = 0; w < 2; ++w) {  // (ah, al) += s + (cp + small words)
                     float2 hi, lo;
-                    two_sum2(ah[u][w], s[u][w], hi, lo);
-                    lo = __fadd2_rn(lo, __fadd2_rn(al[u][w], sub2(cp[u][w], nm[u][w])));
-                    two_sum2(hi, lo, ah[u][w], al[u][w]);
+                    tvbg::gram_two_sum2(ah[u][w], s[u][w], hi, lo);
+                    lo = __fadd2_rn(lo, __fadd2_rn(al[u][w], tvbg::gram_sub2(cp[u][w], nm[u][w])));
+                    tvbg::gram_two_sum2(hi, lo, ah[u][w], al[u][w]);
                 }
         }
         __syncthreads();
