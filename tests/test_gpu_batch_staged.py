@@ -50,3 +50,32 @@ def test_sigmoidal_instances_in_turn(cuda, sizes):
         far.run(nsteps)
         assert rel_err(one.state.cpu().numpy(), far.state.cpu().numpy()) < 1e-5
         assert rel_err(one.ring.cpu().numpy(), far.ring.cpu().numpy()) < 1e-5
+
+
+def test_cta_width_follows_the_ring_of_each_launch(cuda):
+    """Rings of 64 and 512 slots in one sweep: the launch whose staged ring leaves one
+    CTA per SM has 512 threads, the one whose CTAs share an SM 256; the results are those of one speed at
+    a time."""
+    speeds = [4.0, 40.0]
+    w, ln = network.synthetic_connectome(68, 0.3, seed=0)
+    conn = network.Connectivity.from_dense(w, ln)
+    m = model.MPR()
+    x0 = np.random.default_rng(1).uniform(0.05, 0.3, (6, 68, 2)).astype(np.float32)
+
+    def sweep(v, ids):
+        return engine.Sweep(m, coupling.Linear(m), scheme.EulerMaryuyamaStep(0.1), conn, dt=0.1,
+                            couplings=np.full(len(ids), 0.1), speeds=np.asarray(v, np.float32),
+                            state0=x0[ids], seed=5, tpn=4, inst_ids=ids)
+
+    s = sweep(np.resize(speeds, 6), np.arange(6))
+    width = {}
+    for _, _, smem, bk in s.prepare(40):
+        assert smem > 0 and bk > 0
+        width[2 * smem > s.smem_cap] = s._launch_cfg(smem, 4, bk).threads
+    assert width == {True: 512, False: 256}
+    s.run(40)
+    for k, v in enumerate(speeds):
+        ids = np.arange(k, 6, 2)
+        one = sweep([v] * 3, ids)
+        one.run(40)
+        assert np.array_equal(s.state.cpu().numpy()[ids], one.state.cpu().numpy())

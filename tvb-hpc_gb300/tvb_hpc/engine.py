@@ -340,9 +340,7 @@ class InstanceSet:
         cap = max_smem()
         self.ring_bytes = N * self.stride * 4
         self.smem_cap = cap
-        # staged rings of more than half the shared memory leave one CTA per SM:
-        # the blocked kernel then takes 512 threads, mostly gathering warps
-        # (results do not depend on it)
+        # whether some ring is staged and fills more than half the shared memory
         self._one_cta = any(2 * r > cap and r <= self.smem_ring_limit(0, k)
                             for r, k in set(zip(self.ring_bytes.tolist(), self.block_k.tolist())) if k)
         self.table = None
@@ -360,19 +358,34 @@ class InstanceSet:
             self.ring[o:o + N * R] = torch.from_numpy(
                 np.repeat(obs0[b], R).astype(np.float32)).cuda()
 
-    def threads(self, blocked_k=0):
+    def threads(self, blocked_k=0, smem_ring=None):
+        """CTA width.  Staged rings of more than half the shared memory leave one
+        CTA per SM: the blocked kernel then takes 512 threads, mostly gathering
+        warps, else 256.  Results do not depend on it.  smem_ring: the staged bytes
+        of one launch of a set that has such rings; where four CTAs of 256 threads
+        find room beside each other (their registers fill an SM), that launch keeps
+        256 (68 nodes, 2000 instances at 4, 8, 16 and 32 m/s, 400 steps: 1.71 ms, 1.92
+        with 512 in every launch; 84 nodes, 1000 at 5 and 20 m/s, three CTAs an SM at
+        20 m/s: 1.21 with 512, 1.29 with 256)."""
+        one_cta = self._one_cta
+        if one_cta and blocked_k and smem_ring is not None:
+            # an SM has 1 KB beyond one CTA's limit, and takes 1 KB for each CTA
+            cta = smem_ring + self.blocked_aux(blocked_k) + _SMEM_RESERVE + 1024
+            one_cta = 4 * cta > self.smem_cap + 1024
         own = 32 * ((self.N + 31) // 32)
         if blocked_k and self.warps:
             return min(1024, max(own + 32, 32 * int(self.warps)))
         if blocked_k:
-            return min(1024, max(own + 32, 512 if self._one_cta else 256))
+            return min(1024, max(own + 32, 512 if one_cta else 256))
         return own
+
+    def blocked_aux(self, blocked_k):
+        "Shared memory of a CTA of the blocked kernel beyond its ring."
+        return 4 * (2 * blocked_k * self.N * (2 + self.ns) + 4 * self.N) + 32
 
     def smem_ring_limit(self, threads, blocked_k=0):
         if blocked_k:
-            ns = self.ns
-            aux = 4 * (2 * blocked_k * self.N * (2 + ns) + 4 * self.N) + 32
-            return self.smem_cap - aux - _SMEM_RESERVE
+            return self.smem_cap - self.blocked_aux(blocked_k) - _SMEM_RESERVE
         return self.smem_cap - 4 * threads - 16 - _SMEM_RESERVE
 
     def build_table(self, nsteps, smem_allowed=True):
@@ -465,7 +478,7 @@ class Sweep(InstanceSet):
         cfg = nat.tvbg_launch()
         cfg.model = self.model_id
         cfg.cfun = self.cfun_id
-        cfg.threads = self.threads(block_k)
+        cfg.threads = self.threads(block_k, smem_ring)
         cfg.tpn = int(tpn)
         if block_k and cfg.tpn < 2:
             cfg.tpn = 2
