@@ -25,6 +25,12 @@ constexpr int kCovThreads = 256;
 constexpr int kCovTile = 32;
 // static shared memory of cov_update_kernel: its transposing tile
 constexpr size_t kCovStaticBytes = sizeof(double) * kCovTile * (kCovTile + 1);
+constexpr int kCovNodes = 3000;                     // largest network
+constexpr int64_t kCovPassBytes = 192 * 1024;       // a pass's d and e, at least four samples
+// the most dynamic shared memory of a launch: the limit that every launch asks
+// for (another thread's smaller one may come between that and the launch)
+constexpr size_t kCovSmemMax = sizeof(double) * kCovNodes + (kCovPassBytes > 64 * kCovNodes ? kCovPassBytes : 64 * kCovNodes);
+static_assert(kCovSmemMax + kCovStaticBytes <= 227 * 1024, "shared memory of a CTA");
 
 // Tile (ti <= tj) q of the upper triangle of nt x nt tiles, row-major.
 __device__ __forceinline__ void cov_tile(int q, int nt, int& ti, int& tj) {
@@ -155,14 +161,14 @@ __global__ void __launch_bounds__(kCovThreads)
 // Launch over all instances (gridDim.y at most 65535 at a time).
 static int cov_rows(const float* x, int64_t inst_stride, int64_t row_stride, int rows, int n_inst, int N, int64_t n,
                     double* mean, double* m2, cudaStream_t st) {
-    // samples per pass: their d and e in at most 192 KB, at least four
-    int RC = static_cast<int>(192 * 1024 / (16 * static_cast<int64_t>(N)));
+    // samples per pass: as many as kCovPassBytes holds, 4 to 16
+    int RC = static_cast<int>(kCovPassBytes / (16 * static_cast<int64_t>(N)));
     RC = RC > 16 ? 16 : (RC < 4 ? 4 : RC);
     if (RC > rows) RC = rows;
     const size_t smem = sizeof(double) * static_cast<size_t>(N) * (1 + 2 * RC);
     if (smem + kCovStaticBytes > 48u * 1024u) {   // the kernel's own tile counts too
         const cudaError_t e = cudaFuncSetAttribute(cov_update_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                   static_cast<int>(smem));
+                                                   static_cast<int>(kCovSmemMax));
         if (e != cudaSuccess) return set_cuda_error(e, "tvbg_cov_update: smem attribute");
     }
     const int nt = (N + kCovTile - 1) / kCovTile, tiles = nt * (nt + 1) / 2;
@@ -197,7 +203,7 @@ extern "C" int tvbg_cov_update_rows(const float* d_x, int64_t x_stride, int64_t 
                                     void* stream) {
     if (n_inst < 0 || rows < 0 || N <= 0 || n < 0 || x_stride < N || (n_inst > 0 && (!d_x || !d_mean || !d_m2)))
         return set_error(TVBG_EINVAL, "tvbg_cov_update: bad arguments");
-    if (N > 3000) return set_error(TVBG_EINVAL, "tvbg_cov_update: N above 3000");
+    if (N > kCovNodes) return set_error(TVBG_EINVAL, "tvbg_cov_update: N above 3000");
     if (n_inst == 0 || rows == 0) return TVBG_OK;
     return cov_rows(d_x, x_stride, row_stride, rows, n_inst, N, n, d_mean, d_m2,
                     static_cast<cudaStream_t>(stream));

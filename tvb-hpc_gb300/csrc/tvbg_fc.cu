@@ -206,7 +206,11 @@ extern "C" int tvbg_fc_ex(const float* d_x, int32_t n_inst, int32_t T, int32_t N
         const bool half = N <= 96;
         const size_t smem = gram_plane_bytes(half ? 96 : 128) + sizeof(double) * (static_cast<size_t>(N) * (N + 1) / 2);
         auto kfn = half ? fc_small_kernel<96> : fc_small_kernel<128>;
-        cudaError_t e = cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+        // the limit of the kernel's largest N: another thread's smaller call may
+        // come between this and the launch
+        const int top = half ? 96 : kFcSmallMax;
+        const size_t most = gram_plane_bytes(half ? 96 : 128) + sizeof(double) * (static_cast<size_t>(top) * (top + 1) / 2);
+        cudaError_t e = cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(most));
         if (e != cudaSuccess) return set_cuda_error(e, "tvbg_fc: smem attribute");
         kfn<<<n_inst, kGramThreads, smem, st>>>(v, d_fc, d_target, d_err);
     } else {

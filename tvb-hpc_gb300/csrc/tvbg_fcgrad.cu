@@ -321,8 +321,11 @@ int launch_gram_split(SeriesView v, const double* mean, double* G, int n_inst, c
     const int parts = (tiles + kSplitThreads - 1) / kSplitThreads;
     const size_t smem = 8u * (kSplitL + 1) * 4u * static_cast<size_t>((v.N + 3) / 4);
     if (smem > 48u * 1024u) {
+        // the limit of the largest N: another thread's smaller call may come
+        // between this and the launch
         const cudaError_t e = cudaFuncSetAttribute(fcfit_gram_split_kernel<RB>,
-                                                   cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+                                                   cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                   static_cast<int>(8u * (kSplitL + 1) * kSplitMaxN));
         if (e != cudaSuccess) return tvbg::set_cuda_error(e, "tvbg_fcfit_loss: smem attribute");
     }
     fcfit_gram_split_kernel<RB><<<dim3(n_inst, parts), kSplitThreads, smem, st>>>(v, mean, (tiles + parts - 1) / parts, G);
@@ -556,7 +559,7 @@ int launch_dx_rows(SeriesView v, const float* fs, const float* A, float* dx, int
     if (smem > 48u * 1024u) {
         const cudaError_t e = cudaFuncSetAttribute(reinterpret_cast<const void*>(fcfit_dx_rows_kernel<WN, TY>),
                                                    cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                   static_cast<int>(smem));
+                                                   static_cast<int>(4u * 16 * WN * (16 * WN + 8 * TY + 4)));
         if (e != cudaSuccess) return tvbg::set_cuda_error(e, "tvbg_fcfit_loss: smem attribute");
     }
     const dim3 grid(static_cast<unsigned>(n_inst), static_cast<unsigned>((v.T + 8 * TY - 1) / (8 * TY)));

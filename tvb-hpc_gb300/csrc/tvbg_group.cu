@@ -112,7 +112,7 @@ int tvbg_group_occupancy(const tvbg_launch* cfg, int32_t* ctas_per_sm, int32_t* 
     cudaError_t e = cudaSuccess;
     if (smem + kGroupStaticBytes > 48u * 1024u) {  // beyond the default: opt in
         e = cudaFuncSetAttribute(reinterpret_cast<const void*>(kfn),
-                                 cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+                                 cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kGroupSmemMax));
         if (e != cudaSuccess) return set_cuda_error(e, "tvbg_group_occupancy: smem attribute");
     }
     e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, reinterpret_cast<const void*>(kfn),
@@ -137,7 +137,7 @@ int tvbg_group_max_clusters(const tvbg_launch* cfg, int32_t* max_clusters) {
     cudaError_t e = cudaSuccess;
     if (smem + kGroupStaticBytes > 48u * 1024u) {
         e = cudaFuncSetAttribute(reinterpret_cast<const void*>(kfn),
-                                 cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+                                 cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kGroupSmemMax));
         if (e != cudaSuccess) return set_cuda_error(e, "tvbg_group_max_clusters: smem attribute");
     }
     if (cluster > 8) {

@@ -64,7 +64,7 @@ inline int launch_group_kernel(GroupKernelFn kfn, const tvbg_group* d_groups, in
     cudaError_t e = cudaSuccess;
     if (smem + kGroupStaticBytes > 48u * 1024u) {  // beyond the default: opt in
         e = cudaFuncSetAttribute(reinterpret_cast<const void*>(kfn),
-                                 cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+                                 cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kGroupSmemMax));
         if (e != cudaSuccess) return es.cuda(e, "tvbg_group_run: smem attribute");
     }
     if (cluster > 8) {  // 9..16 CTAs: a non-portable cluster size, opted in per kernel

@@ -915,6 +915,14 @@ __global__ void __launch_bounds__(BOUND, 1)
     run_group<M, CF, K, BOUND>(s_grp, csum, s_stage, status);
 }
 
+// The most dynamic shared memory that a group CTA takes (8 steps, 1024 threads,
+// two channels).  A kernel whose CTAs need the opt-in is given this limit at
+// every launch, not its CTAs' own size: the limit belongs to the kernel, and
+// another thread's launch of a smaller CTA would lower it between the two calls.
+constexpr size_t kGroupSmemMax = group_smem_bytes(8, 1024, 2) > group_pipelined_smem_bytes(8, 1024, 2)
+                                     ? group_smem_bytes(8, 1024, 2)
+                                     : group_pipelined_smem_bytes(8, 1024, 2);
+
 // Pipelined variant (run_group_pipelined): blockDim = 2 teams x 8 lanes x
 // node slots; same tables and results as group_kernel.
 template <class M, int CF, int K, int BOUND = 1024>

@@ -167,7 +167,9 @@ int tvbg_rmap_to_avg(int32_t nroi, int32_t nvar, int32_t nnode, const int32_t* d
                         : nvar == 4 ? rmap_to_avg_kernel<4>
                                     : rmap_to_avg_kernel<0>;
     const void* kfn = reinterpret_cast<const void*>(kernel);
-    cudaError_t e = cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+    // the limit of the largest call: another thread's smaller one may come between this and the launch
+    cudaError_t e = cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         static_cast<int>(sizeof(float) * kWarps * kBins));
     if (e == cudaSuccess) e = cudaFuncSetAttribute(kfn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
     if (e != cudaSuccess) return tvbg::set_cuda_error(e, "tvbg_rmap_to_avg: kernel attributes");
     cudaLaunchConfig_t lc;

@@ -318,7 +318,7 @@ bool pipelined_fits(const Request& r) {
         if (smem + kGroupStaticBytes > 48u * 1024u &&
             cudaFuncSetAttribute(reinterpret_cast<const void*>(kfn),
                                  cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 static_cast<int>(smem)) != cudaSuccess)
+                                 static_cast<int>(kGroupSmemMax)) != cudaSuccess)
             return (cudaGetLastError(), false);
         if (r.cluster > 8 &&
             cudaFuncSetAttribute(reinterpret_cast<const void*>(kfn),
