@@ -626,18 +626,25 @@ int tvbg_pack_edges_group(int32_t N, int32_t nnz, const int32_t *row,
 int tvbg_group_run(const tvbg_group *d_groups, int32_t n_groups,
                    const tvbg_launch *cfg, void *stream);
 
-/* Resident CTAs per SM of the group kernel of `cfg`, and the SM count. */
+/* The most CTAs of the group kernel of `cfg` that an SM holds, and the SM
+ * count.  Pipelined CTAs of at most 512 threads have two builds, and a launch
+ * takes the one with more registers a thread, of which fewer are resident,
+ * unless the other needs fewer waves: the answer is the larger one's, which
+ * launches of that many CTAs take. */
 int tvbg_group_occupancy(const tvbg_launch *cfg, int32_t *ctas_per_sm,
                          int32_t *sms);
 
 /*
  * Clusters of cfg->cluster CTAs of the group kernel of `cfg` that can be
  * resident at once (cudaOccupancyMaxActiveClusters); 0 when the shape
- * cannot be launched on the current device.  Used by the batch tuner to
+ * cannot be launched on the current device: the most of any launch, or (_for)
+ * those of a launch of n_groups groups (0: any).  Used by the batch tuner to
  * skip shapes; no counterpart in the reference (its launch shape is a
  * command-line choice, dsl/dsl_cuda/example/cuda_setup.py:53-86).
  */
 int tvbg_group_max_clusters(const tvbg_launch *cfg, int32_t *max_clusters);
+int tvbg_group_max_clusters_for(const tvbg_launch *cfg, int32_t n_groups,
+                                int32_t *max_clusters);
 
 /*
  * dL/dZ = Z A of the FC-fit loss for n_inst instances: d_z [n_inst][T][N]

@@ -24,18 +24,70 @@ GroupKernel lookup_group(int model, int cfun, int k, GroupForm form) {
 const ErrSink kSink{set_error, set_cuda_error};
 
 // Validate a group launch; its dynamic shared memory holds the K coupling
-// sums of every thread.
-int check_group_launch(const tvbg_launch* cfg, int32_t n_groups, GroupKernel* kfn, int* cluster,
-                       size_t* smem) {
+// sums of every thread and the staged edge records.
+int check_group_launch(const tvbg_launch* cfg, int* cluster, size_t* smem) {
     int rc = check_group_cfg(cfg, kSink, cluster, (1u << 4) | (1u << 8), true);
     if (rc) return rc;
+    *smem = cfg->tpn == TVBG_GROUP_PIPELINED
+                ? group_pipelined_smem_bytes(cfg->block_k, cfg->threads, group_channels(cfg->cfun))
+                : group_smem_bytes(cfg->block_k, cfg->threads, group_channels(cfg->cfun));
+    return TVBG_OK;
+}
+
+int find_kernel(const tvbg_launch* cfg, GroupForm form, GroupKernel* kfn) {
+    *kfn = lookup_group(cfg->model, cfg->cfun, cfg->block_k, form);
+    return *kfn ? TVBG_OK
+                : set_error(TVBG_EUNSUPPORTED, "group kernel not built for this model/coupling/block_k");
+}
+
+int opt_in(GroupKernel kfn, int cluster, size_t smem) {
+    cudaError_t e = cudaSuccess;
+    if (smem + kGroupStaticBytes > 48u * 1024u)  // beyond the default
+        e = cudaFuncSetAttribute(reinterpret_cast<const void*>(kfn), cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 static_cast<int>(kGroupSmemMax));
+    if (e == cudaSuccess && cluster > 8)
+        e = cudaFuncSetAttribute(reinterpret_cast<const void*>(kfn), cudaFuncAttributeNonPortableClusterSizeAllowed,
+                                 1);
+    return e == cudaSuccess ? TVBG_OK : set_cuda_error(e, "group kernel attributes");
+}
+
+// The builds that launches of cfg's shape take, by their number of CTAs
+// (group_form): returns their count.
+int shape_forms(const tvbg_launch* cfg, GroupForm forms[2]) {
     const bool pipe = cfg->tpn == TVBG_GROUP_PIPELINED;
-    *kfn = lookup_group(cfg->model, cfg->cfun, cfg->block_k,
-                        group_form(cfg->threads, static_cast<long long>(n_groups) * *cluster, pipe));
-    if (!*kfn)
-        return set_error(TVBG_EUNSUPPORTED, "group kernel not built for this model/coupling/block_k");
-    *smem = pipe ? group_pipelined_smem_bytes(cfg->block_k, cfg->threads, group_channels(cfg->cfun))
-                 : group_smem_bytes(cfg->block_k, cfg->threads, group_channels(cfg->cfun));
+    if (pipe && cfg->threads <= 512) {
+        forms[0] = kPipe512;
+        forms[1] = kPipe768;
+        return 2;
+    }
+    forms[0] = group_form(cfg->threads, 1, pipe);
+    return 1;
+}
+
+// Clusters of one build that are resident at once.
+int resident_clusters(const tvbg_launch* cfg, GroupForm form, int cluster, size_t smem, int32_t* clusters) {
+    GroupKernel kfn = nullptr;
+    int rc = find_kernel(cfg, form, &kfn);
+    if (!rc) rc = opt_in(kfn, cluster, smem);
+    if (rc) return rc;
+    cudaLaunchConfig_t lc;
+    std::memset(&lc, 0, sizeof(lc));
+    lc.gridDim = dim3(static_cast<unsigned>(cluster), 1, 1);
+    lc.blockDim = dim3(static_cast<unsigned>(cfg->threads), 1, 1);
+    lc.dynamicSmemBytes = smem;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = static_cast<unsigned>(cluster);
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    lc.attrs = attr;
+    lc.numAttrs = 1;
+    int n = 0;
+    if (cudaOccupancyMaxActiveClusters(&n, reinterpret_cast<const void*>(kfn), &lc) != cudaSuccess) {
+        cudaGetLastError();  // an unschedulable shape is reported here, before any launch
+        n = 0;
+    }
+    *clusters = n;
     return TVBG_OK;
 }
 
@@ -96,75 +148,66 @@ int tvbg_group_run(const tvbg_group* d_groups, int32_t n_groups, const tvbg_laun
     GroupKernel kfn = nullptr;
     int cluster = 1;
     size_t smem = 0;
-    int rc = check_group_launch(cfg, n_groups, &kfn, &cluster, &smem);
+    int rc = check_group_launch(cfg, &cluster, &smem);
+    if (!rc)
+        rc = find_kernel(cfg, group_form(cfg->threads, static_cast<long long>(n_groups) * cluster,
+                                         cfg->tpn == TVBG_GROUP_PIPELINED), &kfn);
     if (rc) return rc;
     return launch_group_kernel(kfn, d_groups, n_groups, cfg, cluster, smem, stream, kSink);
 }
 
 int tvbg_group_occupancy(const tvbg_launch* cfg, int32_t* ctas_per_sm, int32_t* sms) {
     if (!ctas_per_sm || !sms) return set_error(TVBG_EINVAL, "tvbg_group_occupancy: null");
-    GroupKernel kfn = nullptr;
     int cluster = 1;
     size_t smem = 0;
-    int rc = check_group_launch(cfg, 1, &kfn, &cluster, &smem);
+    int rc = check_group_launch(cfg, &cluster, &smem);
     if (rc) return rc;
-    int n = 0;
-    cudaError_t e = cudaSuccess;
-    if (smem + kGroupStaticBytes > 48u * 1024u) {  // beyond the default: opt in
-        e = cudaFuncSetAttribute(reinterpret_cast<const void*>(kfn),
-                                 cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kGroupSmemMax));
-        if (e != cudaSuccess) return set_cuda_error(e, "tvbg_group_occupancy: smem attribute");
+    GroupForm forms[2];
+    const int nf = shape_forms(cfg, forms);
+    int most = 0;
+    for (int i = 0; i < nf; ++i) {
+        GroupKernel kfn = nullptr;
+        rc = find_kernel(cfg, forms[i], &kfn);
+        if (!rc) rc = opt_in(kfn, 1, smem);
+        if (rc) return rc;
+        int n = 0;
+        const cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, reinterpret_cast<const void*>(kfn),
+                                                                            cfg->threads, smem);
+        if (e != cudaSuccess) return set_cuda_error(e, "cudaOccupancyMaxActiveBlocksPerMultiprocessor");
+        most = n > most ? n : most;
     }
-    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, reinterpret_cast<const void*>(kfn),
-                                                      cfg->threads, smem);
-    if (e != cudaSuccess) return set_cuda_error(e, "cudaOccupancyMaxActiveBlocksPerMultiprocessor");
-    int dev = 0, nsm = 0;
-    e = cudaGetDevice(&dev);
-    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-    if (e != cudaSuccess) return set_cuda_error(e, "tvbg_group_occupancy: SM count");
-    *ctas_per_sm = n;
+    const int nsm = device_sms();
+    if (nsm <= 0) return set_error(TVBG_ECUDA, "tvbg_group_occupancy: SM count");
+    *ctas_per_sm = most;
     *sms = nsm;
     return TVBG_OK;
 }
 
-int tvbg_group_max_clusters(const tvbg_launch* cfg, int32_t* max_clusters) {
-    if (!max_clusters) return set_error(TVBG_EINVAL, "tvbg_group_max_clusters: null");
-    GroupKernel kfn = nullptr;
+int tvbg_group_max_clusters_for(const tvbg_launch* cfg, int32_t n_groups, int32_t* max_clusters) {
+    if (!max_clusters || n_groups < 0) return set_error(TVBG_EINVAL, "tvbg_group_max_clusters: bad arguments");
     int cluster = 1;
     size_t smem = 0;
-    int rc = check_group_launch(cfg, 1, &kfn, &cluster, &smem);
+    int rc = check_group_launch(cfg, &cluster, &smem);
     if (rc) return rc;
-    cudaError_t e = cudaSuccess;
-    if (smem + kGroupStaticBytes > 48u * 1024u) {
-        e = cudaFuncSetAttribute(reinterpret_cast<const void*>(kfn),
-                                 cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kGroupSmemMax));
-        if (e != cudaSuccess) return set_cuda_error(e, "tvbg_group_max_clusters: smem attribute");
+    if (n_groups > 0)
+        return resident_clusters(cfg, group_form(cfg->threads, static_cast<long long>(n_groups) * cluster,
+                                                 cfg->tpn == TVBG_GROUP_PIPELINED),
+                                 cluster, smem, max_clusters);
+    GroupForm forms[2];
+    const int nf = shape_forms(cfg, forms);
+    int32_t most = 0;
+    for (int i = 0; i < nf; ++i) {
+        int32_t n = 0;
+        rc = resident_clusters(cfg, forms[i], cluster, smem, &n);
+        if (rc) return rc;
+        most = n > most ? n : most;
     }
-    if (cluster > 8) {
-        e = cudaFuncSetAttribute(reinterpret_cast<const void*>(kfn),
-                                 cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-        if (e != cudaSuccess) return set_cuda_error(e, "tvbg_group_max_clusters: cluster attribute");
-    }
-    cudaLaunchConfig_t lc;
-    std::memset(&lc, 0, sizeof(lc));
-    lc.gridDim = dim3(static_cast<unsigned>(cluster), 1, 1);
-    lc.blockDim = dim3(static_cast<unsigned>(cfg->threads), 1, 1);
-    lc.dynamicSmemBytes = smem;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = static_cast<unsigned>(cluster);
-    attr[0].val.clusterDim.y = 1;
-    attr[0].val.clusterDim.z = 1;
-    lc.attrs = attr;
-    lc.numAttrs = 1;
-    int n = 0;
-    e = cudaOccupancyMaxActiveClusters(&n, reinterpret_cast<const void*>(kfn), &lc);
-    if (e != cudaSuccess) {
-        cudaGetLastError();  // an unschedulable shape is reported here, before any launch
-        n = 0;
-    }
-    *max_clusters = n;
+    *max_clusters = most;
     return TVBG_OK;
+}
+
+int tvbg_group_max_clusters(const tvbg_launch* cfg, int32_t* max_clusters) {
+    return tvbg_group_max_clusters_for(cfg, 0, max_clusters);
 }
 
 }  // extern "C"

@@ -270,6 +270,7 @@ SIGNATURES = {
     'tvbg_group_run': (ctypes.c_int, [_vp, _i32, ctypes.POINTER(tvbg_launch), _vp]),
     'tvbg_group_occupancy': (ctypes.c_int, [ctypes.c_void_p, _ip, _ip]),
     'tvbg_group_max_clusters': (ctypes.c_int, [ctypes.c_void_p, _ip]),
+    'tvbg_group_max_clusters_for': (ctypes.c_int, [ctypes.c_void_p, _i32, _ip]),
     'tvbg_fcfit_zgrad': (ctypes.c_int, [_vp, _vp, _vp, _i32, _i32, _i32, _vp]),
     'tvbg_fcfit_scratch_bytes': (ctypes.c_int, [_i32, _i32, ctypes.POINTER(_i64)]),
     'tvbg_fcfit_loss': (ctypes.c_int, [_vp, _i64, _vp, _i64, _i64, _i32, _i32, _i32, _i32, _vp,

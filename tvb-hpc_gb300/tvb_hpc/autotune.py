@@ -103,16 +103,17 @@ def group_shapes(N, min_threads=128, clusters=SHAPE_CLUSTERS, pipelined=False):
     return out
 
 
-def group_max_clusters(gset, threads, cluster, tpn=1):
+def group_max_clusters(gset, threads, cluster, tpn=1, n_groups=0):
     """Clusters of `cluster` CTAs of `threads` threads of gset's group kernel
     (tpn 2: the pipelined one) that can be resident at once (0: the shape
-    cannot be launched)."""
+    cannot be launched): of a launch of n_groups groups, or (0) the most of
+    any launch."""
     import ctypes
     from . import _native as nat
     cfg = gset.launch_cfg(int(gset.block_k.max()))
     cfg.threads, cfg.cluster, cfg.tpn = int(threads), int(cluster), int(tpn)
     n = ctypes.c_int32(0)
-    nat.check(nat.load().tvbg_group_max_clusters(ctypes.byref(cfg), ctypes.byref(n)))
+    nat.check(nat.load().tvbg_group_max_clusters_for(ctypes.byref(cfg), int(n_groups), ctypes.byref(n)))
     return int(n.value)
 
 

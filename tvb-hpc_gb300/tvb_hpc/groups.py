@@ -146,7 +146,7 @@ def spread_shape(gset, sms=None):
         return plain
     live = int(gset.pipe_tab[gset.gtab].sum())
     for t, c, _, tpn in reversed(shapes):
-        if G * c <= sms and group_max_clusters(gset, t, c, tpn) >= live:
+        if G * c <= sms and group_max_clusters(gset, t, c, tpn, live) >= live:
             return (t, c, 0, PIPELINED)
     limit = 768 if gset.channels == 1 else 512
     fits = [s for s in shapes if s[0] <= limit and s[1] != 12]
@@ -163,6 +163,7 @@ def device_sms():
 
 
 def group_occupancy(cfg):
+    "The most CTAs of a group launch that an SM holds, and the SM count."
     lib = nat.load()
     per, sms = ctypes.c_int32(0), ctypes.c_int32(0)
     nat.check(lib.tvbg_group_occupancy(ctypes.byref(cfg), ctypes.byref(per), ctypes.byref(sms)))
