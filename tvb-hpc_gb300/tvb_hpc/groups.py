@@ -154,7 +154,12 @@ def spread_shape(gset, sms=None):
         fits = [s for s in shapes if s[0] <= 768]
         if not fits:
             return plain
-    return fits[0] if fits else shapes[0]
+    # one that the device can hold at all: a device with few SMs to a GPC may
+    # have no room for a cluster of 16
+    for s in fits or shapes:
+        if group_max_clusters(gset, *s[:2], s[3], live) > 0:
+            return s
+    return plain
 
 
 def device_sms():
