@@ -127,3 +127,29 @@ def test_adjoint_footprint_counts_recompute_windows():
     assert 20 * per_seg < (2 << 30)
     assert full - small == 20 * per_seg - (1 << 28)
     assert small - tiny == (1 << 28) - per_seg
+
+
+def test_gradient_footprint_where_the_whole_trace_is_kept():
+    """Where FCFit keeps the whole trace (delays of the grouped layout, at most
+    TRACE_BUDGET bytes) a gradient request counts that trace, three rings, dL/dr and
+    the loss scratch, and no checkpoints or windows; longer runs and short
+    delays count those."""
+    from tvb_hpc import adjoint, serve
+    I, N, T, nh = 256, 84, 2000, 512
+    trace = 256 * T * N * 3 * 4
+    assert adjoint.trace_bytes(I, N, T) == trace
+    got = serve.fit_bytes(I, N, T, nh, 15, 500)
+    must = trace + I * N * (2 * 520 + 512) * 4 + I * T * N * 4 + I * N * N * 20
+    assert must < got < 1.05 * must
+    # the lanes that a group of 8 keeps for 1 instance
+    assert serve.fit_bytes(1, N, T, nh, 15, 500) > 8 * T * N * 3 * 4
+    assert serve.fit_bytes(I, N, T, nh, 3, 500) == serve.adjoint_bytes(I, N, T, nh)
+    long = 1 + adjoint.TRACE_BUDGET // (I * N * 12)
+    assert serve.fit_bytes(I, N, long, nh, 15, 500) == serve.adjoint_bytes(I, N, long, nh)
+    w, ln = network.synthetic_connectome(84, 0.3, seed=0)
+    conn = network.Connectivity.from_dense(w, ln)
+    req = serve.Request(rid=0, model='MPR', conn=conn, couplings=np.full(I, 0.1, np.float32),
+                        speeds=np.full(I, 4.0, np.float32), x0=np.zeros((I, N, 2), np.float32), nsteps=T)
+    plain = serve.footprint(req)
+    req.want_grad, req.target = True, np.eye(N)
+    assert trace < serve.footprint(req) - plain < 1e9

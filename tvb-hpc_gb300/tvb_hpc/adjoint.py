@@ -145,6 +145,23 @@ def adjoint_spread_shape(N, groups, sms):
     return adjoint_group_shape(N, pipelined=True)
 
 
+TRACE_BUDGET = 2 << 30   # default bytes of FCFit's traces
+
+
+def fit_layout(dmin, dmax, N):
+    """Layout of FCFit's sweeps: 'groups', the pipelined lane-interleaved group
+    kernel, where it applies (delays >= 2 K - 1, N <= 1024), else 'instances',
+    the per-instance step kernel."""
+    from .groups import plan_group, pipelined_threads
+    k, _ = plan_group(int(dmin), int(dmax))
+    return 'groups' if int(dmin) >= 2 * k - 1 and pipelined_threads(N, 16) else 'instances'
+
+
+def trace_bytes(I, N, T):
+    "r, V and the coupling sum of T steps of I instances in groups of 8 (FP32)."
+    return 4 * (-(-I // 8)) * 8 * T * N * 3
+
+
 class FCFit:
     """
     FC-fit problem for I instances of deterministic MPR + linear coupling.
@@ -179,13 +196,8 @@ class FCFit:
         self.consts = consts
         self.tpn = 1          # gather lanes per node of the per-instance sweeps
         self.adjoint_smem = 'auto'   # adjoint ring in shared memory: 'auto' or False
-        # forward and recomputation sweeps: the pipelined lane-interleaved
-        # group kernel where it applies (delays >= 2 K - 1, N <= 1024), else
-        # the per-instance step kernel
-        from .groups import plan_group, pipelined_threads, device_sms
-        k, _ = plan_group(int(d.min()), int(d.max()))
-        self.layout = ('groups' if int(d.min()) >= 2 * k - 1 and pipelined_threads(self.N, 16)
-                       else 'instances')
+        from .groups import device_sms
+        self.layout = fit_layout(d.min(), d.max(), self.N)
         # the reverse-time kernel on the grouped layout: lane-interleaved and
         # time-blocked (tvbg_adjoint_mpr_groups, blocks of K <= d_min steps)
         # where the delays and N allow, else per instance over the group trace
@@ -215,7 +227,7 @@ class FCFit:
         # copies of the checkpoints within trace_budget; the last window is
         # recomputed at the end of forward() (side stream, overlapping the
         # loss path) when eager_recompute
-        self.trace_budget = 2 << 30
+        self.trace_budget = TRACE_BUDGET
         self.recompute_window = None   # segments per window (None: by trace_budget, or none at all)
         self.eager_recompute = True
         if self.adjoint_kernel == 'groups':
@@ -309,7 +321,7 @@ class FCFit:
         S = -(-self.T // self.C)
         if self.recompute_window is not None and self.recompute_window < S:
             return False
-        return 4 * (-(-self.I // 8)) * 8 * self.T * self.N * 3 <= self.trace_budget
+        return trace_bytes(self.I, self.N, self.T) <= self.trace_budget
 
     def _group_sets(self, G, eta, traced):
         """The forward's and the recomputation's GroupSets, built on first use

@@ -89,7 +89,7 @@ class Request:
 def footprint(req):
     """Device bytes a request needs (rings, state, parameters, edges),
     estimated; a gradient request adds the FC-fit adjoint's memory
-    (adjoint_bytes), which it holds until its gradients are done."""
+    (fit_bytes), which it holds until its gradients are done."""
     from .engine import plan_ring
     N, I = req.conn.nnode, req.couplings.size
     d = req.conn.delays(float(np.min(req.speeds)), req.dt, 'ceil')
@@ -97,13 +97,31 @@ def footprint(req):
     ring = N * ((1 << lognh) + 8) * 4
     base = I * (ring + N * 4 * 6 + 512) + req.conn.nnz * 8 * len(np.unique(req.speeds))
     if req.want_grad and req.model == 'MPR' and req.target is not None:
-        base += adjoint_bytes(I, N, int(req.nsteps), 1 << lognh)
+        d0 = req.conn.delays(float(req.speeds[0]), req.dt, 'ceil')
+        base += fit_bytes(I, N, int(req.nsteps), 1 << lognh, int(d0.min()), int(d0.max()))
     return base
 
 
+def fit_bytes(I, N, T, nh, dmin, dmax):
+    """Device bytes of adjoint.FCFit for I instances, N nodes, T steps with
+    rings of up to nh slots: where it keeps the whole trace (the grouped layout,
+    the trace within its budget), the trace (r, V and the coupling sum in groups
+    of 8), the forward's ring and the adjoint's two (grouped and per instance),
+    dL/dr, the loss scratch (the FC twice, A) and what is per node; else
+    adjoint_bytes."""
+    from . import adjoint
+    if dmin < 3 or adjoint.fit_layout(dmin, dmax, N) != 'groups' or \
+            adjoint.trace_bytes(I, N, T) > adjoint.TRACE_BUDGET:
+        return adjoint_bytes(I, N, T, nh)
+    lanes = 8 * -(-I // 8)
+    rings = (2 * lanes * (nh + 8) + I * nh) * N * 4
+    return (adjoint.trace_bytes(I, N, T) + rings + I * (T + 1) * N * 4 + I * N * N * (8 * 2 + 4)
+            + lanes * N * 128)
+
+
 def adjoint_bytes(I, N, T, nh, checkpoint_every=100, trace_budget=2 << 30):
-    """Device bytes of adjoint.FCFit for I instances, N nodes, T steps:
-    the rate series (FP32 trace), dL/dr (FP32), the loss scratch (FC and A),
+    """Device bytes of adjoint.FCFit for I instances, N nodes, T steps where it
+    works from checkpoints: the rate series (FP32 trace), dL/dr (FP32), the loss scratch (FC and A),
     one state + ring checkpoint per chunk of checkpoint_every steps, the
     recomputation (windows of segments: r, V, S traces and working copies of
     their checkpoints, at most trace_budget) and the adjoint ring."""
