@@ -682,8 +682,9 @@ class GpuStep:
 
 class NetStep:
     """One bench step of the single large network: reset state and ring
-    from resident copies, advance nsteps (one seed launch and one launch per
-    block of K steps, node-parallel)."""
+    from resident copies, advance nsteps (one seed launch; one launch per
+    block of K steps, or one and its copy launch per two or three blocks where
+    the delays allow; node-parallel)."""
 
     def __init__(self, wl, torch):
         from tvb_hpc import model, coupling, scheme, bignet
@@ -700,7 +701,10 @@ class NetStep:
         self.ns = self.sw.ns
         self.status = self.sw.status
         self.tpn = None
-        self.path = 'node-parallel single network, one launch per block of %d steps' % self.sw.block_k
+        st = self.sw._stage
+        self.blocks = 1 if st is None else st.numel() // (8 * self.sw.N)   # blocks of 8 steps per launch
+        self.path = ('node-parallel single network, one launch per %s of %d steps'
+                     % ('block' if self.blocks == 1 else '%d blocks' % self.blocks, self.sw.block_k))
 
     def reset(self, x0=None):
         self.sw.state.copy_(self.x0 if x0 is None else x0)
@@ -722,7 +726,11 @@ class NetStep:
         return evs, None
 
     def launches_per_step(self):
-        return 1 + -(-self.wl['nsteps'] // self.sw.block_k)
+        if self.blocks == 1:
+            return 1 + -(-self.wl['nsteps'] // self.sw.block_k)
+        n, w = self.wl['nsteps'], 8 * self.blocks
+        wide = max(0, -(-(n - 8) // w))            # while more than 8 steps are left
+        return 1 + 2 * wide + (1 if n > wide * w else 0)
 
 
 class LemsStep:
@@ -834,14 +842,15 @@ class AdjointStep:
         return ([(e0, e1)] if time_kernels else []), None
 
     def launches_per_step(self):
-        # forward, Gram, loss, dL/dr, reverse-time kernel; over checkpoints, a
-        # forward per segment, and a recomputation and a reverse per window
-        if self.prob.layout == 'groups' and self.prob._traced():
-            return 5
+        # the loss path (means up to 192 nodes, Gram, loss, dL/dr), the forward and
+        # the reverse-time kernel; over checkpoints a forward per segment, and a
+        # recomputation and a reverse per window or segment
+        loss = 4 if self.prob.N <= 192 else 3
+        traced = self.prob.layout == 'groups' and self.prob._traced()
         segs = -(-self.wl['nsteps'] // self.wl['ckpt'])
         if self.prob.layout == 'groups' and self.prob.adjoint_kernel == 'groups':
-            return segs + 3 + 2 * len(self.prob._windows()[1])
-        return 3 * segs + 3
+            return loss + (2 if traced else segs + 2 * len(self.prob._windows()[1]))
+        return loss + (1 + segs if traced else 3 * segs)
 
     def grad_error(self, n_check=4):
         "Max-norm relative error of dL/dG and dL/deta vs the FP64 oracle on a sample."
@@ -1379,8 +1388,9 @@ def adjoint_finish(args, wl, gs, torch, world, rank, barrier_fn=None):
     h2d = wl['couplings'].nbytes + wl['eta'].nbytes
     d2h = sum(o.numel() * o.element_size() for o in out)
     err = gs.grad_error()
-    # forward, recomputation and reverse pass each stream the rings and state
-    bpn = 3 * algorithmic_bytes_per_node_step(wl, 2)
+    # forward, recomputation (over checkpoints) and reverse pass each stream the rings and state
+    passes = 2 if gs.prob.layout == 'groups' and gs.prob._traced() else 3
+    bpn = passes * algorithmic_bytes_per_node_step(wl, 2)
     peaks = {}
     p = os.path.join(ROOT, 'MEASURED_PEAKS.json')
     if os.path.exists(p):
@@ -1402,7 +1412,8 @@ def adjoint_finish(args, wl, gs, torch, world, rank, barrier_fn=None):
                          'peak_source': 'measured' if peaks.get('hbm_gbs') else 'fallback',
                          'algorithmic_bytes_per_node_step': round(bpn, 2),
                          'note': 'value counts forward node-steps over forward + backward time; '
-                                 'bytes = 3 passes (forward, recomputation, reverse) of 4E + 16'},
+                                 'bytes = %d passes (forward, %sreverse) of 4E + 16'
+                                 % (passes, 'recomputation, ' if passes == 3 else '')},
             'gradient_rel_err_vs_fp64': err, 'clocks': clk}
     if rank == 0 and world == 1 and not args.no_cpu:
         line['cpu_baseline'] = cpu_baseline_adjoint(wl)
