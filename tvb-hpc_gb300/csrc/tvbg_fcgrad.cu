@@ -10,6 +10,7 @@
 // itself, stay FP64 in the caller).
 #include "tvbg_abi_internal.h"
 #include "tvbg_gram.cuh"
+#include "tvbg_step_launch.cuh"
 
 namespace {
 
@@ -338,7 +339,8 @@ int launch_gram_split(SeriesView v, const double* mean, double* G, int n_inst, c
 // 668 and 632, 4 x 84 x 2000 756 and 629, 200 x 31 x 700 328 and 244.
 template <int RB>
 bool split_fills(int n_inst, int N) {
-    return static_cast<int64_t>(n_inst) * split_tiles<RB>(N) >= 152 * kSplitThreads;
+    return static_cast<int64_t>(n_inst) * split_tiles<RB>(N) >=
+           static_cast<int64_t>(tvbg::device_sms()) * kSplitThreads;
 }
 
 // N > kSplitMaxN: FP64 means and Gram by digit products (tvbg_gram.cuh), both

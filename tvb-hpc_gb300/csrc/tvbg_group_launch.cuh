@@ -38,15 +38,6 @@ inline int check_group_cfg(const tvbg_launch* cfg, const ErrSink& es, int* clust
     return TVBG_OK;
 }
 
-// SMs of the current device (0 if it cannot be asked).
-inline int device_sms() {
-    int dev = 0, n = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess ||
-        cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
-        return 0;
-    return n;
-}
-
 // Ring channels of a coupling id (the group kernel's shared-memory sums scale with it).
 inline int group_channels(int cfun) {
     return (cfun == TVBG_CFUN_KURAMOTO || cfun == TVBG_CFUN_LEMS_SC || cfun == TVBG_CFUN_LEMS_2) ? 2

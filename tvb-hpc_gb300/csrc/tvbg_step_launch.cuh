@@ -41,6 +41,15 @@ inline size_t step_smem_bytes(int threads, int smem_ring) {
     return static_cast<size_t>(smem_ring) + 4u * static_cast<size_t>(threads) + 16u;
 }
 
+// SMs of the current device (0 if it cannot be asked).
+inline int device_sms() {
+    int dev = 0, n = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
+        return 0;
+    return n;
+}
+
 // Set the kernel's shared-memory limit and size the grid: n_inst CTAs, or
 // (persistent) cfg->ctas or one CTA per SM with the work counter zeroed on
 // `st`.  *grid = 0 means there is nothing to launch.
