@@ -9,15 +9,15 @@ import types
 import numpy as np
 import pytest
 
-from tvb_hpc import autotune, groups
+from tvb_hpc import autotune, groups, _native as nat
 
 SMS = 152
 
 
-def shape(monkeypatch, N, G, resident, channels=1):
+def shape(monkeypatch, N, G, resident, channels=1, cfun=nat.CFUN_LINEAR):
     "spread_shape of G groups where resident(threads, cluster) clusters fit the device."
     monkeypatch.setattr(autotune, 'group_max_clusters', lambda s, t, c, tpn=1, n=0: resident(t, c))
-    s = types.SimpleNamespace(N=N, n_groups=G, can_pipeline=True, pipelined_built=True, channels=channels,
+    s = types.SimpleNamespace(cfun_id=cfun, N=N, n_groups=G, can_pipeline=True, pipelined_built=True, channels=channels,
                               pipe_tab=np.array([True]), gtab=np.zeros(G, int))
     return groups.spread_shape(s, SMS)
 
@@ -41,3 +41,16 @@ def test_choice_where_every_cluster_fits(monkeypatch):
     assert shape(monkeypatch, 84, 400, free)[:2] == (704, 2)
     assert shape(monkeypatch, 192, 400, free)[:2] == (768, 4)
     assert shape(monkeypatch, 998, 400, free)[:2] == (1024, 16)
+
+
+@pytest.mark.parametrize('N', [30, 84, 200, 400, 700])
+def test_sigmoidal_sets_beyond_residency_are_plain(monkeypatch, N):
+    """The Sigmoidal gather is bound by its exponentials: pipelined only where every
+    group's cluster is resident at once on an SM each."""
+    for G in (1, 8, 64, 512):
+        got = shape(monkeypatch, N, G, lambda t, c: SMS // c, cfun=nat.CFUN_SIGMOIDAL)
+        if got[3] == groups.PIPELINED:
+            assert G * got[1] <= SMS
+        else:
+            assert got == groups.plain_shape(N, G, SMS) + (0, 1)
+    assert shape(monkeypatch, N, 1, lambda t, c: SMS // c, cfun=nat.CFUN_SIGMOIDAL)[3] == groups.PIPELINED

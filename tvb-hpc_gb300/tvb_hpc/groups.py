@@ -129,6 +129,11 @@ def spread_shape(gset, sms=None):
         4.44, 768 x 4 3.45, 512 x 6 3.28).
     Two-channel rings whose CTAs exceed the 768-thread build stay on the plain
     kernel (Kuramoto, N = 998, 10 groups: 1.97 ms against 2.36).
+    More groups than are resident with the Sigmoidal coupling too: its gather
+    takes an exponential and a division per edge and step, and the pipelined
+    kernel has half of its threads for it (100 steps, plain / pipelined: N = 84,
+    256 groups 0.88 / 1.27 ms; N = 200, 64 groups 0.49 / 0.95; N = 400, 32 groups
+    0.58 / 1.65; N = 30, 512 groups 0.32 / 0.48).
     """
     from .autotune import group_max_clusters
     if sms is None:
@@ -148,6 +153,8 @@ def spread_shape(gset, sms=None):
     for t, c, _, tpn in reversed(shapes):
         if G * c <= sms and group_max_clusters(gset, t, c, tpn, live) >= live:
             return (t, c, 0, PIPELINED)
+    if gset.cfun_id == nat.CFUN_SIGMOIDAL:
+        return plain
     limit = 768 if gset.channels == 1 else 512
     fits = [s for s in shapes if s[0] <= limit and s[1] != 12]
     if not fits and gset.channels == 2:
