@@ -366,8 +366,8 @@ int tvbg_fc(const float *d_x, int32_t n_inst, int32_t T, int32_t N,
             double *d_err, void *stream);
 
 /*
- * tvbg_fc with caller scratch: N > 126 needs d_scratch of
- * tvbg_fc_scratch_bytes(n_inst, N) bytes (FP64 means and Gram); smaller N
+ * tvbg_fc with caller scratch: N > 127 needs d_scratch of
+ * tvbg_fc_scratch_bytes(n_inst, N) bytes (FP64 error parts and Gram); smaller N
  * needs none (d_scratch may be NULL).
  */
 int tvbg_fc_scratch_bytes(int32_t n_inst, int32_t N, int64_t *bytes);
@@ -382,7 +382,7 @@ int tvbg_fc_ex(const float *d_x, int32_t n_inst, int32_t T, int32_t N,
  * that may not take cudaMalloc's implicit device synchronisation.  It has no
  * counterpart in the reference.
  *
- * The FP64 scratch of the N > 126 path lives in a file-scope device array of
+ * The FP64 scratch of the N > 127 path lives in a file-scope device array of
  * TVBG_FC_NOALLOC_MAX_DOUBLES doubles (8 MiB), which every GPU that loads the
  * library holds until the process exits; a call needs n_inst * N * (N + 1)
  * doubles and is rejected with TVBG_EINVAL beyond that.  The first call on a
@@ -663,10 +663,11 @@ int tvbg_fcfit_zgrad(const float *d_z, const float *d_a, float *d_out, int32_t n
  * groups): row s < T - 1 at d_x + g * x_inst_stride + l + (s * N + i) *
  * lanes, row T - 1 at d_last + g * last_inst_stride + l + i *
  * last_node_stride (or from d_x too when d_last is NULL).  Computes the
- * Pearson FC to FP64 accuracy (two-pass: means, then the centred Gram, upper
- * triangle only, from exact products of 8-bit digits of the centred samples,
- * about 2^-53 of each node's largest deviation; norms from its diagonal; into
- * d_fc [n_inst][N][N] when not NULL), d_loss[b] = mean_{i<j}
+ * Pearson FC (two-pass: means, then the centred Gram, upper triangle only; up
+ * to 192 nodes in FP32 words with error-free transformations, to 4e-12 of
+ * |c_i| |c_j| or better, above that from exact products of 8-bit digits of
+ * the centred samples, about 2^-53 of each node's largest deviation; norms
+ * from its diagonal; into d_fc [n_inst][N][N] when not NULL), d_loss[b] = mean_{i<j}
  * (FC_ij - target_ij)^2 (FP64) and, when d_dx is not NULL, dL/dX (FP32) at
  * d_dx + b * dx_inst_stride + s * N + i.  target [N][N] FP64; d_scratch of
  * tvbg_fcfit_scratch_bytes().  Restates the Pearson FC of refs/covar.c:70-109
@@ -692,8 +693,8 @@ int tvbg_fcfit_loss_ex(const float *d_x, int64_t x_inst_stride, int32_t x_cols,
 /*
  * Region mapping (tvb_hpc/network.py:179-202).  to_avg: d_roi[i][j] = sum
  * of d_node[k][j] over the nodes k with d_rmap[k] == i (RMapToAvg zeroes roi
- * and accumulates: a sum), one CTA per region, a fixed reduction tree;
- * from_avg: d_node[k][j] = d_roi[d_rmap[k]][j] (RMapFromAvg).  rmap entries
+ * and accumulates: a sum), added up in a fixed order (warps' FP32 sums, FP64
+ * from there); from_avg: d_node[k][j] = d_roi[d_rmap[k]][j] (RMapFromAvg).  rmap entries
  * outside [0, nroi) map to no region (their node rows are left unchanged).
  */
 int tvbg_rmap_to_avg(int32_t nroi, int32_t nvar, int32_t nnode, const int32_t *d_rmap,

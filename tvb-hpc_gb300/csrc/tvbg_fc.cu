@@ -192,7 +192,8 @@ extern "C" int tvbg_fc_scratch_bytes(int32_t n_inst, int32_t N, int64_t* bytes) 
     return TVBG_OK;
 }
 
-// Large-N FC needs caller scratch of tvbg_fc_scratch_bytes() (FP64 means and Gram).
+// Large-N FC needs caller scratch of tvbg_fc_scratch_bytes() (FP64: an error part per
+// node, and the Gram).
 extern "C" int tvbg_fc_ex(const float* d_x, int32_t n_inst, int32_t T, int32_t N,
                           int64_t inst_stride, float* d_fc, const float* d_target, double* d_err,
                           double* d_scratch, void* stream) {
@@ -214,7 +215,7 @@ extern "C" int tvbg_fc_ex(const float* d_x, int32_t n_inst, int32_t T, int32_t N
         if (e != cudaSuccess) return set_cuda_error(e, "tvbg_fc: smem attribute");
         kfn<<<n_inst, kGramThreads, smem, st>>>(v, d_fc, d_target, d_err);
     } else {
-        if (!d_scratch) return set_error(TVBG_EINVAL, "tvbg_fc: N > 126 needs d_scratch (tvbg_fc_scratch_bytes)");
+        if (!d_scratch) return set_error(TVBG_EINVAL, "tvbg_fc: N > 127 needs d_scratch (tvbg_fc_scratch_bytes)");
         // scratch: N error parts per instance, then the Gram
         double* gram = d_scratch + static_cast<long long>(n_inst) * N;
         const size_t smem = gram_plane_bytes(128);
@@ -295,7 +296,7 @@ extern "C" int tvbg_fc_noalloc(const float* d_x, int32_t n_inst, int32_t T, int3
         rc = noalloc_scratch(dev, &scratch);
         if (rc) return rc;
     }
-    // the mean and Gram kernels write every scratch entry they later read,
+    // the Gram and norm kernels write every scratch entry that is read later,
     // so the previous call's contents need no clearing
     return tvbg_fc_ex(d_x, n_inst, T, N, inst_stride, d_fc, d_target, d_err, scratch, stream);
 }

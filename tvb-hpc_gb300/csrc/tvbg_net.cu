@@ -84,7 +84,8 @@ extern "C" int tvbg_net_run(const tvbg_net* net, int64_t t0, int32_t nsteps, con
 // `dmin`: the smallest delay (0 = not known); d_stage: floats for the new
 // slots of blocks launched together, [N][8 J].  J = 3 or 2 blocks of 8 steps
 // share a launch where dmin >= 8 J - 1 and the buffer holds them (lanes mapping,
-// block_k = 8); the tail of fewer than J blocks takes the single-block kernel.
+// block_k = 8); so does a tail of more than 8 steps, and one of at most 8
+// takes the single-block kernel.
 extern "C" int tvbg_net_run_ex(const tvbg_net* net, int64_t t0, int32_t nsteps, const tvbg_launch* cfg,
                                int32_t dmin, float* d_stage, int64_t stage_floats, void* stream) {
     if (!net || !cfg || nsteps < 0 || t0 < 0 || dmin < 0 || stage_floats < 0)

@@ -3,7 +3,9 @@
 // (the reference zeroes roi and accumulates, so it is a sum);
 // RMapFromAvg (194-202): node[k, j] = roi[rmap[k], j].
 //
-// to_avg reads every node once.  One cluster of CTAs takes the nodes in
+// to_avg: one cluster of CTAs reads every node once where nroi * nvar <= 1600
+// (kBins) and nvar <= 32 (kVars); beyond, one cluster for each part of the regions and
+// variables, and each scans the whole rmap.  A cluster's CTAs take the nodes in
 // consecutive parts, warp by warp; each warp adds its nodes, 32 at a time and
 // in order, to bins of its own in shared memory; the warps' bins meet in warp
 // order and the CTAs' in rank order, in FP64.  Every sum has a fixed order, so

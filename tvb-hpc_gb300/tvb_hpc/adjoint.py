@@ -15,8 +15,9 @@ forward traces them itself, in one launch (the group kernel's
 TVBG_F_TRACE_CSUM column), and nothing is computed twice.  Else it runs in
 chunks of `checkpoint_every` steps, keeping the state and the history ring
 at every chunk start (checkpoints) and the rate series.  tvbg_fcfit_loss_ex
-then takes the FC (tvbg_gram.cuh), the loss and dL/dr on the device in one
-call, no library GEMM.
+then takes the FC (its Gram in FP32 error-free arithmetic up to 192 nodes,
+tvbg_gram.cuh above), the loss and dL/dr on the device in one call, no
+library GEMM.
 
 ``FCFit.backward`` runs the reverse-time recursion over the whole trace in
 one launch, on lane-interleaved groups of 8 instances, time-blocked, with two

@@ -65,9 +65,8 @@ def pipelined_shape(gset, clusters=(1, 2, 3, 4, 6, 8, 12, 16), min_ctas=0):
     """(threads, cluster, 0, tpn) of gset on the pipelined kernel's smallest
     cluster that holds one node per slot and gives the set at least min_ctas
     CTAs (when some cluster does), or its plain default shape where the
-    pipelined kernel does not apply (short delays, N > 1024).  With few
-    groups, min_ctas = the SM count spreads them over the GPU (measured on
-    32 groups of N = 84: 704 x 2 8.45 ms per adjoint forward, 256 x 6 8.02)."""
+    pipelined kernel does not apply (short delays, N > 1024).  The smallest
+    cluster suits many groups; for few, spread_shape is the rule."""
     if gset.can_pipeline:
         fits = [(pipelined_threads(gset.N, c), c) for c in clusters]
         fits = [(t, c) for t, c in fits if t]
