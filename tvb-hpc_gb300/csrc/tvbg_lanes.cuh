@@ -37,9 +37,10 @@
 // block: the K slots of an edge are one run of consecutive floats, split over
 // the lanes in 32-byte loads (gather_run), and the sums cross to their owners
 // through shared memory.  L2 serves such runs to one CTA of 512 threads per
-// SM at 20 TB/s from a 48 MB working set, 12.6 TB/s from 96 MB and 8.5 TB/s
-// from 192 MB; one float per lane and load reached 9.4, 7.2 and 6.1, two
-// 16-byte loads 32 bytes apart 10.6, 10.0 and 8.5.
+// SM at 21.6 TB/s from a 48 MB working set, 17.0 TB/s from 96 MB and 9.1 TB/s
+// from 192 MB, in 32-byte loads or in two 16-byte loads that are contiguous
+// over the lanes (21.4, 16.2, 9.2); one float per lane and load reached 10.0, 9.2
+// and 7.2, two 16-byte loads of a lane's own 32 bytes 10.7, 10.6 and 8.6.
 // (Staging the runs in shared memory with cp.async.bulk was measured slower;
 // a rolling window of loads or predicated loads inside the batch spill at
 // these register counts and were slower too.)

@@ -228,9 +228,10 @@ __global__ void __launch_bounds__(256)
 // J blocks of 8 steps per launch, 8 lanes per node: lane k sums the steps
 // tb + k, tb + 8 + k, ..., so an edge reads one run of 8 J slots (32 J bytes) and
 // its record once.  A random source's run costs DRAM about (8 J + 15) / 16 chunks
-// of 64 bytes, so longer runs move fewer bytes a step: about 100 with J = 1, 67
-// with J = 2, 55 with J = 3, the edge records included.  Needs every delay >=
-// 8 J - 1.  The ring is not written: the new slots go to stage[n][8 J] and
+// of 64 bytes, so longer runs move fewer bytes per edge and 8 steps: 104 with
+// J = 1, 68 with J = 2, 56 with J = 3 by that count, the edge records included
+// (captured at 100 000 nodes: 91 with J = 1, 48 with J = 3, DRAM at 69 % of its
+// peak).  Needs every delay >= 8 J - 1.  The ring is not written: the new slots go to stage[n][8 J] and
 // net_copy_kernel puts them in place, so nh > d_max is enough (a run wraps at
 // nh slot by slot).  515 056 nodes, 64 edges a node, 24 steps: 2.62 ms with
 // one block per launch, 1.47 with three and each lane reading every record, 1.15
