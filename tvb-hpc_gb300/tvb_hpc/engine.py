@@ -413,7 +413,8 @@ class InstanceSet:
         tab['lognh'] = self.lognh
         tab['model'] = self.model_id
         tab['cfun'] = self.cfun_id
-        limit = np.array([self.smem_ring_limit(self.threads(k), k) for k in self.block_k])
+        ks, inv = np.unique(self.block_k, return_inverse=True)
+        limit = np.array([self.smem_ring_limit(self.threads(k), k) for k in ks])[inv]
         fits = (self.ring_bytes <= limit) if smem_allowed else np.zeros(I, bool)
         fl = (self.flags | self.order_flags).astype(np.uint32)
         fl = np.where(self.pipe, fl | nat.F_PIPELINE, fl).astype(np.uint32)
