@@ -78,6 +78,90 @@ __global__ void __launch_bounds__(kGramThreads)
     }
 }
 
+// Few nodes and short series: one CTA per instance, FP64 sums of the centred
+// samples, three pairs of the upper triangle per thread.  The digit path works
+// through whole tiles of 96 rows and 64 samples and costs 75 ns an instance before its first
+// sample, this one 12 (us for 4096 instances, digits / FP64 sums: 10 nodes x 20 samples 384 / 72, 50 x 8 525 / 284).
+constexpr int kDirectThreads = 512;
+constexpr int kDirectTile = 32;
+constexpr int kDirectNodes = 50;
+constexpr int kDirectPairs = (kDirectNodes * (kDirectNodes + 1) / 2 + kDirectThreads - 1) / kDirectThreads;
+__global__ void __launch_bounds__(kDirectThreads)
+    fc_direct_kernel(const float* __restrict__ x, int T, int N, long long inst_stride, float* __restrict__ fc,
+                     const float* __restrict__ target, double* __restrict__ err) {
+    __shared__ double mean[kDirectNodes], rn[kDirectNodes];
+    __shared__ double tile[kDirectTile][kDirectNodes];
+    __shared__ double part[kDirectThreads / 32];
+    const float* xb = x + blockIdx.x * inst_stride;
+    const int tid = threadIdx.x, lane = tid % 32, warp = tid / 32;
+    if (tid < N) {
+        double s = 0.0;
+#pragma unroll 8
+        for (int t = 0; t < T; ++t) s += static_cast<double>(__ldg(xb + static_cast<long long>(t) * N + tid));
+        mean[tid] = s / static_cast<double>(T);
+    }
+    const int npairs = N * (N + 1) / 2;
+    double acc[kDirectPairs];
+    int pi[kDirectPairs], pj[kDirectPairs];   // row-major upper triangle
+#pragma unroll
+    for (int q = 0; q < kDirectPairs; ++q) {
+        acc[q] = 0.0;
+        int i = 0, rem = tid + q * kDirectThreads;
+        if (rem < npairs) {
+            while (rem >= N - i) {
+                rem -= N - i;
+                ++i;
+            }
+        } else {
+            rem = 0;
+        }
+        pi[q] = i;
+        pj[q] = i + rem;
+    }
+    for (int t0 = 0; t0 < T; t0 += kDirectTile) {
+        const int nt = T - t0 < kDirectTile ? T - t0 : kDirectTile;
+        __syncthreads();
+        for (int e = tid; e < nt * N; e += kDirectThreads) {
+            const int tt = e / N, i = e - tt * N;
+            tile[tt][i] = static_cast<double>(__ldg(xb + static_cast<long long>(t0 + tt) * N + i)) - mean[i];
+        }
+        __syncthreads();
+#pragma unroll
+        for (int q = 0; q < kDirectPairs; ++q)
+            if (tid + q * kDirectThreads < npairs)
+                for (int tt = 0; tt < nt; ++tt) acc[q] = fma(tile[tt][pi[q]], tile[tt][pj[q]], acc[q]);
+    }
+#pragma unroll
+    for (int q = 0; q < kDirectPairs; ++q)
+        if (tid + q * kDirectThreads < npairs && pi[q] == pj[q]) rn[pi[q]] = 1.0 / sqrt(acc[q]);
+    __syncthreads();
+    double e_local = 0.0;
+    float* fcb = fc + static_cast<long long>(blockIdx.x) * N * N;
+#pragma unroll
+    for (int q = 0; q < kDirectPairs; ++q)
+        if (tid + q * kDirectThreads < npairs) {
+            const int i = pi[q], j = pj[q];
+            const double r = acc[q] * (rn[i] * rn[j]);
+            fcb[i * N + j] = static_cast<float>(r);
+            fcb[j * N + i] = static_cast<float>(r);
+            if (target && i < j) {
+                const double dd = r - static_cast<double>(__ldg(target + i * N + j));
+                e_local = fma(dd, dd, e_local);
+            }
+        }
+    if (err) {
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) e_local += __shfl_down_sync(0xffffffffu, e_local, o);
+        if (lane == 0) part[warp] = e_local;
+        __syncthreads();
+        if (tid == 0) {
+            double e = 0.0;
+            for (int k = 0; k < kDirectThreads / 32; ++k) e += part[k];
+            err[blockIdx.x] = e;
+        }
+    }
+}
+
 // Larger N: the upper triangle of the Gram, one CTA per 64 x 64 tile.
 __global__ void __launch_bounds__(kGramThreads) fc_gram_kernel(SeriesView v, double* __restrict__ gram) {
     extern __shared__ __align__(16) unsigned char fc_smem[];
@@ -179,6 +263,13 @@ using namespace tvbg;
 namespace {
 // Whether N nodes take the one-CTA small path (no scratch).
 bool fc_small_path(int32_t N) { return N <= kFcSmallMax; }
+// Whether the call takes FP64 sums: up to the line where an FP64 kernel had taken as
+// long as the digits.  On it this one wins (us for 4096 instances, FP64 / digits:
+// N = 10, T = 150 231 / 739; N = 16, T = 100 247 / 606; N = 50, T = 20 405 / 571); 64 nodes were equal
+// at T = 3 already.
+bool direct_is_faster(int32_t T, int32_t N) {
+    return N <= kDirectNodes && static_cast<int64_t>(T) * (N * N + 300) <= 70000;
+}
 }  // namespace
 
 extern "C" int tvbg_fc_scratch_bytes(int32_t n_inst, int32_t N, int64_t* bytes) {
@@ -203,7 +294,9 @@ extern "C" int tvbg_fc_ex(const float* d_x, int32_t n_inst, int32_t T, int32_t N
         return set_error(TVBG_EINVAL, "tvbg_fc: d_target and d_err go together");
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     const SeriesView v{d_x, inst_stride, nullptr, 0, 0, T, N, 1, 1};
-    if (fc_small_path(N)) {
+    if (direct_is_faster(T, N)) {
+        fc_direct_kernel<<<n_inst, kDirectThreads, 0, st>>>(d_x, T, N, inst_stride, d_fc, d_target, d_err);
+    } else if (fc_small_path(N)) {
         const bool half = N <= 96;
         const size_t smem = gram_plane_bytes(half ? 96 : 128) + sizeof(double) * (static_cast<size_t>(N) * (N + 1) / 2);
         auto kfn = half ? fc_small_kernel<96> : fc_small_kernel<128>;
