@@ -123,6 +123,53 @@ __global__ void __launch_bounds__(kCovThreads)
     mean[b * N + i] = mi;
 }
 
+// One sample (updates of a running simulation): bound by the passes over m2,
+// which are read and written row by row, without the mirror's transposed
+// writes (300 instances of 84 nodes 17.4 -> 10.8 us, 4096 132 -> 82, 600 of 500 568 -> 398).  Entry (j, i) of the lower triangle takes the product of (i, j), so
+// both kernels give the same bits.  CTA blockIdx.x of gridDim.x takes every
+// gridDim.x-th run of 2048 entries; the means as in cov_update_kernel.
+__global__ void __launch_bounds__(kCovThreads)
+    cov_sample_kernel(const float* __restrict__ x, long long inst_stride, int N, long long n,
+                      double* __restrict__ mean, double* __restrict__ m2) {
+    extern __shared__ double sh[];  // d[N] | e[N]
+    double* d = sh;
+    double* e = sh + N;
+    const long long b = blockIdx.y;
+    double* mb = mean + b * N;
+    double* cb = m2 + b * static_cast<long long>(N) * N;
+    const double rn = 1.0 / static_cast<double>(n + 1);
+    for (int i = threadIdx.x; i < N; i += kCovThreads) {
+        const double mi = n == 0 ? 0.0 : mb[i];
+        const double xi = static_cast<double>(__ldg(x + b * inst_stride + i));
+        const double di = xi - mi;
+        const double m_new = mi + di * rn;
+        d[i] = di;
+        e[i] = xi - m_new;
+        if (gridDim.x == 1) mb[i] = m_new;
+    }
+    __syncthreads();
+    // entries q, q + 256, ...: eight of them in flight
+    constexpr int U = 8;
+    const int NN = N * N, step_i = kCovThreads / N, step_j = kCovThreads % N;
+    int q = blockIdx.x * (U * kCovThreads) + threadIdx.x;
+    for (; q < NN; q += gridDim.x * (U * kCovThreads)) {
+        double a[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) a[u] = n != 0 && q + u * kCovThreads < NN ? cb[q + u * kCovThreads] : 0.0;
+        int i = q / N, j = q - i * N;
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            if (q + u * kCovThreads < NN) cb[q + u * kCovThreads] = fma(d[min(i, j)], e[max(i, j)], a[u]);
+            i += step_i;
+            j += step_j;
+            if (j >= N) {
+                j -= N;
+                ++i;
+            }
+        }
+    }
+}
+
 // 32 x 32 tiles, a reciprocal square root per node of the tile and two
 // products per pair (a root and a division per entry took 72 us for 256 x 84
 // nodes).
@@ -158,9 +205,47 @@ __global__ void __launch_bounds__(kCovThreads)
     }
 }
 
+// Few nodes (N <= 32): a warp per instance, eight to a CTA; the arithmetic of
+// cov_corr_kernel, whose CTA per instance is mostly start and synchronisation.
+__global__ void __launch_bounds__(kCovThreads)
+    cov_corr_small_kernel(const double* __restrict__ m2, int n_inst, int N, float* __restrict__ corr) {
+    const long long b = blockIdx.x * static_cast<long long>(kCovThreads / 32) + threadIdx.x / 32;
+    if (b >= n_inst) return;   // whole warps
+    const int lane = threadIdx.x % 32, NN = N * N;
+    const double* cb = m2 + b * NN;
+    const double r = lane < N ? 1.0 / sqrt(cb[lane * N + lane]) : 0.0;
+#pragma unroll 4
+    for (int q0 = 0; q0 < NN; q0 += 32) {
+        const int q = q0 + lane, i = q < NN ? q / N : 0, j = q < NN ? q % N : 0;
+        const double ri = __shfl_sync(0xffffffffu, r, i), rj = __shfl_sync(0xffffffffu, r, j);
+        if (q < NN)
+            corr[b * NN + q] = static_cast<float>(cb[i <= j ? q : j * N + i] * (ri * rj));
+    }
+}
+
 // Launch over all instances (gridDim.y at most 65535 at a time).
 static int cov_rows(const float* x, int64_t inst_stride, int64_t row_stride, int rows, int n_inst, int N, int64_t n,
                     double* mean, double* m2, cudaStream_t st) {
+    // (many instances of one tile: cov_update_kernel, 4096 of 5 nodes 15 us against 17)
+    if (rows == 1 && !(N <= kCovTile && n_inst >= 600)) {
+        // few instances of many nodes: about 1200 CTAs share the entries (and a
+        // launch more sets the means)
+        const int runs = (N * N + 8 * kCovThreads - 1) / (8 * kCovThreads);
+        int parts = N <= 64 || n_inst >= 600 || (N <= 100 && n_inst >= 150) ? 1 : 1200 / n_inst;
+        parts = parts > runs ? runs : parts;
+        for (int b0 = 0; b0 < n_inst; b0 += 65535) {
+            const unsigned nb = static_cast<unsigned>(n_inst - b0 < 65535 ? n_inst - b0 : 65535);
+            const float* xb = x + b0 * inst_stride;
+            double* mb = mean + static_cast<int64_t>(b0) * N;
+            cov_sample_kernel<<<dim3(static_cast<unsigned>(parts), nb), kCovThreads, 2u * sizeof(double) * N, st>>>(
+                xb, inst_stride, N, n, mb, m2 + static_cast<int64_t>(b0) * N * N);
+            if (parts > 1)
+                cov_mean_kernel<<<dim3(static_cast<unsigned>((N + kCovThreads - 1) / kCovThreads), nb), kCovThreads, 0,
+                                  st>>>(xb, inst_stride, row_stride, 1, N, n, mb);
+        }
+        const cudaError_t e = cudaGetLastError();
+        return e == cudaSuccess ? TVBG_OK : set_cuda_error(e, "tvbg_cov_update launch");
+    }
     // samples per pass: as many as kCovPassBytes holds, 4 to 16
     int RC = static_cast<int>(kCovPassBytes / (16 * static_cast<int64_t>(N)));
     RC = RC > 16 ? 16 : (RC < 4 ? 4 : RC);
@@ -214,6 +299,15 @@ extern "C" int tvbg_cov_corr(const double* d_m2, int32_t n_inst, int32_t N, floa
     if (n_inst < 0 || N <= 0 || (n_inst > 0 && (!d_m2 || !d_corr)))
         return set_error(TVBG_EINVAL, "tvbg_cov_corr: bad arguments");
     if (n_inst == 0) return TVBG_OK;
+    // us, a warp / a tile of 32 x 32 per instance: N = 5, 600 instances 5.0 / 8.8, one 4.3 / 5.0;
+    // N = 24, 1200 instances 10.8 / 13.1, 600 10.8 / 8.9; N = 32, 4096 instances 37 / 34
+    if (N <= 10 || (N <= 24 && n_inst >= 1000)) {
+        constexpr int kPer = kCovThreads / 32;
+        cov_corr_small_kernel<<<static_cast<unsigned>((static_cast<int64_t>(n_inst) + kPer - 1) / kPer), kCovThreads, 0,
+                                static_cast<cudaStream_t>(stream)>>>(d_m2, n_inst, N, d_corr);
+        const cudaError_t es = cudaGetLastError();
+        return es == cudaSuccess ? TVBG_OK : set_cuda_error(es, "tvbg_cov_corr launch");
+    }
     const long long nt = (static_cast<long long>(N) + kCovTile - 1) / kCovTile, tiles = nt * (nt + 1) / 2;
     if (tiles > 0x7fffffffLL) return set_error(TVBG_EINVAL, "tvbg_cov_corr: N too large");
     for (int b0 = 0; b0 < n_inst; b0 += 65535) {
