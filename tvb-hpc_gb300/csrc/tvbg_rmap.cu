@@ -3,7 +3,8 @@
 // (the reference zeroes roi and accumulates, so it is a sum);
 // RMapFromAvg (194-202): node[k, j] = roi[rmap[k], j].
 //
-// to_avg: one cluster of CTAs reads every node once where nroi * nvar <= 1600
+// to_avg: few nodes are scanned by one CTA per region (rmap_scan_kernel).  Else
+// one cluster of CTAs reads every node once where nroi * nvar <= 1600
 // (kBins) and nvar <= 32 (kVars); beyond, one cluster for each part of the regions and
 // variables, and each scans the whole rmap.  A cluster's CTAs take the nodes in
 // consecutive parts, warp by warp; each warp adds its nodes, 32 at a time and
@@ -134,6 +135,66 @@ __global__ void __launch_bounds__(kThreads, 1)
     tvbg::group_barrier(C > 1);   // no CTA leaves while its sums may be read
 }
 
+// Few nodes: one CTA per region and NJ variables scans the whole map; the
+// threads add their strided nodes, and meet in a fixed tree, in pairs of FP32
+// words (TwoSum; FP64 adds, two per SM and clock, made the scan twice as slow).
+constexpr int kScanThreads = 256;
+constexpr int kScanVars = 4;
+
+struct SumPair {
+    float s = 0.0f, c = 0.0f;
+    __device__ __forceinline__ void add(float x, float xc) {
+        const float t = __fadd_rn(s, x), b = __fsub_rn(t, s);
+        const float e = __fadd_rn(__fsub_rn(s, __fsub_rn(t, b)), __fsub_rn(x, b));
+        s = t;
+        c = __fadd_rn(c, __fadd_rn(e, xc));
+    }
+    // an infinite or NaN sum has a NaN error word
+    __device__ __forceinline__ float value() const { return isfinite(s) ? __fadd_rn(s, c) : s; }
+};
+
+template <int NJ>
+__global__ void __launch_bounds__(kScanThreads)
+    rmap_scan_kernel(int nvar, int nnode, const int32_t* __restrict__ rmap, const float* __restrict__ node,
+                     float* __restrict__ roi) {
+    __shared__ float2 part[kScanThreads / 32][NJ];
+    const int i = blockIdx.x, warp = threadIdx.x / 32, lane = threadIdx.x % 32;
+    for (int j0 = blockIdx.y * NJ; j0 < nvar; j0 += gridDim.y * NJ) {
+        SumPair s[NJ];
+        constexpr int U = 8;   // map entries read ahead
+        for (int k0 = threadIdx.x; k0 < nnode; k0 += U * kScanThreads) {
+            int r[U];
+#pragma unroll
+            for (int u = 0; u < U; ++u) r[u] = k0 + u * kScanThreads < nnode ? __ldg(rmap + k0 + u * kScanThreads) : -1;
+#pragma unroll
+            for (int u = 0; u < U; ++u)
+                if (r[u] == i) {
+                    const float* p = node + static_cast<size_t>(k0 + u * kScanThreads) * nvar + j0;
+#pragma unroll
+                    for (int j = 0; j < NJ; ++j)
+                        if (j0 + j < nvar) s[j].add(__ldg(p + j), 0.0f);
+                }
+        }
+#pragma unroll
+        for (int j = 0; j < NJ; ++j) {
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) {
+                const float x = __shfl_down_sync(0xffffffffu, s[j].s, o), c = __shfl_down_sync(0xffffffffu, s[j].c, o);
+                s[j].add(x, c);
+            }
+            if (lane == 0) part[warp][j] = make_float2(s[j].s, s[j].c);
+        }
+        __syncthreads();
+        if (threadIdx.x < NJ && j0 + static_cast<int>(threadIdx.x) < nvar) {
+            SumPair t;
+#pragma unroll
+            for (int w = 0; w < kScanThreads / 32; ++w) t.add(part[w][threadIdx.x].x, part[w][threadIdx.x].y);
+            roi[static_cast<size_t>(i) * nvar + j0 + threadIdx.x] = t.value();
+        }
+        __syncthreads();
+    }
+}
+
 __global__ void rmap_from_avg_kernel(int nroi, int nvar, long long n, const int32_t* __restrict__ rmap,
                                      const float* __restrict__ roi, float* __restrict__ node) {
     for (long long e = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; e < n;
@@ -143,6 +204,20 @@ __global__ void rmap_from_avg_kernel(int nroi, int nvar, long long n, const int3
         const int i = __ldg(rmap + k);
         if (i >= 0 && i < nroi) node[e] = __ldg(roi + static_cast<size_t>(i) * nvar + j);
     }
+}
+
+// Which kernel: their times in ns.  The scan takes 5 us and 0.06 us for every 256
+// nodes (0.12 with few regions, whose warps add at every trip), and all its CTAs
+// together 3 ns each and 0.2 ps per map entry; the cluster takes 9 us and 22 ns
+// for every bin, which 32 warps clear and add up.  us, scan / cluster, random maps:
+// 4000 nodes of 400 regions, 4 variables 6.8 / 47, 16 000 9.3 / 46; 8000 of 2
+// regions, one variable 7.4 / 13, 16 000 of 2, two variables about 18 / 13.
+bool scan_is_faster(int nroi, int nvar, int nnode) {
+    const double ctas = static_cast<double>(nroi) * ((nvar + kScanVars - 1) / kScanVars);
+    const double scan = 5000.0 + nnode / (nroi < 128 ? 2.2 : 4.0) + ctas * (3.0 + nnode / 5000.0);
+    const int nj = std::min(nvar, kVars);
+    const double bins = static_cast<double>(std::min(nroi, kBins / nj)) * nj;   // of one cluster
+    return scan < 9000.0 + 22.0 * bins;
 }
 
 }  // namespace
@@ -155,6 +230,14 @@ int tvbg_rmap_to_avg(int32_t nroi, int32_t nvar, int32_t nnode, const int32_t* d
         (nroi > 0 && nvar > 0 && !d_roi))
         return tvbg::set_error(TVBG_EINVAL, "tvbg_rmap_to_avg: bad arguments");
     if (nroi == 0 || nvar == 0) return TVBG_OK;
+    if (scan_is_faster(nroi, nvar, nnode)) {
+        const int gv = (nvar + kScanVars - 1) / kScanVars;
+        const auto scan = nvar <= 2 ? rmap_scan_kernel<2> : rmap_scan_kernel<kScanVars>;
+        scan<<<dim3(static_cast<unsigned>(nroi), static_cast<unsigned>(std::min(gv, 65535))), kScanThreads, 0,
+                           static_cast<cudaStream_t>(stream)>>>(nvar, nnode, d_rmap, d_node, d_roi);
+        const cudaError_t es = cudaGetLastError();
+        return es == cudaSuccess ? TVBG_OK : tvbg::set_cuda_error(es, "tvbg_rmap_to_avg launch");
+    }
     const int nj = std::min(nvar, kVars);
     const int roi_step = std::min(nroi, kBins / nj);
     const long long gy = (static_cast<long long>(nroi) + roi_step - 1) / roi_step;
