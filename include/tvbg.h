@@ -693,8 +693,8 @@ int tvbg_fcfit_loss_ex(const float *d_x, int64_t x_inst_stride, int32_t x_cols,
 /*
  * Region mapping (tvb_hpc/network.py:179-202).  to_avg: d_roi[i][j] = sum
  * of d_node[k][j] over the nodes k with d_rmap[k] == i (RMapToAvg zeroes roi
- * and accumulates: a sum), added up in a fixed order (warps' FP32 sums, FP64
- * from there); from_avg: d_node[k][j] = d_roi[d_rmap[k]][j] (RMapFromAvg).  rmap entries
+ * and accumulates: a sum), added up in a fixed order (few nodes: in pairs of
+ * FP32 words; else warps' FP32 sums, FP64 from there); from_avg: d_node[k][j] = d_roi[d_rmap[k]][j] (RMapFromAvg).  rmap entries
  * outside [0, nroi) map to no region (their node rows are left unchanged).
  */
 int tvbg_rmap_to_avg(int32_t nroi, int32_t nvar, int32_t nnode, const int32_t *d_rmap,
