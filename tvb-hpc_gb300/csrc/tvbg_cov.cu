@@ -300,8 +300,9 @@ extern "C" int tvbg_cov_corr(const double* d_m2, int32_t n_inst, int32_t N, floa
         return set_error(TVBG_EINVAL, "tvbg_cov_corr: bad arguments");
     if (n_inst == 0) return TVBG_OK;
     // us, a warp / a tile of 32 x 32 per instance: N = 5, 600 instances 5.0 / 8.8, one 4.3 / 5.0;
-    // N = 24, 1200 instances 10.8 / 13.1, 600 10.8 / 8.9; N = 32, 4096 instances 37 / 34
-    if (N <= 10 || (N <= 24 && n_inst >= 1000)) {
+    // N = 10, 64 instances 6.8 / 5.2, 600 6.8 / 8.9; N = 24, 600 instances 10.8 / 8.9, 1200 10.8 / 13.1;
+    // N = 32, 4096 instances 37 / 34
+    if (N <= 6 || (N <= 16 && n_inst >= 400) || (N <= 24 && n_inst >= 1000)) {
         constexpr int kPer = kCovThreads / 32;
         cov_corr_small_kernel<<<static_cast<unsigned>((static_cast<int64_t>(n_inst) + kPer - 1) / kPer), kCovThreads, 0,
                                 static_cast<cudaStream_t>(stream)>>>(d_m2, n_inst, N, d_corr);
